@@ -392,9 +392,9 @@ def run_ours(args, w):
     launches = int(reduce_over_ranks([float(st1["all_launches"] - st0["all_launches"])], "sum", device="cuda")[0])
 
     # roofline of the fused iteration kernel over the timed region
-    it_launches = st1["launches"] - st0["launches"]
+    # (per iteration: a launch of the on-chip form runs many)
     it_ms = st1["kernel_ms"] - st0["kernel_ms"]
-    avg_launch_s = it_ms / 1000.0 / max(it_launches, 1)
+    avg_launch_s = it_ms / 1000.0 / max((st1["cell_updates"] - st0["cell_updates"]) // (n * n), 1)
     bytes_alg = 64 * n * n  # Ux, Uy, Vx, Vy read once and written once, FP64
     achieved = bytes_alg / avg_launch_s / 1e9
     peak, peak_kind = measured_peaks()
@@ -413,12 +413,13 @@ def run_ours(args, w):
             "e2e": None,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": ncu_traffic(args.workload),
-                         "kernel": "k_iter_stream (fused stress, J2 return, momentum update)",
+                         "kernel": "fused stress, J2 return, momentum update (k_iter_chip for runs of "
+                                   "iterations of a grid that fits on chip, else the kernel form above)",
                          "algorithmic_bytes_per_launch": bytes_alg, "avg_launch_us": avg_launch_s * 1e6,
                          "peak_source": peak_kind,
-                         "note": "the %d^2 state (%.0f MB) is L2-resident within a step, so this fraction "
-                                 "measures throughput against a bound the kernel does not meet here; the "
-                                 "HBM-resident case of the same kernel is roofline_hbm" % (n, 13 * 8 * n * n / 1e6)},
+                         "note": "per iteration; on chip the %d^2 state does not leave the SMs between "
+                                 "iterations, so this fraction measures throughput against a bound the kernel "
+                                 "does not meet here; the HBM-resident case is roofline_hbm" % n},
             "gpu_launches": launches,
             "clocks": clocks.summary(),
             "cell_updates_per_s": iters_per_s * n * n,

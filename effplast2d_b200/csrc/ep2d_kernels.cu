@@ -4,6 +4,7 @@
 #include <type_traits>
 
 #include "ep2d_device.cuh"
+#include "ep2d_iter_chip.cuh"
 #include "ep2d_iter_f64.cuh"
 #include "ep2d_iter_stream.cuh"
 
@@ -117,8 +118,17 @@ int occupancy_ty(bool record) {
   return e == cudaSuccess && n > 0 ? n : 1;
 }
 
+template <bool PLASTIC, typename TV>
+cudaError_t set_chip_attr() {
+  return cudaFuncSetAttribute(k_iter_chip<PLASTIC, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, CHIP_SMEM);
+}
+
 cudaError_t prepare_kernels_impl() {
   cudaError_t e;
+  if ((e = set_chip_attr<false, double>()) != cudaSuccess) return e;
+  if ((e = set_chip_attr<true, double>()) != cudaSuccess) return e;
+  if ((e = set_chip_attr<false, float>()) != cudaSuccess) return e;
+  if ((e = set_chip_attr<true, float>()) != cudaSuccess) return e;
   if ((e = set_attrs_ty<8, double>()) != cudaSuccess) return e;
   if ((e = set_attrs_ty<16, double>()) != cudaSuccess) return e;
   if ((e = set_attrs_ty<32, double>()) != cudaSuccess) return e;
@@ -242,6 +252,59 @@ cudaError_t launch_iter_resident(const Geo& g, const Fields& f, int src, bool pl
     n_iter -= n;
   }
   return cudaSuccess;
+}
+
+// The shape of the on-chip form for a grid.  Rows first: the fewest rows per warp (a march
+// of R rows costs R + 3 row steps, and a warp's latency sets the time of a small grid) for
+// which every tile finds a place among CHIP_SMS CTAs of CHIP_WARPS warps.  Then the fewest
+// warps per SM, in tiles of at least 4 warps, and more tiles per CTA rather than fewer: while one
+// waits for its neighbours' rims another computes (1024^2, us an iteration: 4 tiles of
+// 4 warps 9.9, 2 of 8 10.3, 1 of 16 10.7; 512^2, 6 rows: 3 of 4 4.27, 2 of 6 4.34, 4 of 4 4.78;
+// 256^2, 2 rows: 2 of 5 2.70, 2 of 7 2.89, 1 of 10 2.85).
+ChipShape chip_shape(int nx, int ny) {
+  ChipShape best;
+  const int ncx = (nx + STREAM_COLS - 1) / STREAM_COLS;
+  for (int rows = 2; rows <= 18 && !best.warps; rows += 2) {
+    int best_cost = 1 << 30;
+    for (int groups = 1; groups <= 4; groups++)
+      for (int warps = 4; groups * warps <= CHIP_WARPS; warps++) {
+        const int ncy = (ny + warps * rows - 1) / (warps * rows);
+        if ((int64_t)ncx * ncy > (int64_t)CHIP_SMS * groups || chip_smem_bytes(groups, warps, rows) > CHIP_SMEM)
+          continue;
+        const int cost = groups * warps + (groups == 1 ? 1 : 0);  // warps per SM
+        if (cost <= best_cost) {
+          best_cost = cost;
+          best.warps = warps;
+          best.rows = rows;
+          best.groups = groups;
+          best.ncx = ncx;
+          best.ncy = ncy;
+        }
+      }
+  }
+  return best;
+}
+
+size_t chip_rim_bytes(const ChipShape& s) {
+  return (size_t)2 * s.ncx * s.ncy * (4 * s.warps * s.rows + 4 * STREAM_COLS) * RIM_BYTES;
+}
+
+cudaError_t launch_iter_chip(const Geo& g, const Fields& f, int src, bool plastic, bool mixed, const ChipShape& s,
+                             int n_iter, uint32_t tag, void* rim, unsigned long long timeout_ns, cudaStream_t stream) {
+  if (n_iter < 2 || s.warps < 1 || s.groups < 1 || s.warps * s.groups > 16 || s.rows < 2 || (s.rows & 1) || !f.gbar || !rim)
+    return cudaErrorInvalidValue;
+  const void* kern = mixed ? (plastic ? (const void*)k_iter_chip<true, float> : (const void*)k_iter_chip<false, float>)
+                           : (plastic ? (const void*)k_iter_chip<true, double> : (const void*)k_iter_chip<false, double>);
+  Geo ga = g;
+  Fields fa = f;
+  int srca = src, na = n_iter, nw = s.warps, rows = s.rows, ncx = s.ncx, ncy = s.ncy;
+  uint32_t ta = tag;
+  char* ra = static_cast<char*>(rim);
+  unsigned long long to = timeout_ns;
+  void* args[] = {&ga, &fa, &srca, &na, &nw, &rows, &ncx, &ncy, &ta, &ra, &to};
+  const int blocks = (s.ncx * s.ncy + s.groups - 1) / s.groups;
+  return cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(32 * s.warps * s.groups), args,
+                                     chip_smem_bytes(s.groups, s.warps, s.rows), stream);
 }
 
 cudaError_t launch_grid_barrier_check(unsigned* gbar, int blocks, int missing, int rounds,

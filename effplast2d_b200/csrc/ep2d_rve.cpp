@@ -319,6 +319,19 @@ size_t n_samples(const ep2d_params& p) {
   return (size_t)(k * k * 20);
 }
 
+// the on-chip form's shape for an RVE: only where the parameters leave the kernel to the library
+ChipShape chip_of(const ep2d_params& p) {
+  return p.kernel == EP2D_KERNEL_AUTO && p.rows == 0 ? chip_shape(p.nx, p.ny) : ChipShape{};
+}
+
+// On-chip launches of different handles take turns on a device: their CTAs wait on one another, so
+// two such grids that each found room for only part of their CTAs would wait for each other
+// until their waits ran out.  Held from the launch to its completion.
+std::mutex& chip_turn(int dev) {
+  static std::mutex mu[64];
+  return mu[dev & 63];
+}
+
 std::mutex g_prep_mu;
 std::set<int> g_prepared;
 }  // namespace
@@ -340,6 +353,7 @@ size_t Rve::footprint(const ep2d_params& p) {
   b += align256(partial_elems(p) * sizeof(double));      // averaging partials
   b += align256((2 * NAVG + n_samples(p) + 4) * sizeof(double));  // sums, samples, vmax, barrier
   b += align256(n_samples(p) * sizeof(unsigned long long));
+  b += align256(chip_rim_bytes(chip_of(p)));             // rim records of the on-chip form
   return b;
 }
 
@@ -479,6 +493,9 @@ int Rve::create(const ep2d_params& p, cudaStream_t s) {
   f.gbar = reinterpret_cast<unsigned*>(d_out + 2 * NAVG + holes.size() + 2);  // zeroed above, never reset
   cp += align256((2 * NAVG + n_samples(p) + 4) * sizeof(double));
   d_idx = reinterpret_cast<unsigned long long*>(cp);
+  cp += align256(n_samples(p) * sizeof(unsigned long long));
+  d_rim = cp;
+  chip = sms >= CHIP_SMS ? chip_of(p) : ChipShape{};
 
   EP2D_CK(cudaMallocHost(&h_pin, (2 * NAVG + holes.size() + 2) * sizeof(double) + 64));
   std::vector<unsigned long long> codes(holes.size());
@@ -602,7 +619,39 @@ int Rve::capture(int parity) {
   return EP2D_OK;
 }
 
+// n plain iterations in one launch of the on-chip form; *done = false where the device has no
+// room for its CTAs (the other forms take over for good).
+int Rve::run_chip(int64_t n, bool* done) {
+  std::lock_guard<std::mutex> turn(chip_turn(device));
+  *done = true;
+  while (n > 0) {
+    // chunks of an even length keep the parity; a chunk of one iteration cannot arise
+    const int64_t chunk = n > ((int64_t)1 << 30) ? (int64_t)1 << 29 : n;
+    const cudaError_t e = launch_iter_chip(g, f, cur, prm.nl > 1, mixed(), chip, (int)chunk, chip_tag, d_rim,
+                                           CHIP_TIMEOUT_NS, stream);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+      cudaGetLastError();
+      chip = ChipShape{};
+      *done = false;
+      return EP2D_OK;
+    }
+    EP2D_CK(e);
+    chip_tag += (uint32_t)chunk;
+    cur ^= (int)(chunk & 1);
+    launches++;
+    resident_launches++;
+    n -= chunk;
+  }
+  EP2D_CK(cudaStreamSynchronize(stream));
+  return EP2D_OK;
+}
+
 int Rve::run_plain(int64_t n) {
+  if (chip.warps && n >= CHIP_MIN_RUN && !f32 && !track) {
+    bool done = false;
+    const int rc = run_chip(n, &done);
+    if (rc || done) return rc;
+  }
   if (shape.form == FORM_RESIDENT && !f32 && !track) {
     // one cooperative launch for all n iterations (n == 1: an ordinary tile launch)
     if (n > 1) {
@@ -667,8 +716,8 @@ double Rve::error_from_vmax(double vmx, double vmy) const {
   return (vmx / (d.dX * (prm.nx - 1)) + vmy / (d.dY * (prm.ny - 1))) * d.dT / std::max(a, b);
 }
 
-// The resident form's barrier error flag (sticky), read back; EP2D_OK if the RVE never
-// ran that form.
+// The error flag of the forms whose CTAs wait on one another (sticky), read back; EP2D_OK if
+// the RVE never ran one.
 int Rve::check_resident() {
   if (!resident_launches) return EP2D_OK;
   unsigned* hf = reinterpret_cast<unsigned*>(h_pin + 2 * NAVG + holes.size() + 2);
@@ -676,7 +725,7 @@ int Rve::check_resident() {
   EP2D_CK(cudaStreamSynchronize(stream));
   if (*hf)
     return fail(EP2D_ERR_CUDA,
-                "resident form: a grid barrier wait ran out (a CTA did not arrive); the RVE's state is invalid");
+                "resident or on-chip form: a wait for another CTA ran out; the RVE's state is invalid");
   return EP2D_OK;
 }
 

@@ -102,7 +102,7 @@ class Rve {
   int iterate(int64_t n, bool record_last);  // n iterations; the last one records stresses
   int launch_one(bool record);                // one iteration kernel (no stats)
   int reset_vmax();
-  int check_resident();  // the resident form's barrier error flag (sticky)
+  int check_resident();  // the error flag of the forms with bounded waits (sticky)
   int read_error(double* error);              // after a recording launch: D2H + error formula
   int finish_time_step(int step, int it);     // averaging etc. into the record
   double error_from_vmax(double vmx, double vmy) const;
@@ -122,6 +122,11 @@ class Rve {
   Geo g{};
   Fields f{};
   IterShape shape{};  // form and rows of the iteration kernel (shape_of(prm))
+  // runs of plain iterations in the on-chip form (warps == 0: not taken): the library's
+  // choice (EP2D_KERNEL_AUTO, rows 0) on grids that fit on chip
+  ChipShape chip{};
+  void* d_rim = nullptr;   // its rim records
+  uint32_t chip_tag = 1;   // the next unused record tag
   // velocities stored in FP32 (the mixed path, and both phases of the FP32 bulk)
   bool mixed() const { return prm.precision == EP2D_MIXED || prm.precision == EP2D_F32_BULK; }
   // FP32 bulk: true while the state is in its FP32 form (u' in f.ux32/uy32)
@@ -154,7 +159,7 @@ class Rve {
   // statistics
   double kernel_ms = 0.0;
   int64_t launches = 0;      // fused iteration kernel (a resident launch counts once)
-  int64_t resident_launches = 0;  // of them, resident-form launches
+  int64_t resident_launches = 0;  // of them, resident-form and on-chip launches (bounded waits)
   int64_t aux_launches = 0;  // preload, averaging, boundary, gather, mask
   int64_t cell_updates = 0;
 
@@ -168,6 +173,7 @@ class Rve {
 
  private:
   int run_plain(int64_t n);
+  int run_chip(int64_t n, bool* done);
   int capture(int parity);
   cudaGraphExec_t gexec_[2] = {nullptr, nullptr};
   cudaGraphExec_t gexec32_[2] = {nullptr, nullptr};  // FP32 bulk (hold the affine strains)

@@ -108,6 +108,24 @@ constexpr unsigned long long RESIDENT_TIMEOUT_NS = 2000000000ull;  // 2 s per ba
 // out[0] = CTAs that passed all `rounds`; gbar (4 words) zeroed first
 cudaError_t launch_grid_barrier_check(unsigned* gbar, int blocks, int missing, int rounds,
                                       unsigned long long timeout_ns, unsigned* out, cudaStream_t stream);
+// The on-chip form (ep2d_iter_chip.cuh): ncx x ncy tiles of STREAM_COLS columns x (warps x
+// rows) rows, `groups` tiles to a CTA, one CTA per SM, all resident at once.  warps == 0:
+// the grid does not fit on chip.
+struct ChipShape {
+  int warps = 0, rows = 0, groups = 0, ncx = 0, ncy = 0;
+};
+constexpr int CHIP_SMS = 148;    // SMs of a B200
+constexpr int CHIP_WARPS = 16;   // warps per CTA: 128 registers per thread
+constexpr int CHIP_SMEM = 226 * 1024;
+constexpr unsigned long long CHIP_TIMEOUT_NS = 10000000000ull;  // 10 s per wait
+constexpr int CHIP_MIN_RUN = 8;  // shorter runs of plain iterations are launched one by one
+ChipShape chip_shape(int nx, int ny);
+// bytes of the rim records of a shape (zeroed when the RVE is created)
+size_t chip_rim_bytes(const ChipShape& s);
+// n_iter >= 2 plain iterations of one RVE from buffer src in one cooperative launch; `tag`:
+// a number the RVE's earlier launches have not used (they used n_iter numbers from theirs on)
+cudaError_t launch_iter_chip(const Geo& g, const Fields& f, int src, bool plastic, bool mixed, const ChipShape& s,
+                             int n_iter, uint32_t tag, void* rim, unsigned long long timeout_ns, cudaStream_t stream);
 // clear the M_YN / M_YC bits of every node
 cudaError_t launch_clear_track(const Geo& g, uint8_t* mask, cudaStream_t stream);
 // one iteration of the FP32 bulk (stream form, segments of seg_h rows): u' and V in

@@ -63,7 +63,10 @@ enum {
   EP2D_KERNEL_AUTO = 0,   /* the library's choice (the stream form, segments of 4 to 64
                              rows by grid size; the tile form for grids too small to occupy
                              the GPU even with 4-row segments, the resident form for small
-                             elastic ones; batches: timed) */
+                             elastic ones; batches: timed).  A single RVE whose grid fits
+                             on chip (up to about 1080^2) runs the plain iterations between
+                             two recording launches in one cooperative launch with its
+                             state held on the SMs; handles take turns for such launches */
   EP2D_KERNEL_TILE = 1,   /* one CTA per 32-column x `rows`-row tile, stencil halos in
                              shared memory; rows 8, 16 or 32 */
   EP2D_KERNEL_STREAM = 2, /* one warp per 28-column strip segment of `rows` rows, marching
@@ -387,8 +390,8 @@ int ep2d_average_fields_noalloc(int32_t nx, int32_t ny, const double pa[EP2D_NPA
 int ep2d_abi_sizes(int64_t* out, int32_t n);
 
 /* Counters of this handle since creation: device time of the iteration loops measured
- * with CUDA events on the handle's stream (ms), launches of the fused iteration kernel,
- * cell updates (nx*ny per iteration), and all kernel launches (iteration kernel plus
+ * with CUDA events on the handle's stream (ms), launches of the fused iteration kernel
+ * (a launch of many iterations counts once), cell updates (nx*ny per iteration), and all kernel launches (iteration kernel plus
  * preload, reductions and gathers).  Any pointer may be NULL. */
 int ep2d_get_stats(ep2d_handle* h, double* kernel_ms, int64_t* iter_launches, int64_t* cell_updates,
                    int64_t* all_launches);
@@ -403,7 +406,9 @@ int ep2d_iterate_f32(ep2d_handle* h, int64_t n_iter);
 int ep2d_get_f32_iterations(ep2d_handle* h, int64_t* f32_iterations);
 /* The iteration kernel this handle launches: EP2D_KERNEL_TILE, EP2D_KERNEL_STREAM or
  * EP2D_KERNEL_RESIDENT and its rows per tile / strip segment (the parameters' choice, or
- * the library's).  No counterpart in the reference. */
+ * the library's; for EP2D_KERNEL_AUTO that of its single launches, the runs of plain
+ * iterations of a grid that fits on chip having a form of their own).  No counterpart in
+ * the reference. */
 int ep2d_get_kernel_shape(ep2d_handle* h, int32_t* kernel, int32_t* rows);
 /* The resident form's grid barrier on its own, for checking its failure path without a
  * fault: one cooperative launch of `blocks` CTAs (all resident at once) on `device`

@@ -1,0 +1,72 @@
+"""The on-chip form: a run of plain iterations in one launch, the state on the SMs.
+
+The library takes it (kernel AUTO) for runs of 8 plain iterations or more on grids that fit on chip.
+It evaluates the same per-cell formulas as the other forms, so every field must
+equal the stream form's bit for bit.  The grids sit at the edges of its split: one tile,
+one column or row past a 28-column strip or a tile of rows, the widest and tallest that
+fit at a given number of rows per warp (2 to 18), and the first that does not fit.
+"""
+import threading
+
+import numpy as np
+import pytest
+
+import effplast2d_b200 as ep
+from test_gpu_kernels import FIELDS, PLASTIC_FIELDS, _pa, _random_state
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(nx, ny, pa, nl, st, counts, precision, **kw):
+    s = ep.Solver(nx, ny, pa, nl=nl, precision=precision, **kw)
+    for k, v in st.items():
+        s.set(k, v)
+    for n in counts:
+        s.iterate(n)
+    out = {f: s.get(f) for f in FIELDS + (PLASTIC_FIELDS if nl > 1 else [])}
+    launches = s.stats()["launches"]
+    s.close()
+    return out, launches
+
+
+# (8, 8): one tile, smaller than it in both directions; 28, 29, 57: strips of 28 columns and
+# one column over; rows 2 to 18 per warp (chip_shape: 128^2 2, 400^2 4, 520^2 6, 700^2 10, 1024^2 16,
+# 1060^2 18); 1100^2 does not fit and stays with the stream form
+GRIDS = [(8, 8), (28, 17), (29, 9), (57, 130), (128, 128), (301, 203), (403, 401), (521, 517), (64, 2047), (2047, 64),
+         (700, 699), (1024, 1024), (1061, 1060), (1100, 1100)]
+
+
+@pytest.mark.parametrize("nx,ny", GRIDS, ids=["%dx%d" % g for g in GRIDS])
+@pytest.mark.parametrize("nl,precision", [(1, ep.FP64), (3, ep.FP64), (2, ep.MIXED)], ids=["elastic", "plastic", "mixed"])
+def test_chip_form_matches_stream_form(nx, ny, nl, precision):
+    pa = _pa(nx, ny, n_pores=2, porosity=0.03, yield_stress=1e-5)
+    st = _random_state(nx, ny, 41)
+    counts = (9, 1, 30, 33)  # runs of 8, 29 and 32 plain iterations: both parities
+    a, la = _run(nx, ny, pa, nl, st, counts, precision, kernel=ep.KERNEL_STREAM, rows=16)
+    b, lb = _run(nx, ny, pa, nl, st, counts, precision)
+    for f in a:
+        assert np.array_equal(b[f], a[f], equal_nan=True), (f, float(np.nanmax(np.abs(b[f] - a[f]))))
+    assert la == 73
+    if max(nx, ny) < 1100 or min(nx, ny) == 64:
+        assert lb == 7  # three on-chip launches, four recording ones
+
+
+def test_chip_form_two_threads():
+    # on-chip launches of different handles take turns; both finish with the single-thread result
+    nx = ny = 200
+    pa = _pa(nx, ny, n_pores=3, porosity=0.02, yield_stress=1e-5)
+    sts = [_random_state(nx, ny, 50 + k) for k in range(2)]
+    want = [_run(nx, ny, pa, 3, st, (400,), ep.FP64)[0] for st in sts]
+    got = [None, None]
+
+    def work(k):
+        got[k] = _run(nx, ny, pa, 3, sts[k], (100,) * 4, ep.FP64)[0]
+
+    ths = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in ths:
+        t.start()
+    for t in ths:
+        t.join()
+    for k in range(2):
+        for f in ("Ux", "Uy", "Vx", "Vy"):
+            assert np.array_equal(got[k][f], want[k][f]), (k, f)
