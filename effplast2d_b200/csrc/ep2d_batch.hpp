@@ -85,6 +85,13 @@ class BatchEngine {
   int run_solo_launches(int slot);     // one checkpoint interval through the single-RVE path
   void finish_interval(const std::vector<char>& batched);  // every active RVE's checkpoint
   int autotune(int64_t* k, int64_t n_avail);
+  // on-chip launches of the batched RVEs: a wave is the RVEs of one launch and its shape
+  struct Wave {
+    std::vector<int> slots;
+    ChipShape shape;
+  };
+  bool plan_waves(const std::vector<char>& batched);  // false: the batched launches are faster
+  int run_waves(int64_t n, bool* done);               // n plain iterations of every RVE of the waves
   int grow(int need);
 
   std::vector<Slot> slots_;
@@ -98,6 +105,12 @@ class BatchEngine {
   unsigned long long* d_vmax_ = nullptr;
   unsigned long long* h_vmax_ = nullptr;
   int cap_slots_ = 0, cap_tiles_ = 0;
+  std::vector<Wave> waves_;
+  uint64_t waves_version_ = ~0ull;  // set_version_ they were planned for
+  bool use_waves_ = false;
+  bool waves_ok_ = true;            // false: the device has no room for their CTAs
+  unsigned* d_flag_ = nullptr;      // error flag of the on-chip launches
+  unsigned* h_flag_ = nullptr;
   uint64_t set_version_ = 0;    // bumped whenever an RVE joins or retires
   uint64_t tuned_version_ = 0;  // set_version_ the current shape was tuned for
   cudaGraphExec_t graph_ = nullptr;

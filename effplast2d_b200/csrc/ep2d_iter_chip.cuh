@@ -18,7 +18,7 @@
 // vector store and is valid on its own).  Records are double-buffered by iteration parity: a CTA
 // overwrites iteration t's records in iteration t + 2, after it has read its neighbours'
 // records of t + 1, which they wrote after reading all of t's.  Waits are bounded: a CTA that
-// waits longer than timeout_ns sets the RVE's error flag (gbar[2]) and leaves, the others
+// waits longer than timeout_ns sets its RVE's error flag and leaves, the others
 // follow, and the host reports the RVE as failed.
 //
 // Within a CTA the two lowest and two highest rows of a warp are read by the warps below
@@ -327,27 +327,32 @@ __device__ __forceinline__ void chip_march(const Geo& g, const ChipMat* __restri
   tmem_st_wait();
 }
 
-// n_iter plain iterations of one RVE from buffer `src`, ending in buffer src ^ (n_iter & 1)
-// (n_iter >= 2: when the buffers coincide, a CTA writes back only after its neighbours have
-// read it).  blockDim.x / 32 warps of `rows` rows each (even); grid = ncx tiles per row of
-// tiles x the tile rows.  rim: records [2][CTA][4 H + 112 cells][2].
-template <bool PLASTIC, typename TV>
-__global__ void __launch_bounds__(512, 1) k_iter_chip(Geo g, Fields f, int src, int n_iter, int nw, int rows, int ncx,
-                                                      int ncy, uint32_t tag0, char* rim,
-                                                      unsigned long long timeout_ns) {
+// a.n_iter plain iterations of every job's RVE from its buffer `src`, ending in buffer
+// src ^ (n_iter & 1) (n_iter >= 2: when the buffers coincide, a tile is written back only after
+// its neighbours have read it).  CTAs of groups of a.warps warps, a group per tile, a.rows rows per
+// warp.  rim: records [2][tile][4 H + 112 cells].  PLASTIC 0, 1: all jobs; 2: per job.
+template <int PLASTIC, int JOBS, typename TV>
+__global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_constant__ ChipArgs<JOBS> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t s_tmem;
+  int jb = 0;
+  if (JOBS > 1)
+    while (jb + 1 < a.njobs && (int)blockIdx.x >= a.job[jb + 1].cta0) jb++;
+  const ChipJob& job = a.job[jb];
+  const Geo& g = job.g;
+  const Fields& f = job.f;
+  const int nw = a.warps, rows = a.rows, n_iter = a.n_iter, ncx = job.ncx, ncy = job.ncy, src = job.src;
   const int lane = threadIdx.x & 31, wc = threadIdx.x >> 5;  // warp of the CTA
   const int group = wc / nw, w = wc - group * nw;             // its group, warp of the group
   const int groups = (int)(blockDim.x >> 5) / nw;
-  const int tile = blockIdx.x * groups + group;
+  const int tile = ((int)blockIdx.x - job.cta0) * groups + group;
   const bool idle = tile >= ncx * ncy;
   const int cx = tile % ncx, cy = tile / ncx;
   const int nx = g.nx, ny = g.ny, pitch = g.pitch;
   const int H = nw * rows, x0 = STREAM_COLS * cx, y0 = H * cy;
   const int npairs = rows / 2, ppw = chip_pairs_per_warp(rows);
   const int ncol = chip_col_polls(rows), npoll = chip_polls(nw, rows);
-  if (__syncthreads_or(*reinterpret_cast<volatile unsigned*>(f.gbar + 2) != 0)) return;  // an earlier launch failed
+  if (__syncthreads_or(*reinterpret_cast<volatile unsigned*>(job.flag) != 0)) return;  // an earlier launch failed
 
   ChipMat* mats = reinterpret_cast<ChipMat*>(smem_raw);
   char* urows = reinterpret_cast<char*>(smem_raw) + CHIP_MATS * sizeof(ChipMat) + group * chip_group_bytes(nw, rows);
@@ -463,14 +468,19 @@ __global__ void __launch_bounds__(512, 1) k_iter_chip(Geo g, Fields f, int src, 
         const char* below = rd_below + par * CHIP_PAIR;
         const char* above = rd_above + par * CHIP_PAIR;
         const uint8_t* ix = idx + (w * rows) * 32;
-        if (interior) chip_march<PLASTIC, false, TV>(g, mats, ix, below, own, above, npairs, par, i, jA, vmem);
-        else chip_march<PLASTIC, true, TV>(g, mats, ix, below, own, above, npairs, par, i, jA, vmem);
+        auto march = [&](auto plastic_c) {
+          constexpr bool P = decltype(plastic_c)::value;
+          if (interior) chip_march<P, false, TV>(g, mats, ix, below, own, above, npairs, par, i, jA, vmem);
+          else chip_march<P, true, TV>(g, mats, ix, below, own, above, npairs, par, i, jA, vmem);
+        };
+        if (PLASTIC == 1 || (PLASTIC == 2 && job.plastic)) march(std::true_type{});
+        else march(std::false_type{});
       }
       if (it + 1 >= n_iter) break;
       __syncwarp();
-      const uint32_t tag = tag0 + (uint32_t)it;
-      char* out = rim + par * rim_parity + (size_t)tile * cells * RIM_BYTES;
-      const char* in = rim + par * rim_parity;
+      const uint32_t tag = job.tag + (uint32_t)it;
+      char* out = job.rim + par * rim_parity + (size_t)tile * cells * RIM_BYTES;
+      const char* in = job.rim + par * rim_parity;
       auto put = [&](int cell, int r, int col) {
         rim_put(out + cell * RIM_BYTES,
                 reinterpret_cast<const double2*>(own + chip_pair_off(r >> 1, npairs, par ^ 1))[(r & 1) * 32 + col], tag);
@@ -503,8 +513,8 @@ __global__ void __launch_bounds__(512, 1) k_iter_chip(Geo g, Fields f, int src, 
             if ((++tries & 1023u) == 0) {  // bounded: look at the clock and the error flag now and then
               const unsigned long long now = global_ns();
               if (since == 0) since = now;
-              if (now - since > timeout_ns) atomicExch(&f.gbar[2], 1u);
-              if (*reinterpret_cast<volatile unsigned*>(f.gbar + 2)) {
+              if (now - since > a.timeout_ns) atomicExch(job.flag, 1u);
+              if (*reinterpret_cast<volatile unsigned*>(job.flag)) {
                 failed = 1;
                 break;
               }

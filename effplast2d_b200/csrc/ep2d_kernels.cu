@@ -118,17 +118,23 @@ int occupancy_ty(bool record) {
   return e == cudaSuccess && n > 0 ? n : 1;
 }
 
-template <bool PLASTIC, typename TV>
+template <int PLASTIC, int JOBS, typename TV>
 cudaError_t set_chip_attr() {
-  return cudaFuncSetAttribute(k_iter_chip<PLASTIC, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, CHIP_SMEM);
+  return cudaFuncSetAttribute(k_iter_chip<PLASTIC, JOBS, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, CHIP_SMEM);
+}
+
+template <typename TV>
+cudaError_t set_chip_attrs() {
+  cudaError_t e;
+  if ((e = set_chip_attr<0, 1, TV>()) != cudaSuccess) return e;
+  if ((e = set_chip_attr<1, 1, TV>()) != cudaSuccess) return e;
+  return set_chip_attr<2, CHIP_JOBS, TV>();
 }
 
 cudaError_t prepare_kernels_impl() {
   cudaError_t e;
-  if ((e = set_chip_attr<false, double>()) != cudaSuccess) return e;
-  if ((e = set_chip_attr<true, double>()) != cudaSuccess) return e;
-  if ((e = set_chip_attr<false, float>()) != cudaSuccess) return e;
-  if ((e = set_chip_attr<true, float>()) != cudaSuccess) return e;
+  if ((e = set_chip_attrs<double>()) != cudaSuccess) return e;
+  if ((e = set_chip_attrs<float>()) != cudaSuccess) return e;
   if ((e = set_attrs_ty<8, double>()) != cudaSuccess) return e;
   if ((e = set_attrs_ty<16, double>()) != cudaSuccess) return e;
   if ((e = set_attrs_ty<32, double>()) != cudaSuccess) return e;
@@ -285,26 +291,59 @@ ChipShape chip_shape(int nx, int ny) {
   return best;
 }
 
-size_t chip_rim_bytes(const ChipShape& s) {
-  return (size_t)2 * s.ncx * s.ncy * (4 * s.warps * s.rows + 4 * STREAM_COLS) * RIM_BYTES;
+// The tallest tiles a launch may use are CHIP_WARPS warps x 18 rows, the shortest those of the
+// grid's own shape: 4 records per row of padded height and 4 x STREAM_COLS per tile.
+size_t chip_rim_bytes(int nx, int ny) {
+  const ChipShape s = chip_shape(nx, ny);
+  if (!s.warps) return 0;
+  return (size_t)2 * RIM_BYTES * s.ncx * (4 * ((size_t)ny + CHIP_WARPS * 18) + 4 * STREAM_COLS * (size_t)s.ncy);
 }
 
-cudaError_t launch_iter_chip(const Geo& g, const Fields& f, int src, bool plastic, bool mixed, const ChipShape& s,
-                             int n_iter, uint32_t tag, void* rim, unsigned long long timeout_ns, cudaStream_t stream) {
-  if (n_iter < 2 || s.warps < 1 || s.groups < 1 || s.warps * s.groups > 16 || s.rows < 2 || (s.rows & 1) || !f.gbar || !rim)
-    return cudaErrorInvalidValue;
-  const void* kern = mixed ? (plastic ? (const void*)k_iter_chip<true, float> : (const void*)k_iter_chip<false, float>)
-                           : (plastic ? (const void*)k_iter_chip<true, double> : (const void*)k_iter_chip<false, double>);
-  Geo ga = g;
-  Fields fa = f;
-  int srca = src, na = n_iter, nw = s.warps, rows = s.rows, ncx = s.ncx, ncy = s.ncy;
-  uint32_t ta = tag;
-  char* ra = static_cast<char*>(rim);
-  unsigned long long to = timeout_ns;
-  void* args[] = {&ga, &fa, &srca, &na, &nw, &rows, &ncx, &ncy, &ta, &ra, &to};
-  const int blocks = (s.ncx * s.ncy + s.groups - 1) / s.groups;
+int chip_ctas(int nx, int ny, int groups, int warps, int rows) {
+  const int ncx = (nx + STREAM_COLS - 1) / STREAM_COLS, ncy = (ny + warps * rows - 1) / (warps * rows);
+  return (ncx * ncy + groups - 1) / groups;
+}
+size_t chip_smem(int groups, int warps, int rows) { return chip_smem_bytes(groups, warps, rows); }
+
+namespace {
+template <int JOBS>
+cudaError_t launch_chip_jobs(const ChipJob* jobs, int njobs, const void* kern, const ChipShape& s, int n_iter, int blocks,
+                             unsigned long long timeout_ns, cudaStream_t stream) {
+  ChipArgs<JOBS> a;
+  a.njobs = njobs;
+  a.warps = s.warps;
+  a.rows = s.rows;
+  a.n_iter = n_iter;
+  a.timeout_ns = timeout_ns;
+  std::copy(jobs, jobs + njobs, a.job);
+  void* args[] = {&a};
   return cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(32 * s.warps * s.groups), args,
                                      chip_smem_bytes(s.groups, s.warps, s.rows), stream);
+}
+}  // namespace
+
+cudaError_t launch_iter_chip(ChipJob* jobs, int njobs, bool mixed, const ChipShape& s, int n_iter,
+                             unsigned long long timeout_ns, cudaStream_t stream) {
+  if (njobs < 1 || njobs > CHIP_JOBS || n_iter < 2 || s.warps < 1 || s.groups < 1 ||
+      s.warps * s.groups > CHIP_WARPS || s.rows < 2 || s.rows > 18 || (s.rows & 1))
+    return cudaErrorInvalidValue;
+  int blocks = 0;
+  for (int k = 0; k < njobs; k++) {
+    ChipJob& j = jobs[k];
+    if (!j.rim || !j.flag) return cudaErrorInvalidValue;
+    j.ncx = (j.g.nx + STREAM_COLS - 1) / STREAM_COLS;
+    j.ncy = (j.g.ny + s.warps * s.rows - 1) / (s.warps * s.rows);
+    j.cta0 = blocks;
+    blocks += (j.ncx * j.ncy + s.groups - 1) / s.groups;
+  }
+  if (njobs == 1) {
+    const bool pl = jobs[0].plastic != 0;
+    const void* kern = mixed ? (pl ? (const void*)k_iter_chip<1, 1, float> : (const void*)k_iter_chip<0, 1, float>)
+                             : (pl ? (const void*)k_iter_chip<1, 1, double> : (const void*)k_iter_chip<0, 1, double>);
+    return launch_chip_jobs<1>(jobs, 1, kern, s, n_iter, blocks, timeout_ns, stream);
+  }
+  const void* kern = mixed ? (const void*)k_iter_chip<2, CHIP_JOBS, float> : (const void*)k_iter_chip<2, CHIP_JOBS, double>;
+  return launch_chip_jobs<CHIP_JOBS>(jobs, njobs, kern, s, n_iter, blocks, timeout_ns, stream);
 }
 
 cudaError_t launch_grid_barrier_check(unsigned* gbar, int blocks, int missing, int rounds,

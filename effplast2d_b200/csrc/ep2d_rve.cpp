@@ -319,22 +319,17 @@ size_t n_samples(const ep2d_params& p) {
   return (size_t)(k * k * 20);
 }
 
-// the on-chip form's shape for an RVE: only where the parameters leave the kernel to the library
-ChipShape chip_of(const ep2d_params& p) {
-  return p.kernel == EP2D_KERNEL_AUTO && p.rows == 0 ? chip_shape(p.nx, p.ny) : ChipShape{};
-}
-
-// On-chip launches of different handles take turns on a device: their CTAs wait on one another, so
-// two such grids that each found room for only part of their CTAs would wait for each other
-// until their waits ran out.  Held from the launch to its completion.
-std::mutex& chip_turn(int dev) {
-  static std::mutex mu[64];
-  return mu[dev & 63];
-}
+// the on-chip form is taken only where the parameters leave the kernel to the library
+bool chip_allowed(const ep2d_params& p) { return p.kernel == EP2D_KERNEL_AUTO && p.rows == 0; }
 
 std::mutex g_prep_mu;
 std::set<int> g_prepared;
 }  // namespace
+
+std::mutex& chip_turn(int dev) {
+  static std::mutex mu[64];
+  return mu[dev & 63];
+}
 
 int prepare_device(int dev) {
   std::lock_guard<std::mutex> lk(g_prep_mu);
@@ -353,7 +348,7 @@ size_t Rve::footprint(const ep2d_params& p) {
   b += align256(partial_elems(p) * sizeof(double));      // averaging partials
   b += align256((2 * NAVG + n_samples(p) + 4) * sizeof(double));  // sums, samples, vmax, barrier
   b += align256(n_samples(p) * sizeof(unsigned long long));
-  b += align256(chip_rim_bytes(chip_of(p)));             // rim records of the on-chip form
+  if (chip_allowed(p)) b += align256(chip_rim_bytes(p.nx, p.ny));  // rim records of the on-chip form
   return b;
 }
 
@@ -495,7 +490,7 @@ int Rve::create(const ep2d_params& p, cudaStream_t s) {
   d_idx = reinterpret_cast<unsigned long long*>(cp);
   cp += align256(n_samples(p) * sizeof(unsigned long long));
   d_rim = cp;
-  chip = sms >= CHIP_SMS ? chip_of(p) : ChipShape{};
+  chip = chip_allowed(p) && sms >= CHIP_SMS ? chip_shape(p.nx, p.ny) : ChipShape{};
 
   EP2D_CK(cudaMallocHost(&h_pin, (2 * NAVG + holes.size() + 2) * sizeof(double) + 64));
   std::vector<unsigned long long> codes(holes.size());
@@ -619,6 +614,19 @@ int Rve::capture(int parity) {
   return EP2D_OK;
 }
 
+ChipJob Rve::chip_job(int n, unsigned* flag) {
+  ChipJob j{};
+  j.g = g;
+  j.f = f;
+  j.rim = d_rim;
+  j.flag = flag;
+  j.src = cur;
+  j.plastic = prm.nl > 1 ? 1 : 0;
+  j.tag = chip_tag;
+  chip_tag += (uint32_t)n;
+  return j;
+}
+
 // n plain iterations in one launch of the on-chip form; *done = false where the device has no
 // room for its CTAs (the other forms take over for good).
 int Rve::run_chip(int64_t n, bool* done) {
@@ -627,8 +635,8 @@ int Rve::run_chip(int64_t n, bool* done) {
   while (n > 0) {
     // chunks of an even length keep the parity; a chunk of one iteration cannot arise
     const int64_t chunk = n > ((int64_t)1 << 30) ? (int64_t)1 << 29 : n;
-    const cudaError_t e = launch_iter_chip(g, f, cur, prm.nl > 1, mixed(), chip, (int)chunk, chip_tag, d_rim,
-                                           CHIP_TIMEOUT_NS, stream);
+    ChipJob job = chip_job((int)chunk, f.gbar + 2);
+    const cudaError_t e = launch_iter_chip(&job, 1, mixed(), chip, (int)chunk, CHIP_TIMEOUT_NS, stream);
     if (e == cudaErrorCooperativeLaunchTooLarge) {
       cudaGetLastError();
       chip = ChipShape{};
@@ -636,7 +644,6 @@ int Rve::run_chip(int64_t n, bool* done) {
       return EP2D_OK;
     }
     EP2D_CK(e);
-    chip_tag += (uint32_t)chunk;
     cur ^= (int)(chunk & 1);
     launches++;
     resident_launches++;

@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -62,6 +63,11 @@ IterShape shape_of(const ep2d_params& p, int sm_count = 0);
 // Device row pitch (elements) for an nx-wide grid.
 int row_pitch(int nx);
 
+// On-chip launches of different handles take turns on a device: their CTAs wait on one
+// another, so two such grids that each found room for only part of their CTAs would wait for
+// each other until their waits ran out.  Held from the launch to its completion.
+std::mutex& chip_turn(int dev);
+
 // Per-device kernel attributes, once per device (the device must be current).
 int prepare_device(int dev);
 
@@ -106,6 +112,9 @@ class Rve {
   int read_error(double* error);              // after a recording launch: D2H + error formula
   int finish_time_step(int step, int it);     // averaging etc. into the record
   double error_from_vmax(double vmx, double vmy) const;
+  // this RVE as a job of an on-chip launch of n iterations (its tags are then used); the
+  // launch flips `cur` by n & 1 when it has been made
+  ChipJob chip_job(int n, unsigned* flag);
 
   int get_field(int field, double* host) const;
   int set_field(int field, const double* host);
@@ -125,7 +134,7 @@ class Rve {
   // runs of plain iterations in the on-chip form (warps == 0: not taken): the library's
   // choice (EP2D_KERNEL_AUTO, rows 0) on grids that fit on chip
   ChipShape chip{};
-  void* d_rim = nullptr;   // its rim records
+  char* d_rim = nullptr;   // its rim records
   uint32_t chip_tag = 1;   // the next unused record tag
   // velocities stored in FP32 (the mixed path, and both phases of the FP32 bulk)
   bool mixed() const { return prm.precision == EP2D_MIXED || prm.precision == EP2D_F32_BULK; }

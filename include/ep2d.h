@@ -192,7 +192,7 @@ typedef struct ep2d_batch_config {
 typedef struct ep2d_batch_stats {
   double kernel_ms;       /* device time of the iteration launches (CUDA events) */
   double wall_ms;
-  int64_t launches;       /* batched iteration launches */
+  int64_t launches;       /* iteration launches (an on-chip launch of many iterations counts once) */
   int64_t all_launches;   /* every kernel launched, post-processing included */
   int64_t cell_updates;   /* sum over RVEs of nx*ny per iteration */
   int32_t rows;           /* rows per tile / strip segment used */
@@ -326,8 +326,9 @@ int ep2d_polar_fields(ep2d_handle* h, double load_value, double* snu_rr, double*
 /* ---- batch ---------------------------------------------------------------------- */
 /* Solve n RVEs together: every RVE runs ComputeEffModuli's chain (EffPlast2D.cu:179-229)
  * with the reference's convergence test and checkpoint cadence; all active RVEs advance
- * in lockstep through one persistent batched kernel per iteration, captured in a CUDA
- * graph; finished RVEs retire at their checkpoint.  results[k] is what the reference
+ * in lockstep checkpoint intervals, side by side in on-chip launches of a whole interval
+ * (EP2D_KERNEL_AUTO, rows 0) or through one persistent batched kernel per iteration,
+ * captured in a CUDA graph; finished RVEs retire at their checkpoint.  results[k] is what the reference
  * binary would compute for specs[k].  Fails with EP2D_ERR_NOMEM if the RVEs do not fit
  * on the device at once (the server admits them progressively instead). */
 int ep2d_batch_solve(const ep2d_batch_config* cfg, const ep2d_rve_spec* specs, int32_t n,

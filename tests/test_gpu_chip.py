@@ -12,6 +12,7 @@ import numpy as np
 import pytest
 
 import effplast2d_b200 as ep
+from effplast2d_b200 import batch as B
 from test_gpu_kernels import FIELDS, PLASTIC_FIELDS, _pa, _random_state
 
 pytestmark = pytest.mark.gpu
@@ -70,3 +71,24 @@ def test_chip_form_two_threads():
     for k in range(2):
         for f in ("Ux", "Uy", "Vx", "Vy"):
             assert np.array_equal(got[k][f], want[k][f]), (k, f)
+
+
+@pytest.mark.parametrize("precision", [ep.FP64, ep.MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("sides", [[8 + 3 * (k % 20) for k in range(70)], [700, 640, 512, 300, 33]],
+                         ids=["more-than-a-launch-takes", "two-waves"])
+def test_batch_waves_match_stream_batch(sides, precision):
+    # on-chip waves (AUTO) against the batched stream launches (pinned shape), elastic and
+    # plastic RVEs side by side: equal results
+    specs = []
+    for k, n in enumerate(sides):
+        pa = ep.make_pa(20.0, 20.0, n, n, yield_stress=1e-5, porosity=0.005 + 0.0005 * (k % 7), n_pores=1)
+        specs.append(B.spec(n, pa, 1 + k % 3, 1, -6e-5, (1.0, 0.8, 0.3)))
+    kw = dict(niter=800, check_every=400, precision=precision)
+    a, _ = B.batch_solve(specs, kernel=ep.KERNEL_STREAM, rows=16, **kw)
+    b, _ = B.batch_solve(specs, **kw)
+    for x, y in zip(a, b):
+        assert x["total_iterations"] == y["total_iterations"]
+        for kind in ("num", "num_per", "an"):
+            for m in ("kphi", "kd", "g"):
+                u, v = x[kind][m], y[kind][m]
+                assert u == v or (np.isnan(u) and np.isnan(v)), (kind, m, u, v)
