@@ -428,7 +428,7 @@ int BatchEngine::run_waves(int64_t n, bool* done) {
     const int64_t chunk = n > ((int64_t)1 << 30) ? (int64_t)1 << 29 : n;
     for (const Wave& w : waves_) {
       jobs.clear();
-      for (int q : w.slots) jobs.push_back(slots_[q].rve->chip_job((int)chunk, d_flag_));
+      for (int q : w.slots) jobs.push_back(slots_[q].rve->chip_job(d_flag_));
       const cudaError_t e = launch_iter_chip(jobs.data(), (int)jobs.size(), cfg.precision == EP2D_MIXED, w.shape,
                                              (int)chunk, CHIP_TIMEOUT_NS, stream);
       if (e == cudaErrorCooperativeLaunchTooLarge && !*done) {  // no room for the CTAs here

@@ -63,8 +63,9 @@ __host__ __device__ constexpr size_t chip_group_bytes(int warps, int rows) {
   return (size_t)(warps * chip_pairs_per_warp(rows) + 4) * CHIP_PAIR + (size_t)(warps * rows + 4) * 32 +
          (size_t)warps * chip_polls(warps, rows) * 32 * sizeof(uint2);
 }
-__host__ __device__ constexpr size_t chip_smem_bytes(int groups, int warps, int rows) {
-  return CHIP_MATS * sizeof(ChipMat) + groups * chip_group_bytes(warps, rows);
+// with tracking, a byte of yield bits per (row, column) behind the groups' regions
+__host__ __device__ constexpr size_t chip_smem_bytes(int groups, int warps, int rows, bool track = false) {
+  return CHIP_MATS * sizeof(ChipMat) + groups * (chip_group_bytes(warps, rows) + (track ? warps * rows * 32 : 0));
 }
 
 // barrier of one group's threads that also ORs a flag over them
@@ -142,7 +143,7 @@ struct VPair<float> {
 // Record of a cell: {lo, tag, hi, tag} of Ux and of Uy, one 256-bit access.
 struct RimRecord {
   uint32_t w[8];
-  __device__ bool ready(uint32_t tag) const { return w[1] == tag && w[3] == tag && w[5] == tag && w[7] == tag; }
+  __device__ bool ready(uint32_t tag) const { return ((w[1] ^ tag) | (w[3] ^ tag) | (w[5] ^ tag) | (w[7] ^ tag)) == 0; }
   __device__ double2 value() const {
     return make_double2(__hiloint2double((int)w[2], (int)w[0]), __hiloint2double((int)w[6], (int)w[4]));
   }
@@ -174,11 +175,15 @@ __device__ __forceinline__ uint32_t chip_pair_off(int q, int npairs, int par) {
 // One iteration of one warp's rows jA .. jA + 2 npairs - 1 (copy `par` to copy par ^ 1).
 // rd0 / rdN: the row pairs below and above the warp's own; idx: material indices of row
 // jA - 2 on, 32 per row; vmem: tensor-memory address of the warp's V.
-template <bool PLASTIC, bool EDGE, typename TV>
+// NP: the number of row pairs where it is known (1 to 3: the march unrolled, so that its rows'
+// chains overlap: 256^2, 2 rows, 2.70 -> 2.54 us an iteration; 448^2, 4 rows, 3.76 -> 3.55; 512^2, 6
+// rows, 4.29 -> 4.07), else 0.
+template <bool PLASTIC, bool EDGE, int NP, typename TV, bool TRACK>
 __device__ __forceinline__ void chip_march(const Geo& g, const ChipMat* __restrict__ mats, const uint8_t* idx,
-                                           const char* rd0, char* own, const char* rdN, int npairs, int par, int i,
-                                           int jA, uint32_t vmem) {
+                                           const char* rd0, char* own, const char* rdN, int npairs_in, int par, int i,
+                                           int jA, uint32_t vmem, uint8_t* yielded) {
   constexpr int VW = sizeof(VPair<TV>) / 4;
+  const int npairs = NP ? NP : npairs_in;
   const int lane = threadIdx.x & 31;
   const int nx = g.nx, ny = g.ny;
   const int right = lane < 31 ? 1 : 0;
@@ -237,7 +242,9 @@ __device__ __forceinline__ void chip_march(const Geo& g, const ChipMat* __restri
 
   auto pair = [&](auto stage_c, int p, const char* rd, char* wr) {
     constexpr int STAGE = decltype(stage_c)::value;
-    __syncwarp();  // the other lanes have read the rows this step overwrites
+    // the other lanes have read the rows this step overwrites (with one or two pairs every
+    // row is double-buffered)
+    if (NP == 0 || NP > 2) __syncwarp();
     VPair<TV> v;
     if constexpr (STAGE == 2) tmem_ld(vmem + (p - 2) * VW, v.w);
     const double2* ra = reinterpret_cast<const double2*>(rd) + lane;
@@ -273,6 +280,14 @@ __device__ __forceinline__ void chip_march(const Geo& g, const ChipMat* __restri
           xr1 = mul_rn(x1, f1);
           yr1 = mul_rn(y1, f1);
           cw1 = mul_rn(c1, factor(m1, coh2x16, coh4));
+          if (TRACK) {  // J2 > coh from the trial stresses (get_sigma_2D.m:126-138); a corner inside the grid
+            uint8_t* yl = yielded + 2 * (p - 2) * 32 + lane;
+            const bool c_in = !EDGE || i < nx - 1;
+            const int b0 = (n0 > coh2 ? M_YN : 0) | (c_in && (!EDGE || ja < ny - 1) && m0 > coh2x16 ? M_YC : 0);
+            const int b1 = (n1 > coh2 ? M_YN : 0) | (c_in && (!EDGE || ja + 1 < ny - 1) && m1 > coh2x16 ? M_YC : 0);
+            yl[0] |= b0;
+            yl[32] |= b1;
+          }
         }
       }
       const double sx0 = sub_rn(xr0, pb), sy0 = sub_rn(yr0, pb), sx1 = sub_rn(xr1, p1), sy1 = sub_rn(yr1, p1);
@@ -320,7 +335,7 @@ __device__ __forceinline__ void chip_march(const Geo& g, const ChipMat* __restri
   };
   pair(std::integral_constant<int, 0>{}, 0, rd0, nullptr);
   pair(std::integral_constant<int, 1>{}, 1, own + chip_pair_off(0, npairs, par), nullptr);
-#pragma unroll kChipUnroll
+#pragma unroll (NP ? NP : kChipUnroll)
   for (int p = 2; p <= npairs + 1; p++)
     pair(std::integral_constant<int, 2>{}, p, p <= npairs ? own + chip_pair_off(p - 1, npairs, par) : rdN,
          own + chip_pair_off(p - 2, npairs, par ^ 1));
@@ -331,7 +346,8 @@ __device__ __forceinline__ void chip_march(const Geo& g, const ChipMat* __restri
 // src ^ (n_iter & 1) (n_iter >= 2: when the buffers coincide, a tile is written back only after
 // its neighbours have read it).  CTAs of groups of a.warps warps, a group per tile, a.rows rows per
 // warp.  rim: records [2][tile][4 H + 112 cells].  PLASTIC 0, 1: all jobs; 2: per job.
-template <int PLASTIC, int JOBS, typename TV>
+// TRACK: also mark the nodes and corners that yield at any of the iterations (M_YN, M_YC).
+template <int PLASTIC, int JOBS, typename TV, bool TRACK = false>
 __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_constant__ ChipArgs<JOBS> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t s_tmem;
@@ -360,6 +376,7 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
   char* halo_t = halo_b + 2 * CHIP_PAIR;  // the rows below and above the tile, two copies each
   uint8_t* idx = reinterpret_cast<uint8_t*>(halo_t + 2 * CHIP_PAIR);
   uint2* polls = reinterpret_cast<uint2*>(idx + (H + 4) * 32);
+  uint8_t* yielded = smem_raw + chip_smem_bytes(groups, nw, rows) + wc * rows * 32;  // TRACK only
 
   if (wc == 0) {  // one CTA per SM takes all of the SM's tensor memory
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
@@ -392,6 +409,8 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
       return u;
     };
     char* own = urows + w * ppw * CHIP_PAIR;
+    if (TRACK)
+      for (int r = 0; r < rows; r++) yielded[r * 32 + lane] = 0;
     for (int r = 0; r < rows; r++) {
       const double2 u = load_u(jA + r);
       for (int par = 0; par < 2; par++)
@@ -470,15 +489,24 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
         const uint8_t* ix = idx + (w * rows) * 32;
         auto march = [&](auto plastic_c) {
           constexpr bool P = decltype(plastic_c)::value;
-          if (interior) chip_march<P, false, TV>(g, mats, ix, below, own, above, npairs, par, i, jA, vmem);
-          else chip_march<P, true, TV>(g, mats, ix, below, own, above, npairs, par, i, jA, vmem);
+          auto rows_of = [&](auto np_c) {
+            constexpr int NP = decltype(np_c)::value;
+            if (interior)
+              chip_march<P, false, NP, TV, TRACK>(g, mats, ix, below, own, above, npairs, par, i, jA, vmem, yielded);
+            else
+              chip_march<P, true, NP, TV, TRACK>(g, mats, ix, below, own, above, npairs, par, i, jA, vmem, yielded);
+          };
+          if (npairs == 1) rows_of(std::integral_constant<int, 1>{});
+          else if (npairs == 2) rows_of(std::integral_constant<int, 2>{});
+          else if (npairs == 3) rows_of(std::integral_constant<int, 3>{});
+          else rows_of(std::integral_constant<int, 0>{});
         };
         if (PLASTIC == 1 || (PLASTIC == 2 && job.plastic)) march(std::true_type{});
         else march(std::false_type{});
       }
       if (it + 1 >= n_iter) break;
       __syncwarp();
-      const uint32_t tag = job.tag + (uint32_t)it;
+      const uint32_t tag = (uint32_t)it + 1;  // the records start as zeros
       char* out = job.rim + par * rim_parity + (size_t)tile * cells * RIM_BYTES;
       const char* in = job.rim + par * rim_parity;
       auto put = [&](int cell, int r, int col) {
@@ -495,32 +523,42 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
             if (lane < STREAM_COLS) put(4 * H + (2 + r) * STREAM_COLS + lane, rows - 2 + r, 2 + lane);
       }
       int failed = 0;
-      for (int t0 = 0; t0 < npoll && !failed; t0 += kRimInFlight) {  // records in flight per lane
+      for (int t0 = 0; t0 < npoll && !failed; t0 += kRimInFlight) {
         uint2 e[kRimInFlight];
         RimRecord rec[kRimInFlight];
+        bool wait[kRimInFlight];
 #pragma unroll
         for (int k = 0; k < kRimInFlight; k++) {
           e[k].x = 0xffffffffu;
           if (t0 + k < npoll) e[k] = polls[(w * npoll + t0 + k) * 32 + lane];
-          if (e[k].x != 0xffffffffu) rim_get(in + (size_t)e[k].x * RIM_BYTES, rec[k]);
+          wait[k] = e[k].x != 0xffffffffu;
         }
         unsigned tries = 0;
         unsigned long long since = 0;
+        for (;;) {
+          bool any = false;
+#pragma unroll
+          for (int k = 0; k < kRimInFlight; k++)
+            if (wait[k]) rim_get(in + (size_t)e[k].x * RIM_BYTES, rec[k]);
+#pragma unroll
+          for (int k = 0; k < kRimInFlight; k++) {
+            if (wait[k]) wait[k] = !rec[k].ready(tag);
+            any |= wait[k];
+          }
+          if (!__any_sync(0xffffffffu, any)) break;
+          if ((++tries & 1023u) == 0) {  // bounded: look at the clock and the error flag now and then
+            const unsigned long long now = global_ns();
+            if (since == 0) since = now;
+            if (now - since > a.timeout_ns) atomicExch(job.flag, 1u);
+            if (__any_sync(0xffffffffu, *reinterpret_cast<volatile unsigned*>(job.flag) != 0)) {
+              failed = 1;
+              break;
+            }
+          }
+        }
 #pragma unroll
         for (int k = 0; k < kRimInFlight; k++) {
           if (e[k].x == 0xffffffffu) continue;
-          while (!rec[k].ready(tag)) {
-            if ((++tries & 1023u) == 0) {  // bounded: look at the clock and the error flag now and then
-              const unsigned long long now = global_ns();
-              if (since == 0) since = now;
-              if (now - since > a.timeout_ns) atomicExch(job.flag, 1u);
-              if (*reinterpret_cast<volatile unsigned*>(job.flag)) {
-                failed = 1;
-                break;
-              }
-            }
-            rim_get(in + (size_t)e[k].x * RIM_BYTES, rec[k]);
-          }
           const uint32_t off = (e[k].y & ~1u) + ((e[k].y & 1u) ? (uint32_t)(par ^ 1) * CHIP_PAIR : 0u);
           *reinterpret_cast<double2*>(urows + off) = rec[k].value();
         }
@@ -546,6 +584,7 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
             uyo[j * pitch + i] = u.y;
             fvx[j * pitch + i] = v.get(2 * r);
             fvy[j * pitch + i] = v.get(2 * r + 1);
+            if (TRACK) const_cast<uint8_t*>(f.mask)[j * pitch + i] |= yielded[(2 * q + r) * 32 + lane];
           }
         }
       }

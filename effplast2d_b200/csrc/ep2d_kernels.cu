@@ -118,9 +118,9 @@ int occupancy_ty(bool record) {
   return e == cudaSuccess && n > 0 ? n : 1;
 }
 
-template <int PLASTIC, int JOBS, typename TV>
+template <int PLASTIC, int JOBS, typename TV, bool TRACK = false>
 cudaError_t set_chip_attr() {
-  return cudaFuncSetAttribute(k_iter_chip<PLASTIC, JOBS, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, CHIP_SMEM);
+  return cudaFuncSetAttribute(k_iter_chip<PLASTIC, JOBS, TV, TRACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, CHIP_SMEM);
 }
 
 template <typename TV>
@@ -128,6 +128,7 @@ cudaError_t set_chip_attrs() {
   cudaError_t e;
   if ((e = set_chip_attr<0, 1, TV>()) != cudaSuccess) return e;
   if ((e = set_chip_attr<1, 1, TV>()) != cudaSuccess) return e;
+  if ((e = set_chip_attr<1, 1, TV, true>()) != cudaSuccess) return e;
   return set_chip_attr<2, CHIP_JOBS, TV>();
 }
 
@@ -291,24 +292,32 @@ ChipShape chip_shape(int nx, int ny) {
   return best;
 }
 
-// The tallest tiles a launch may use are CHIP_WARPS warps x 18 rows, the shortest those of the
-// grid's own shape: 4 records per row of padded height and 4 x STREAM_COLS per tile.
-size_t chip_rim_bytes(int nx, int ny) {
+size_t chip_rim_bytes(int nx, int ny, int warps, int rows) {
+  const size_t ncx = (nx + STREAM_COLS - 1) / STREAM_COLS, ncy = (ny + warps * rows - 1) / (warps * rows);
+  return 2 * RIM_BYTES * ncx * ncy * (4 * (size_t)warps * rows + 4 * STREAM_COLS);
+}
+
+// 4 records per row of padded height and 4 x STREAM_COLS per tile: the shortest tiles of at
+// least 4 warps, and the tallest padding, decide
+size_t chip_rim_capacity(int nx, int ny) {
   const ChipShape s = chip_shape(nx, ny);
-  if (!s.warps) return 0;
-  return (size_t)2 * RIM_BYTES * s.ncx * (4 * ((size_t)ny + CHIP_WARPS * 18) + 4 * STREAM_COLS * (size_t)s.ncy);
+  size_t most = 0;
+  if (s.warps)
+    for (int rows = s.rows; rows <= 18; rows += 2)
+      for (int warps = 4; warps <= CHIP_WARPS; warps++) most = std::max(most, chip_rim_bytes(nx, ny, warps, rows));
+  return most;
 }
 
 int chip_ctas(int nx, int ny, int groups, int warps, int rows) {
   const int ncx = (nx + STREAM_COLS - 1) / STREAM_COLS, ncy = (ny + warps * rows - 1) / (warps * rows);
   return (ncx * ncy + groups - 1) / groups;
 }
-size_t chip_smem(int groups, int warps, int rows) { return chip_smem_bytes(groups, warps, rows); }
+size_t chip_smem(int groups, int warps, int rows, bool track) { return chip_smem_bytes(groups, warps, rows, track); }
 
 namespace {
 template <int JOBS>
 cudaError_t launch_chip_jobs(const ChipJob* jobs, int njobs, const void* kern, const ChipShape& s, int n_iter, int blocks,
-                             unsigned long long timeout_ns, cudaStream_t stream) {
+                             unsigned long long timeout_ns, cudaStream_t stream, bool track = false) {
   ChipArgs<JOBS> a;
   a.njobs = njobs;
   a.warps = s.warps;
@@ -318,14 +327,15 @@ cudaError_t launch_chip_jobs(const ChipJob* jobs, int njobs, const void* kern, c
   std::copy(jobs, jobs + njobs, a.job);
   void* args[] = {&a};
   return cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(32 * s.warps * s.groups), args,
-                                     chip_smem_bytes(s.groups, s.warps, s.rows), stream);
+                                     chip_smem_bytes(s.groups, s.warps, s.rows, track), stream);
 }
 }  // namespace
 
 cudaError_t launch_iter_chip(ChipJob* jobs, int njobs, bool mixed, const ChipShape& s, int n_iter,
-                             unsigned long long timeout_ns, cudaStream_t stream) {
-  if (njobs < 1 || njobs > CHIP_JOBS || n_iter < 2 || s.warps < 1 || s.groups < 1 ||
-      s.warps * s.groups > CHIP_WARPS || s.rows < 2 || s.rows > 18 || (s.rows & 1))
+                             unsigned long long timeout_ns, cudaStream_t stream, bool track) {
+  if (njobs < 1 || njobs > CHIP_JOBS || (track && njobs > 1) || n_iter < 2 || s.warps < 1 || s.groups < 1 ||
+      s.warps * s.groups > CHIP_WARPS || s.rows < 2 || s.rows > 18 || (s.rows & 1) ||
+      chip_smem_bytes(s.groups, s.warps, s.rows, track) > CHIP_SMEM)
     return cudaErrorInvalidValue;
   int blocks = 0;
   for (int k = 0; k < njobs; k++) {
@@ -334,10 +344,16 @@ cudaError_t launch_iter_chip(ChipJob* jobs, int njobs, bool mixed, const ChipSha
     j.ncx = (j.g.nx + STREAM_COLS - 1) / STREAM_COLS;
     j.ncy = (j.g.ny + s.warps * s.rows - 1) / (s.warps * s.rows);
     j.cta0 = blocks;
+    const cudaError_t e = cudaMemsetAsync(j.rim, 0, chip_rim_bytes(j.g.nx, j.g.ny, s.warps, s.rows), stream);
+    if (e != cudaSuccess) return e;
     blocks += (j.ncx * j.ncy + s.groups - 1) / s.groups;
   }
   if (njobs == 1) {
     const bool pl = jobs[0].plastic != 0;
+    if (track && pl)
+      return launch_chip_jobs<1>(jobs, 1, mixed ? (const void*)k_iter_chip<1, 1, float, true>
+                                                : (const void*)k_iter_chip<1, 1, double, true>,
+                                 s, n_iter, blocks, timeout_ns, stream, true);
     const void* kern = mixed ? (pl ? (const void*)k_iter_chip<1, 1, float> : (const void*)k_iter_chip<0, 1, float>)
                              : (pl ? (const void*)k_iter_chip<1, 1, double> : (const void*)k_iter_chip<0, 1, double>);
     return launch_chip_jobs<1>(jobs, 1, kern, s, n_iter, blocks, timeout_ns, stream);

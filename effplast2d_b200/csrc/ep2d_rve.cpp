@@ -321,6 +321,12 @@ size_t n_samples(const ep2d_params& p) {
 
 // the on-chip form is taken only where the parameters leave the kernel to the library
 bool chip_allowed(const ep2d_params& p) { return p.kernel == EP2D_KERNEL_AUTO && p.rows == 0; }
+// the stress arrays are contiguous, and those a recording launch writes (p to txy; with the
+// return map also txyav, j2, j2xy) hold the rim records of a run if they can
+size_t own_rim_bytes(const ep2d_params& p) {
+  const size_t need = chip_allowed(p) ? chip_rim_capacity(p.nx, p.ny) : 0;
+  return need > (p.nl > 1 ? 7 : 4) * align256(field_elems(p) * sizeof(double)) ? align256(need) : 0;
+}
 
 std::mutex g_prep_mu;
 std::set<int> g_prepared;
@@ -348,7 +354,7 @@ size_t Rve::footprint(const ep2d_params& p) {
   b += align256(partial_elems(p) * sizeof(double));      // averaging partials
   b += align256((2 * NAVG + n_samples(p) + 4) * sizeof(double));  // sums, samples, vmax, barrier
   b += align256(n_samples(p) * sizeof(unsigned long long));
-  if (chip_allowed(p)) b += align256(chip_rim_bytes(p.nx, p.ny));  // rim records of the on-chip form
+  b += own_rim_bytes(p);                                 // rim records of the on-chip form
   return b;
 }
 
@@ -489,7 +495,7 @@ int Rve::create(const ep2d_params& p, cudaStream_t s) {
   cp += align256((2 * NAVG + n_samples(p) + 4) * sizeof(double));
   d_idx = reinterpret_cast<unsigned long long*>(cp);
   cp += align256(n_samples(p) * sizeof(unsigned long long));
-  d_rim = cp;
+  d_rim = own_rim_bytes(p) ? cp : reinterpret_cast<char*>(f.p);
   chip = chip_allowed(p) && sms >= CHIP_SMS ? chip_shape(p.nx, p.ny) : ChipShape{};
 
   EP2D_CK(cudaMallocHost(&h_pin, (2 * NAVG + holes.size() + 2) * sizeof(double) + 64));
@@ -614,7 +620,7 @@ int Rve::capture(int parity) {
   return EP2D_OK;
 }
 
-ChipJob Rve::chip_job(int n, unsigned* flag) {
+ChipJob Rve::chip_job(unsigned* flag) const {
   ChipJob j{};
   j.g = g;
   j.f = f;
@@ -622,8 +628,6 @@ ChipJob Rve::chip_job(int n, unsigned* flag) {
   j.flag = flag;
   j.src = cur;
   j.plastic = prm.nl > 1 ? 1 : 0;
-  j.tag = chip_tag;
-  chip_tag += (uint32_t)n;
   return j;
 }
 
@@ -635,8 +639,8 @@ int Rve::run_chip(int64_t n, bool* done) {
   while (n > 0) {
     // chunks of an even length keep the parity; a chunk of one iteration cannot arise
     const int64_t chunk = n > ((int64_t)1 << 30) ? (int64_t)1 << 29 : n;
-    ChipJob job = chip_job((int)chunk, f.gbar + 2);
-    const cudaError_t e = launch_iter_chip(&job, 1, mixed(), chip, (int)chunk, CHIP_TIMEOUT_NS, stream);
+    ChipJob job = chip_job(f.gbar + 2);
+    const cudaError_t e = launch_iter_chip(&job, 1, mixed(), chip, (int)chunk, CHIP_TIMEOUT_NS, stream, track);
     if (e == cudaErrorCooperativeLaunchTooLarge) {
       cudaGetLastError();
       chip = ChipShape{};
@@ -654,7 +658,8 @@ int Rve::run_chip(int64_t n, bool* done) {
 }
 
 int Rve::run_plain(int64_t n) {
-  if (chip.warps && n >= CHIP_MIN_RUN && !f32 && !track) {
+  if (chip.warps && n >= CHIP_MIN_RUN && !f32 &&
+      (!track || chip_smem(chip.groups, chip.warps, chip.rows, true) <= CHIP_SMEM)) {
     bool done = false;
     const int rc = run_chip(n, &done);
     if (rc || done) return rc;

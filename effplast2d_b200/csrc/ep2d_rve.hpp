@@ -112,9 +112,9 @@ class Rve {
   int read_error(double* error);              // after a recording launch: D2H + error formula
   int finish_time_step(int step, int it);     // averaging etc. into the record
   double error_from_vmax(double vmx, double vmy) const;
-  // this RVE as a job of an on-chip launch of n iterations (its tags are then used); the
-  // launch flips `cur` by n & 1 when it has been made
-  ChipJob chip_job(int n, unsigned* flag);
+  // this RVE as a job of an on-chip launch of n iterations; the caller flips `cur` by n & 1
+  // when it has been made
+  ChipJob chip_job(unsigned* flag) const;
 
   int get_field(int field, double* host) const;
   int set_field(int field, const double* host);
@@ -134,8 +134,9 @@ class Rve {
   // runs of plain iterations in the on-chip form (warps == 0: not taken): the library's
   // choice (EP2D_KERNEL_AUTO, rows 0) on grids that fit on chip
   ChipShape chip{};
-  char* d_rim = nullptr;   // its rim records
-  uint32_t chip_tag = 1;   // the next unused record tag
+  // its rim records: in the stress arrays, which only recording launches write and every run of
+  // plain iterations is followed by one; in memory of their own where a small grid's are too small
+  char* d_rim = nullptr;
   // velocities stored in FP32 (the mixed path, and both phases of the FP32 bulk)
   bool mixed() const { return prm.precision == EP2D_MIXED || prm.precision == EP2D_F32_BULK; }
   // FP32 bulk: true while the state is in its FP32 form (u' in f.ux32/uy32)

@@ -120,9 +120,8 @@ constexpr int CHIP_SMEM = 226 * 1024;
 constexpr unsigned long long CHIP_TIMEOUT_NS = 10000000000ull;  // 10 s per wait
 constexpr int CHIP_MIN_RUN = 8;  // shorter runs of plain iterations are launched one by one
 ChipShape chip_shape(int nx, int ny);
-// One RVE of an on-chip launch: its fields, rim records (chip_rim_bytes), error flag, buffer
-// holding U, tiles, first CTA, and a record tag its earlier launches have not used (a launch of n
-// iterations uses n tags from `tag` on).
+// One RVE of an on-chip launch: its fields, rim records (chip_rim_bytes; zeroed by the launch),
+// error flag, buffer holding U, tiles and first CTA.
 struct ChipJob {
   Geo g;
   Fields f;
@@ -130,7 +129,6 @@ struct ChipJob {
   unsigned* flag;
   int src, plastic;
   int ncx, ncy, cta0;
-  uint32_t tag;
 };
 constexpr int CHIP_JOBS = 64;  // RVEs of one launch
 template <int JOBS>
@@ -139,17 +137,19 @@ struct ChipArgs {
   unsigned long long timeout_ns;
   ChipJob job[JOBS];
 };
-// bytes of the rim records an RVE needs in any shape a launch may give it (zeroed when the
-// RVE is created); 0 for a grid that does not fit on chip
-size_t chip_rim_bytes(int nx, int ny);
+// bytes of a grid's rim records at a given warps x rows, and the most any shape may need
+// that a launch takes for it (0 for a grid that does not fit on chip)
+size_t chip_rim_bytes(int nx, int ny, int warps, int rows);
+size_t chip_rim_capacity(int nx, int ny);
 // tiles and CTAs of a grid at a given warps x rows x groups
 int chip_ctas(int nx, int ny, int groups, int warps, int rows);
-size_t chip_smem(int groups, int warps, int rows);
+size_t chip_smem(int groups, int warps, int rows, bool track = false);
 // n_iter >= 2 plain iterations of the jobs' RVEs in one cooperative launch: CTAs of s.groups tiles of
 // s.warps x s.rows (s.ncx, s.ncy unused); fills in the jobs' tiles and CTAs.  Each wait gives up
 // after timeout_ns, which sets the job's flag
+// (track: also mark what yields, as launch_iter does; one job)
 cudaError_t launch_iter_chip(ChipJob* jobs, int njobs, bool mixed, const ChipShape& s, int n_iter,
-                             unsigned long long timeout_ns, cudaStream_t stream);
+                             unsigned long long timeout_ns, cudaStream_t stream, bool track = false);
 // clear the M_YN / M_YC bits of every node
 cudaError_t launch_clear_track(const Geo& g, uint8_t* mask, cudaStream_t stream);
 // one iteration of the FP32 bulk (stream form, segments of seg_h rows): u' and V in

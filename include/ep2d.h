@@ -299,9 +299,9 @@ int ep2d_analytic_fields(ep2d_handle* h, double delta_p, double tau_infty, doubl
  * on = 1 clears the zone and, from then on, every iteration marks each node and corner
  * whose trial J2 exceeds coh (Plast(iPlast) = 1, PlastXY(iPlastXY) = 1); the marks
  * accumulate over iterations, time steps and load steps until tracking is turned on
- * again (cleared) or off (kept).  While tracking, the handle launches the stream form of
- * the iteration kernel (tracking instantiation; results unchanged, both forms round
- * alike) and the FP32 phase of EP2D_F32_BULK marks nothing.  ep2d_polar_fields uses the
+ * again (cleared) or off (kept).  While tracking, the handle launches tracking
+ * instantiations of the stream form (single launches) and of the on-chip form (results
+ * unchanged, all forms round alike) and the FP32 phase of EP2D_F32_BULK marks nothing.  ep2d_polar_fields uses the
  * accumulated zone once tracking has been turned on.  No counterpart in the reference's
  * CUDA path. */
 int ep2d_track_plastic_zone(ep2d_handle* h, int32_t on);

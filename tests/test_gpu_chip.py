@@ -24,7 +24,7 @@ def _run(nx, ny, pa, nl, st, counts, precision, **kw):
         s.set(k, v)
     for n in counts:
         s.iterate(n)
-    out = {f: s.get(f) for f in FIELDS + (PLASTIC_FIELDS if nl > 1 else [])}
+    out = {f: s.get(f) for f in FIELDS + PLASTIC_FIELDS}  # (elastic: the latter stay zero)
     launches = s.stats()["launches"]
     s.close()
     return out, launches
@@ -50,6 +50,30 @@ def test_chip_form_matches_stream_form(nx, ny, nl, precision):
     assert la == 73
     if max(nx, ny) < 1100 or min(nx, ny) == 64:
         assert lb == 7  # three on-chip launches, four recording ones
+
+
+@pytest.mark.parametrize("nx,ny", [(9, 12), (96, 131), (257, 256), (530, 300), (1061, 1060)])
+@pytest.mark.parametrize("precision", [ep.FP64, ep.MIXED], ids=["fp64", "mixed"])
+def test_chip_tracking_matches_stream_tracking(nx, ny, precision):
+    # the yield bits of every iteration, single launches and on-chip runs alike, and the fields
+    pa = _pa(nx, ny, n_pores=1, porosity=0.02, yield_stress=1e-5)
+    st = _random_state(nx, ny, 61)
+    out = []
+    for kw in (dict(kernel=ep.KERNEL_STREAM, rows=16), {}):
+        s = ep.Solver(nx, ny, pa, nl=2, precision=precision, **kw)
+        for k, v in st.items():
+            s.set(k, v)
+        s.track_plastic_zone(True)
+        s.iterate(40)
+        s.iterate(3)
+        s.iterate(61)
+        d = s.polar_fields(-6e-5)
+        d.update({f: s.get(f) for f in ("Ux", "Vy", "J2XY")})
+        out.append(d)
+        s.close()
+    assert out[0]["Plast"].max() > 0
+    for k in out[0]:
+        assert np.array_equal(out[0][k], out[1][k]), k
 
 
 def test_chip_form_two_threads():
