@@ -370,7 +370,7 @@ int ep2d_server_destroy(ep2d_server* s);
  *   (nx*ny), tau_xy ((nx-1)*(ny-1)), ux ((nx+1)*ny), uy (nx*(ny+1)); pa: pa.dat values;
  *   out_dev[11] (caller's device memory) = sigma[0..3], sigma_per[0..3], eps_per[0..2],
  *   divided as the reference divides them (the values ep2d_step_record holds).
- * The reduction's partial sums use a fixed device array of 2048 x 11 doubles (176 KiB,
+ * The reduction's partial sums use a fixed device array of 2048 x 12 doubles and 256 counts (193 KiB,
  * held by every GPU that loads the library until the process exits), so ny may be at
  * most 8194; a larger ny returns EP2D_ERR_ARG without touching the GPU, as do dX or dY
  * not positive and N outside [1, 64].  A CUDA error left pending by earlier work is
