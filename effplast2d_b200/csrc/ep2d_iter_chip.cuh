@@ -34,24 +34,18 @@
 #pragma once
 
 #include "ep2d_iter_f64.cuh"
-#include "ep2d_iter_stream.cuh"
-#include "ep2d_stencil.cuh"
+#include "ep2d_march.cuh"
 #include "ep2d_types.hpp"
 
 namespace ep2d {
 
-// material constants of a node and a corner, by the 7-bit index of chip_index
-struct __align__(16) ChipMat {
-  double k, g2, g4, pad;
-};
-constexpr int CHIP_MATS = 128;
 // row pairs per turn of the march's loop: 2 measured best (1024^2, 16 rows: 9.85 us an
 // iteration; 1: 10.5, 4: 9.94 with spills)
 constexpr int kChipUnroll = 2;
 
-// shared memory, in bytes: materials, U rows (32 columns of (Ux, Uy)) in pairs, the material
-// index of every (row, column), and the poll list
-constexpr int CHIP_ROW = 32 * 16, CHIP_PAIR = 2 * CHIP_ROW;
+// shared memory, in bytes, u = the size of a displacement: materials, U rows (32 columns of
+// (Ux, Uy)) in pairs, the material index of every (row, column), and the poll list
+__host__ __device__ constexpr int chip_pair_bytes(int u) { return 2 * 32 * 2 * u; }
 __host__ __device__ constexpr int chip_pairs_per_warp(int rows) { return rows == 2 ? 2 : rows / 2 + 2; }
 // cells a lane polls: of the columns beside its warp's rows (4 per row), of the rows below
 // and above the tile (2 x 2 x 32 cells, spread over the group's warps)
@@ -59,13 +53,13 @@ __host__ __device__ constexpr int chip_col_polls(int rows) { return (4 * rows + 
 __host__ __device__ constexpr int chip_polls(int warps, int rows) {
   return chip_col_polls(rows) + (4 + warps - 1) / warps;
 }
-__host__ __device__ constexpr size_t chip_group_bytes(int warps, int rows) {
-  return (size_t)(warps * chip_pairs_per_warp(rows) + 4) * CHIP_PAIR + (size_t)(warps * rows + 4) * 32 +
+__host__ __device__ constexpr size_t chip_group_bytes(int warps, int rows, int u) {
+  return (size_t)(warps * chip_pairs_per_warp(rows) + 4) * chip_pair_bytes(u) + (size_t)(warps * rows + 4) * 32 +
          (size_t)warps * chip_polls(warps, rows) * 32 * sizeof(uint2);
 }
 // with tracking, a byte of yield bits per (row, column) behind the groups' regions
-__host__ __device__ constexpr size_t chip_smem_bytes(int groups, int warps, int rows, bool track = false) {
-  return CHIP_MATS * sizeof(ChipMat) + groups * (chip_group_bytes(warps, rows) + (track ? warps * rows * 32 : 0));
+__host__ __device__ constexpr size_t chip_smem_bytes(int groups, int warps, int rows, bool track = false, int u = 8) {
+  return N_MATS * 4 * u + groups * (chip_group_bytes(warps, rows, u) + (track ? warps * rows * 32 : 0));
 }
 
 // barrier of one group's threads that also ORs a flag over them
@@ -140,217 +134,131 @@ struct VPair<float> {
 };
 
 // ---- rim records ------------------------------------------------------------------------
-// Record of a cell: {lo, tag, hi, tag} of Ux and of Uy, one 256-bit access.
-struct RimRecord {
+// Record of a cell: {lo, tag, hi, tag} of Ux and of Uy, one 256-bit access; for float
+// displacements {Ux, tag, Uy, tag}, one 128-bit access.
+template <typename T>
+struct RimRecord;
+template <>
+struct RimRecord<double> {
+  static constexpr int BYTES = 32;
   uint32_t w[8];
   __device__ bool ready(uint32_t tag) const { return ((w[1] ^ tag) | (w[3] ^ tag) | (w[5] ^ tag) | (w[7] ^ tag)) == 0; }
   __device__ double2 value() const {
     return make_double2(__hiloint2double((int)w[2], (int)w[0]), __hiloint2double((int)w[6], (int)w[4]));
   }
+  __device__ void get(const char* rec) {
+    asm volatile("ld.relaxed.gpu.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                 : "l"(rec)
+                 : "memory");
+  }
+  static __device__ void put(char* rec, const double2& u, uint32_t tag) {
+    asm volatile("st.relaxed.gpu.global.v8.b32 [%0], {%1,%5,%2,%5,%3,%5,%4,%5};" ::"l"(rec), "r"(__double2loint(u.x)),
+                 "r"(__double2hiint(u.x)), "r"(__double2loint(u.y)), "r"(__double2hiint(u.y)), "r"(tag)
+                 : "memory");
+  }
 };
-constexpr int RIM_BYTES = 32;
+template <>
+struct RimRecord<float> {
+  static constexpr int BYTES = 16;
+  uint32_t w[4];
+  __device__ bool ready(uint32_t tag) const { return ((w[1] ^ tag) | (w[3] ^ tag)) == 0; }
+  __device__ float2 value() const { return make_float2(__uint_as_float(w[0]), __uint_as_float(w[2])); }
+  __device__ void get(const char* rec) {
+    asm volatile("ld.relaxed.gpu.global.v4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+                 : "l"(rec)
+                 : "memory");
+  }
+  static __device__ void put(char* rec, const float2& u, uint32_t tag) {
+    asm volatile("st.relaxed.gpu.global.v4.b32 [%0], {%1,%3,%2,%3};" ::"l"(rec), "r"(__float_as_uint(u.x)),
+                 "r"(__float_as_uint(u.y)), "r"(tag)
+                 : "memory");
+  }
+};
 // records a lane has in flight while it polls: 2 (3 and 4 cost the march registers, 128 being
 // all there are: 1024^2 9.85 -> 10.6 us an iteration)
 constexpr int kRimInFlight = 2;
-__device__ __forceinline__ void rim_put(char* rec, const double2& u, uint32_t tag) {
-  asm volatile("st.relaxed.gpu.global.v8.b32 [%0], {%1,%5,%2,%5,%3,%5,%4,%5};" ::"l"(rec), "r"(__double2loint(u.x)),
-               "r"(__double2hiint(u.x)), "r"(__double2loint(u.y)), "r"(__double2hiint(u.y)), "r"(tag)
-               : "memory");
-}
-__device__ __forceinline__ void rim_get(const char* rec, RimRecord& r) {
-  asm volatile("ld.relaxed.gpu.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]), "=r"(r.w[5]), "=r"(r.w[6]),
-                 "=r"(r.w[7])
-               : "l"(rec)
-               : "memory");
-}
-
 // where a warp's row pairs lie: pair q of its rows/2, copy `par` of the double-buffered ones
+template <typename T>
 __device__ __forceinline__ uint32_t chip_pair_off(int q, int npairs, int par) {
-  if (q == 0) return par * CHIP_PAIR;
-  if (q == npairs - 1) return (2 + par) * CHIP_PAIR;
-  return (3 + q) * CHIP_PAIR;
+  constexpr uint32_t PAIR = chip_pair_bytes(sizeof(T));
+  if (q == 0) return par * PAIR;
+  if (q == npairs - 1) return (2 + par) * PAIR;
+  return (3 + q) * PAIR;
 }
 
-// One iteration of one warp's rows jA .. jA + 2 npairs - 1 (copy `par` to copy par ^ 1).
-// rd0 / rdN: the row pairs below and above the warp's own; idx: material indices of row
-// jA - 2 on, 32 per row; vmem: tensor-memory address of the warp's V.
-// NP: the number of row pairs where it is known (1 to 3: the march unrolled, so that its rows'
-// chains overlap: 256^2, 2 rows, 2.70 -> 2.54 us an iteration; 448^2, 4 rows, 3.76 -> 3.55; 512^2, 6
-// rows, 4.29 -> 4.07), else 0.
-template <bool PLASTIC, bool EDGE, int NP, typename TV, bool TRACK>
-__device__ __forceinline__ void chip_march(const Geo& g, const ChipMat* __restrict__ mats, const uint8_t* idx,
-                                           const char* rd0, char* own, const char* rdN, int npairs_in, int par, int i,
-                                           int jA, uint32_t vmem, uint8_t* yielded) {
-  constexpr int VW = sizeof(VPair<TV>) / 4;
-  const int npairs = NP ? NP : npairs_in;
-  const int lane = threadIdx.x & 31;
-  const int nx = g.nx, ny = g.ny;
-  const int right = lane < 31 ? 1 : 0;
-  const bool col_own = lane >= 2 && lane < 2 + STREAM_COLS && (!EDGE || i < nx);
-  const double rdX = g.rdX, rdY = g.rdY, third = 1.0 / 3.0;
-  const double coh = g.coh, coh2 = g.coh2, coh4 = g.coh4, coh2x16 = g.coh2x16;
-  const double dT = g.dT, cX = g.cX, cY = g.cY, dtrX = g.dtrX, dtrY = g.dtrY;
-  int sa = 0, sb = 0;  // lanes of the node's clamped corner columns
-  if (EDGE) {
-    const int a = min(max(i - 1, 0), nx - 3) - i;
-    sa = min(max(lane + a, 0), 31);
-    sb = min(max(lane + a + 1, 0), 31);
-  }
+// Rows of one warp's tile part for pair_march: U in shared memory (from copy `par` to copy
+// par ^ 1), V in tensor memory.  NP: the number of row pairs where it is known (1 to 3: the march
+// unrolled, so that its rows' chains overlap: 256^2, 2 rows, 2.70 -> 2.54 us an iteration; 448^2,
+// 4 rows, 3.76 -> 3.55; 512^2, 6 rows, 4.29 -> 4.07), else 0.
+template <typename T, typename TV, bool EDGE, int NP>
+struct ChipIo {
+  using U2 = Vec2<T>;
+  static constexpr int VW = sizeof(VPair<TV>) / 4;
+  const MatT<T>* mats;
+  const uint8_t* idx;       // material indices of row jA - 2 on, 32 per row, this lane's column
+  const char *below, *above;  // the row pairs below and above the warp's own
+  char* own;
+  const char* rd;           // the pair read at this step, and at the one before
+  const char* rd_prev;
+  int npairs, par, right, rows_left;  // rows_left: own rows inside the grid (EDGE)
+  bool col_own;
+  uint32_t vmem;
+  uint8_t* yielded;         // TRACK: yield bits of the warp's rows, this lane's column
+  VPair<TV> v;
 
-  double uxc = 0, uxc_r = 0, uyc = 0;             // U of the last row read
-  double pb = 0, xb = 0, yb = 0, cb = 0;          // trial stresses of the last row
-  double hz = 0, h0 = 0, h1 = 0;                  // corner pair sums of the last three rows
-  double syq = 0, cq = 0, cq_l = 0;               // returned: total syy, corner of the row below
-  const char* rd_prev = rd0;
-
-  auto corner_pair = [&](double c) {
-    return EDGE ? add_rn(shfl_idx(c, sa), shfl_idx(c, sb)) : add_rn(shfl_up1(c), c);
-  };
-  // 4-corner sum of node row j from the pair sums of corner rows j - 2 .. j + 1
-  auto corner_sum = [&](int j, double hm2, double hm1, double hj, double hp1) {
-    if (EDGE) return j == 0 ? add_rn(hj, hp1) : j == ny - 1 ? add_rn(hm2, hm1) : add_rn(hm1, hj);
-    return add_rn(hm1, hj);
-  };
-  // 16 J2^2 of a corner of row j from the node deviators of rows j and j + 1
-  auto corner_j2 = [&](double x, double y, double c, double xn, double yn) {
-    const double vx = add_rn(x, xn), vy = add_rn(y, yn);
-    const double tx = add_rn(vx, shfl_dn(vx)), ty = add_rn(vy, shfl_dn(vy));
-    return corner_j2sq16(tx, ty, c);
-  };
-  // return_factor without a branch of its own: rsqrt of a value that is always in range
-  auto factor = [&](double j2, double lim2, double lim) {
-    const bool yields = j2 > lim2;
-    const double r = mul_rn(lim, rsqrt(yields ? j2 : lim2));
-    return yields ? r : 1.0;
-  };
-  // faces of row j: new velocities and displacements from the old ones
-  auto face = [&](int j, double sx, double sx_l, double sy, double cw_l, TV& vx, TV& vy, double2& u) {
-    const double vxo = (double)vx, vyo = (double)vy;
-    const TV vxs = (TV)face_velocity_s(vxo, cX, sub_rn(sx, sx_l), dtrX, sub_rn(cw_l, cq_l), dtrY);
-    const TV vys = (TV)face_velocity_s(vyo, cY, sub_rn(sy, syq), dtrY, sub_rn(cq, cq_l), dtrX);
-    if (EDGE) {
-      if (i > 0 && j > 0 && j < ny - 1) vx = vxs;
-      if (i > 0 && i < nx - 1 && j > 0) vy = vys;
-    } else {
-      vx = vxs;
-      vy = vys;
-    }
-    u.x = advance(u.x, (double)vx, dT);
-    u.y = advance(u.y, (double)vy, dT);
-  };
-
-  auto pair = [&](auto stage_c, int p, const char* rd, char* wr) {
-    constexpr int STAGE = decltype(stage_c)::value;
+  template <int STAGE>
+  __device__ __forceinline__ void begin(int p) {
     // the other lanes have read the rows this step overwrites (with one or two pairs every
     // row is double-buffered)
     if (NP == 0 || NP > 2) __syncwarp();
-    VPair<TV> v;
     if constexpr (STAGE == 2) tmem_ld(vmem + (p - 2) * VW, v.w);
-    const double2* ra = reinterpret_cast<const double2*>(rd) + lane;
-    const double2 ua = ra[0], uar = ra[right], ub = ra[32], ubr = ra[32 + right];
-    const uint8_t* ip = idx + (2 * p) * 32 + lane;  // row ka
-    double p1 = 0, x1 = 0, y1 = 0, c1 = 0, p2, x2, y2, c2, hs1 = 0, hs2 = 0;
-    if constexpr (STAGE >= 1) {  // trial of row ka - 1
-      const ChipMat& m = mats[ip[-32]];
-      node_trial(sub_rn(uxc_r, uxc), sub_rn(ua.y, uyc), m.k, m.g2, rdX, rdY, third, p1, x1, y1);
-      c1 = corner_trial(m.g4, sub_rn(uar.x, uxc_r), sub_rn(uar.y, ua.y), rdX, rdY);
-      if (PLASTIC) hs1 = corner_pair(c1);
-    }
-    {  // trial of row ka
-      const ChipMat& m = mats[ip[0]];
-      node_trial(sub_rn(uar.x, ua.x), sub_rn(ub.y, ua.y), m.k, m.g2, rdX, rdY, third, p2, x2, y2);
-      c2 = corner_trial(m.g4, sub_rn(ubr.x, uar.x), sub_rn(ubr.y, ub.y), rdX, rdY);
-      if (PLASTIC) hs2 = corner_pair(c2);
-    }
-    const int ja = jA + 2 * p - 4;  // row ka - 2
-    if constexpr (STAGE == 2) {
-      const double2* uo = reinterpret_cast<const double2*>(rd_prev) + lane;
-      double2 u0 = uo[0], u1 = uo[32];
-      double xr0 = xb, yr0 = yb, cw0 = cb, xr1 = x1, yr1 = y1, cw1 = c1;
-      if (PLASTIC) {
-        const double n0 = node_j2sq_h(xb, yb, corner_sum(ja, hz, h0, h1, hs1));
-        const double n1 = node_j2sq_h(x1, y1, corner_sum(ja + 1, h0, h1, hs1, hs2));
-        const double m0 = corner_j2(xb, yb, cb, x1, y1), m1 = corner_j2(x1, y1, c1, x2, y2);
-        if (__any_sync(0xffffffffu, n0 > coh2 || n1 > coh2 || m0 > coh2x16 || m1 > coh2x16)) {
-          const double f0 = factor(n0, coh2, coh), f1 = factor(n1, coh2, coh);
-          xr0 = mul_rn(xb, f0);
-          yr0 = mul_rn(yb, f0);
-          cw0 = mul_rn(cb, factor(m0, coh2x16, coh4));
-          xr1 = mul_rn(x1, f1);
-          yr1 = mul_rn(y1, f1);
-          cw1 = mul_rn(c1, factor(m1, coh2x16, coh4));
-          if (TRACK) {  // J2 > coh from the trial stresses (get_sigma_2D.m:126-138); a corner inside the grid
-            uint8_t* yl = yielded + 2 * (p - 2) * 32 + lane;
-            const bool c_in = !EDGE || i < nx - 1;
-            const int b0 = (n0 > coh2 ? M_YN : 0) | (c_in && (!EDGE || ja < ny - 1) && m0 > coh2x16 ? M_YC : 0);
-            const int b1 = (n1 > coh2 ? M_YN : 0) | (c_in && (!EDGE || ja + 1 < ny - 1) && m1 > coh2x16 ? M_YC : 0);
-            yl[0] |= b0;
-            yl[32] |= b1;
-          }
-        }
-      }
-      const double sx0 = sub_rn(xr0, pb), sy0 = sub_rn(yr0, pb), sx1 = sub_rn(xr1, p1), sy1 = sub_rn(yr1, p1);
-      const double cw0_l = shfl_up1(cw0), sx0_l = shfl_up1(sx0);
-      const double cw1_l = shfl_up1(cw1), sx1_l = shfl_up1(sx1);
-      tmem_ld_wait(v.w);
-      TV v0x = v.get(0), v0y = v.get(1), v1x = v.get(2), v1y = v.get(3);
-      face(ja, sx0, sx0_l, sy0, cw0_l, v0x, v0y, u0);
-      syq = sy0;
-      cq = cw0;
-      cq_l = cw0_l;
-      face(ja + 1, sx1, sx1_l, sy1, cw1_l, v1x, v1y, u1);
-      syq = sy1;
-      cq = cw1;
-      cq_l = cw1_l;
-      v.set(0, v0x);
-      v.set(1, v0y);
-      v.set(2, v1x);
-      v.set(3, v1y);
-      tmem_st(vmem + (p - 2) * VW, v.w);
-      double2* un = reinterpret_cast<double2*>(wr) + lane;
-      if (col_own && (!EDGE || ja < ny)) un[0] = u0;
-      if (col_own && (!EDGE || ja + 1 < ny)) un[32] = u1;
-    } else if constexpr (STAGE == 1) {
-      double yr = y1;
-      cq = c1;
-      if (PLASTIC) {
-        yr = mul_rn(y1, factor(node_j2sq_h(x1, y1, corner_sum(ja + 1, h0, h1, hs1, hs2)), coh2, coh));
-        cq = mul_rn(c1, factor(corner_j2(x1, y1, c1, x2, y2), coh2x16, coh4));
-      }
-      syq = sub_rn(yr, p1);
-      cq_l = shfl_up1(cq);
-    }
-    uxc = ub.x;
-    uxc_r = ubr.x;
-    uyc = ub.y;
-    pb = p2;
-    xb = x2;
-    yb = y2;
-    cb = c2;
-    hz = h1;
-    h0 = hs1;
-    h1 = hs2;
     rd_prev = rd;
-  };
-  pair(std::integral_constant<int, 0>{}, 0, rd0, nullptr);
-  pair(std::integral_constant<int, 1>{}, 1, own + chip_pair_off(0, npairs, par), nullptr);
-#pragma unroll (NP ? NP : kChipUnroll)
-  for (int p = 2; p <= npairs + 1; p++)
-    pair(std::integral_constant<int, 2>{}, p, p <= npairs ? own + chip_pair_off(p - 1, npairs, par) : rdN,
-         own + chip_pair_off(p - 2, npairs, par ^ 1));
-  tmem_st_wait();
-}
+    rd = p == 0 ? below : p <= npairs ? own + chip_pair_off<T>(p - 1, npairs, par) : above;
+  }
+  __device__ __forceinline__ void rows(int, U2& ua, U2& uar, U2& ub, U2& ubr) {
+    const U2* r = reinterpret_cast<const U2*>(rd) + (threadIdx.x & 31);
+    ua = r[0];
+    uar = r[right];
+    ub = r[32];
+    ubr = r[32 + right];
+  }
+  __device__ __forceinline__ const MatT<T>& mat(int p, int r) { return mats[idx[(2 * p - 1 + r) * 32]]; }
+  __device__ __forceinline__ void old(int, U2& u0, U2& u1, TV (&vv)[4]) {
+    const U2* r = reinterpret_cast<const U2*>(rd_prev) + (threadIdx.x & 31);
+    u0 = r[0];
+    u1 = r[32];
+    tmem_ld_wait(v.w);
+#pragma unroll
+    for (int k = 0; k < 4; k++) vv[k] = v.get(k);
+  }
+  __device__ __forceinline__ void store(int p, const U2& u0, const U2& u1, const TV (&vv)[4]) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) v.set(k, vv[k]);
+    tmem_st(vmem + (p - 2) * VW, v.w);
+    U2* un = reinterpret_cast<U2*>(own + chip_pair_off<T>(p - 2, npairs, par ^ 1)) + (threadIdx.x & 31);
+    if (col_own && (!EDGE || 2 * p - 4 < rows_left)) un[0] = u0;
+    if (col_own && (!EDGE || 2 * p - 3 < rows_left)) un[32] = u1;
+  }
+  __device__ __forceinline__ void yields(int p, bool n0, bool n1, bool c0, bool c1) {
+    uint8_t* y = yielded + 2 * (p - 2) * 32;
+    y[0] |= (n0 ? M_YN : 0) | (c0 ? M_YC : 0);
+    y[32] |= (n1 ? M_YN : 0) | (c1 ? M_YC : 0);
+  }
+};
 
 // a.n_iter plain iterations of every job's RVE from its buffer `src`, ending in buffer
 // src ^ (n_iter & 1) (n_iter >= 2: when the buffers coincide, a tile is written back only after
 // its neighbours have read it).  CTAs of groups of a.warps warps, a group per tile, a.rows rows per
 // warp.  rim: records [2][tile][4 H + 112 cells].  PLASTIC 0, 1: all jobs; 2: per job.
 // TRACK: also mark the nodes and corners that yield at any of the iterations (M_YN, M_YC).
-template <int PLASTIC, int JOBS, typename TV, bool TRACK = false>
+template <int PLASTIC, int JOBS, typename T, typename TV, bool TRACK = false>
 __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_constant__ ChipArgs<JOBS> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t s_tmem;
+  using U2 = Vec2<T>;
+  constexpr int US = sizeof(T), PAIR = chip_pair_bytes(US), RIM_BYTES = RimRecord<T>::BYTES;
   int jb = 0;
   if (JOBS > 1)
     while (jb + 1 < a.njobs && (int)blockIdx.x >= a.job[jb + 1].cta0) jb++;
@@ -370,13 +278,13 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
   const int ncol = chip_col_polls(rows), npoll = chip_polls(nw, rows);
   if (__syncthreads_or(*reinterpret_cast<volatile unsigned*>(job.flag) != 0)) return;  // an earlier launch failed
 
-  ChipMat* mats = reinterpret_cast<ChipMat*>(smem_raw);
-  char* urows = reinterpret_cast<char*>(smem_raw) + CHIP_MATS * sizeof(ChipMat) + group * chip_group_bytes(nw, rows);
-  char* halo_b = urows + nw * ppw * CHIP_PAIR;
-  char* halo_t = halo_b + 2 * CHIP_PAIR;  // the rows below and above the tile, two copies each
-  uint8_t* idx = reinterpret_cast<uint8_t*>(halo_t + 2 * CHIP_PAIR);
+  MatT<T>* mats = reinterpret_cast<MatT<T>*>(smem_raw);
+  char* urows = reinterpret_cast<char*>(smem_raw) + N_MATS * sizeof(MatT<T>) + group * chip_group_bytes(nw, rows, US);
+  char* halo_b = urows + nw * ppw * PAIR;
+  char* halo_t = halo_b + 2 * PAIR;  // the rows below and above the tile, two copies each
+  uint8_t* idx = reinterpret_cast<uint8_t*>(halo_t + 2 * PAIR);
   uint2* polls = reinterpret_cast<uint2*>(idx + (H + 4) * 32);
-  uint8_t* yielded = smem_raw + chip_smem_bytes(groups, nw, rows) + wc * rows * 32;  // TRACK only
+  uint8_t* yielded = smem_raw + chip_smem_bytes(groups, nw, rows, false, US) + wc * rows * 32;  // TRACK only
 
   if (wc == 0) {  // one CTA per SM takes all of the SM's tensor memory
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
@@ -384,14 +292,7 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  for (int t = threadIdx.x; t < CHIP_MATS; t += blockDim.x) {
-    ChipMat m{0.0, 0.0, g4z_entry(t >> 2, g.G0, g.Gp), 0.0};
-    if (!(t & M_NODE)) {
-      m.k = (t & M_MAT) ? g.Kp : g.K0;
-      m.g2 = __dmul_rn(2.0, (t & M_MAT) ? g.Gp : g.G0);
-    }
-    mats[t] = m;
-  }
+  for (int t = threadIdx.x; t < N_MATS; t += blockDim.x) mats[t] = mat_entry<T>(g, t);
   __syncthreads();
   if (!idle) {
     const int i = x0 - 2 + lane;
@@ -400,26 +301,26 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
 
     // U of the tile and its halo, both copies of the double-buffered rows (faces outside the
     // arrays: 0; the face column nx of Ux and row ny of Uy never change)
-    const double* __restrict__ ux = f.ux[src];
-    const double* __restrict__ uy = f.uy[src];
+    const T* __restrict__ ux = u_field<T>(f, false, src);
+    const T* __restrict__ uy = u_field<T>(f, true, src);
     auto load_u = [&](int j) {
-      double2 u;
-      u.x = (i >= 0 && i <= nx && j >= 0 && j < ny) ? ux[j * pitch + i] : 0.0;
-      u.y = (i >= 0 && i < nx && j >= 0 && j <= ny) ? uy[j * pitch + i] : 0.0;
+      U2 u;
+      u.x = (i >= 0 && i <= nx && j >= 0 && j < ny) ? ux[j * pitch + i] : (T)0;
+      u.y = (i >= 0 && i < nx && j >= 0 && j <= ny) ? uy[j * pitch + i] : (T)0;
       return u;
     };
-    char* own = urows + w * ppw * CHIP_PAIR;
+    char* own = urows + w * ppw * PAIR;
     if (TRACK)
       for (int r = 0; r < rows; r++) yielded[r * 32 + lane] = 0;
     for (int r = 0; r < rows; r++) {
-      const double2 u = load_u(jA + r);
+      const U2 u = load_u(jA + r);
       for (int par = 0; par < 2; par++)
-        reinterpret_cast<double2*>(own + chip_pair_off(r >> 1, npairs, par))[32 * (r & 1) + lane] = u;
+        reinterpret_cast<U2*>(own + chip_pair_off<T>(r >> 1, npairs, par))[32 * (r & 1) + lane] = u;
     }
     for (int q = w; q < 4; q += nw) {  // both copies: cells outside the arrays are never polled
-      const double2 u = load_u(q < 2 ? y0 - 2 + q : y0 + H + q - 2);
+      const U2 u = load_u(q < 2 ? y0 - 2 + q : y0 + H + q - 2);
       for (int par = 0; par < 2; par++)
-        reinterpret_cast<double2*>((q < 2 ? halo_b : halo_t) + par * CHIP_PAIR)[32 * (q & 1) + lane] = u;
+        reinterpret_cast<U2*>((q < 2 ? halo_b : halo_t) + par * PAIR)[32 * (q & 1) + lane] = u;
     }
 
     // what this lane polls: cell of the records (0xffffffff: none), destination in shared
@@ -436,7 +337,7 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
         if (r < rows && ci >= 0 && ci < nx && cj < ny) {
           e.x = cta_of(q < 2 ? -1 : 1, 0) * cells + (w * rows + r) * 4 + (q < 2 ? 2 + q : q - 2);
           const int pq = r >> 1;
-          e.y = (uint32_t)(own - urows) + chip_pair_off(pq, npairs, 0) + ((r & 1) * 32 + col) * 16;
+          e.y = (uint32_t)(own - urows) + chip_pair_off<T>(pq, npairs, 0) + ((r & 1) * 32 + col) * 2 * US;
           if (pq == 0 || pq == npairs - 1) e.y |= 1;
         }
         pl[t * 32] = e;
@@ -451,7 +352,7 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
           if (lane < 2) e.x = cta_of(-1, dy) * cells + row * 4 + 2 + lane;
           else if (lane >= 30) e.x = cta_of(1, dy) * cells + row * 4 + lane - 30;
           else e.x = cta_of(0, dy) * cells + 4 * H + (below ? 2 * STREAM_COLS : 0) + r * STREAM_COLS + lane - 2;
-          e.y = ((uint32_t)((below ? halo_b : halo_t) - urows) + (r * 32 + lane) * 16) | 1;
+          e.y = ((uint32_t)((below ? halo_b : halo_t) - urows) + (r * 32 + lane) * 2 * US) | 1;
         }
         pl[t * 32] = e;
       }
@@ -476,30 +377,46 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
     }
     tmem_st_wait();
 
-    const char* rd_below = w > 0 ? own - ppw * CHIP_PAIR + (npairs == 1 ? 0 : 2 * CHIP_PAIR) : halo_b;
-    const char* rd_above = w < nw - 1 ? own + ppw * CHIP_PAIR : halo_t;
+    const char* rd_below = w > 0 ? own - ppw * PAIR + (npairs == 1 ? 0 : 2 * PAIR) : halo_b;
+    const char* rd_above = w < nw - 1 ? own + ppw * PAIR : halo_t;
     const bool interior = x0 - 2 >= 1 && x0 + 29 <= nx - 3 && jA >= 3 && jA + rows <= ny - 2;
     const size_t rim_parity = (size_t)(ncx * ncy) * cells * RIM_BYTES;
     int it = 0;
     for (;; it++) {
       const int par = it & 1;
       if (jA < ny) {
-        const char* below = rd_below + par * CHIP_PAIR;
-        const char* above = rd_above + par * CHIP_PAIR;
-        const uint8_t* ix = idx + (w * rows) * 32;
+        const char* below = rd_below + par * PAIR;
+        const char* above = rd_above + par * PAIR;
         auto march = [&](auto plastic_c) {
           constexpr bool P = decltype(plastic_c)::value;
           auto rows_of = [&](auto np_c) {
             constexpr int NP = decltype(np_c)::value;
-            if (interior)
-              chip_march<P, false, NP, TV, TRACK>(g, mats, ix, below, own, above, npairs, par, i, jA, vmem, yielded);
-            else
-              chip_march<P, true, NP, TV, TRACK>(g, mats, ix, below, own, above, npairs, par, i, jA, vmem, yielded);
+            auto run = [&](auto edge_c) {
+              constexpr bool EDGE = decltype(edge_c)::value;
+              ChipIo<T, TV, EDGE, NP> io;
+              io.mats = mats;
+              io.idx = idx + w * rows * 32 + lane;
+              io.below = below;
+              io.above = above;
+              io.own = own;
+              io.rd = below;
+              io.npairs = NP ? NP : npairs;
+              io.par = par;
+              io.right = lane < 31 ? 1 : 0;
+              io.rows_left = ny - jA;
+              io.col_own = col_own;
+              io.vmem = vmem;
+              io.yielded = yielded + lane;
+              pair_march<T, TV, P, EDGE, NP, TRACK, kChipUnroll>(g, io, npairs, i, jA);
+            };
+            if (interior) run(std::false_type{});
+            else run(std::true_type{});
           };
           if (npairs == 1) rows_of(std::integral_constant<int, 1>{});
           else if (npairs == 2) rows_of(std::integral_constant<int, 2>{});
           else if (npairs == 3) rows_of(std::integral_constant<int, 3>{});
           else rows_of(std::integral_constant<int, 0>{});
+          tmem_st_wait();
         };
         if (PLASTIC == 1 || (PLASTIC == 2 && job.plastic)) march(std::true_type{});
         else march(std::false_type{});
@@ -510,8 +427,8 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
       char* out = job.rim + par * rim_parity + (size_t)tile * cells * RIM_BYTES;
       const char* in = job.rim + par * rim_parity;
       auto put = [&](int cell, int r, int col) {
-        rim_put(out + cell * RIM_BYTES,
-                reinterpret_cast<const double2*>(own + chip_pair_off(r >> 1, npairs, par ^ 1))[(r & 1) * 32 + col], tag);
+        RimRecord<T>::put(out + cell * RIM_BYTES,
+                reinterpret_cast<const U2*>(own + chip_pair_off<T>(r >> 1, npairs, par ^ 1))[(r & 1) * 32 + col], tag);
       };
       if (jA < ny) {
         for (int c = lane; c < 4 * rows; c += 32) put(w * rows * 4 + c, c >> 2, (c & 3) < 2 ? 2 + (c & 3) : 26 + (c & 3));
@@ -525,7 +442,7 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
       int failed = 0;
       for (int t0 = 0; t0 < npoll && !failed; t0 += kRimInFlight) {
         uint2 e[kRimInFlight];
-        RimRecord rec[kRimInFlight];
+        RimRecord<T> rec[kRimInFlight];
         bool wait[kRimInFlight];
 #pragma unroll
         for (int k = 0; k < kRimInFlight; k++) {
@@ -539,7 +456,7 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
           bool any = false;
 #pragma unroll
           for (int k = 0; k < kRimInFlight; k++)
-            if (wait[k]) rim_get(in + (size_t)e[k].x * RIM_BYTES, rec[k]);
+            if (wait[k]) rec[k].get(in + (size_t)e[k].x * RIM_BYTES);
 #pragma unroll
           for (int k = 0; k < kRimInFlight; k++) {
             if (wait[k]) wait[k] = !rec[k].ready(tag);
@@ -559,8 +476,8 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
 #pragma unroll
         for (int k = 0; k < kRimInFlight; k++) {
           if (e[k].x == 0xffffffffu) continue;
-          const uint32_t off = (e[k].y & ~1u) + ((e[k].y & 1u) ? (uint32_t)(par ^ 1) * CHIP_PAIR : 0u);
-          *reinterpret_cast<double2*>(urows + off) = rec[k].value();
+          const uint32_t off = (e[k].y & ~1u) + ((e[k].y & 1u) ? (uint32_t)(par ^ 1) * PAIR : 0u);
+          *reinterpret_cast<U2*>(urows + off) = rec[k].value();
         }
       }
       if (group_barrier_or(1 + group, 32 * nw, failed)) break;
@@ -569,8 +486,8 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
     // back to global memory: U of the last copy written, V
     if (jA < ny) {
       __syncwarp();
-      double* uxo = f.ux[src ^ (n_iter & 1)];
-      double* uyo = f.uy[src ^ (n_iter & 1)];
+      T* uxo = u_field<T>(f, false, src ^ (n_iter & 1));
+      T* uyo = u_field<T>(f, true, src ^ (n_iter & 1));
       const int par = (it & 1) ^ 1;
       for (int q = 0; q < npairs; q++) {
         VPair<TV> v;
@@ -579,7 +496,7 @@ __global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_c
         for (int r = 0; r < 2; r++) {
           const int j = jA + 2 * q + r;
           if (col_own && j < ny) {
-            const double2 u = reinterpret_cast<const double2*>(own + chip_pair_off(q, npairs, par))[32 * r + lane];
+            const U2 u = reinterpret_cast<const U2*>(own + chip_pair_off<T>(q, npairs, par))[32 * r + lane];
             uxo[j * pitch + i] = u.x;
             uyo[j * pitch + i] = u.y;
             fvx[j * pitch + i] = v.get(2 * r);

@@ -27,8 +27,7 @@
 
 #include <type_traits>
 
-#include "ep2d_stencil.cuh"
-#include "ep2d_types.hpp"
+#include "ep2d_march.cuh"
 
 namespace ep2d {
 
@@ -73,28 +72,10 @@ struct StreamWarpSmem {
   KG2<TU> kgz[4];
 };
 
-// c = corner table index of the corner (i, j) from the mask bytes of nodes (i, j) and
-// (i, j + 1); the four material bits of g4z's index: bit 0 node (i, j), bit 3 (i+1, j),
-// bit 1 (i, j+1), bit 4 (i+1, j+1); bit 2 the corner's pore bit
-__device__ __forceinline__ int corner_index(int m_j, int m_j1) {
-  return (m_j & (M_MAT | M_CORNER | M_MAT_R)) | ((m_j1 & (M_MAT | M_MAT_R)) << 1);
-}
-__device__ __forceinline__ double g4z_entry(int c, double G0, double Gp) {
-  return (c & 4) ? 0.0 : corner_g4(c & 1, (c >> 3) & 1, (c >> 1) & 1, (c >> 4) & 1, G0, Gp);
-}
-
 template <typename TU, typename TV>
 constexpr size_t stream_smem_bytes() {
   return sizeof(StreamWarpSmem<TU, TV>) * STREAM_WARPS;
 }
-
-template <typename T>
-__device__ __forceinline__ T shfl_idx(T v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-template <typename T>
-__device__ __forceinline__ T shfl_dn(T v) { return __shfl_down_sync(0xffffffffu, v, 1); }
-template <typename T>
-__device__ __forceinline__ T shfl_up1(T v) { return __shfl_up_sync(0xffffffffu, v, 1); }
-__device__ __forceinline__ int shfl_dn_i(int v) { return __shfl_down_sync(0xffffffffu, v, 1); }
 
 // cp.async of 4, 8 or 16 bytes; with ok == false nothing is read and the destination is
 // zero-filled (src-size 0), `src` then only has to be a valid address.
@@ -123,18 +104,6 @@ __device__ __forceinline__ void cp_async_wait() {
 // inside the grid with jA >= 3 and jB <= ny-2
 __device__ __forceinline__ bool stream_interior(int nx, int ny, int strip, int jA, int jB) {
   return strip >= 1 && STREAM_COLS * strip + 29 <= nx - 3 && jA >= 3 && jB <= ny - 2;
-}
-
-// The displacement arrays of a form: FP64 U, or the FP32 bulk's perturbations u'.
-template <typename TU>
-__device__ __forceinline__ TU* u_field(const Fields& f, bool y, int buf);
-template <>
-__device__ __forceinline__ double* u_field<double>(const Fields& f, bool y, int buf) {
-  return y ? f.uy[buf] : f.ux[buf];
-}
-template <>
-__device__ __forceinline__ float* u_field<float>(const Fields& f, bool y, int buf) {
-  return y ? f.uy32[buf] : f.ux32[buf];
 }
 
 // One strip segment.  TU = double: the FP64 stencil (velocities stored as TV); TU =
@@ -482,6 +451,198 @@ __global__ void __launch_bounds__(32 * STREAM_WARPS) k_iter_stream_batch(const B
       stream_segment<false, RECORD, double, TV>(e.g, e.f, src, u.y & 0xffff, u.y >> 16, seg_h, sm, vmx, vmy);
     stream_fold_vmax<RECORD>(vmx, vmy, e.f.vmax);
   }
+}
+
+// ---- plain launches of one RVE: the pair march over a ring of row pairs -------------------
+// Two rows per step (ep2d_march.cuh), the rows in a per-warp ring of row pairs filled by
+// cp.async, PAIR_DEPTH pairs ahead of use: pair k is read at step k (U of its rows) and at
+// step k + 1 (old U and V of the faces), and its slot is refilled after that.  3 pairs ahead
+// measured slower (2048^2 58.6 us an iteration against 53.3: less L1 beside the larger rings).
+// Offsets into a field are 32-bit bytes from its base (fields of 4 GB and more stay with
+// k_iter_stream): a store or copy then needs no 64-bit address arithmetic (53.3 -> 52.5).
+//
+// us per iteration with the return map, k_iter_stream before / this: 2048^2 60.5 / 52.5 (5.1 TB/s of the
+// 64 B per cell, 0.78 of the measured HBM rate), 1536^2 44.5 / 30.6 and 1200^2 25.6 / 19.8 (with
+// segments that fill one wave, shape_of), 2048^2 elastic 61.7 / 49.5, FP32 bulk 41.7 / 34.5.  What bounds it
+// at 2048^2: issue (205 warp instructions per strip row where all yields, 64 % of
+// cycles) together with HBM.
+constexpr int PAIR_DEPTH = 2;
+constexpr int PAIR_SLOTS = PAIR_DEPTH + 2;
+
+template <typename TU, typename TV>
+struct __align__(16) StreamPair {
+  TU ux[2][32];
+  TU uy[2][32];
+  TV vx[2][32];
+  TV vy[2][32];
+  uint32_t m[2][12];  // mask bytes of columns x0 - 4 .. x0 + 31 (x0: the strip's first)
+};
+template <typename TU, typename TV>
+constexpr size_t stream_pair_smem_bytes() {
+  return N_MATS * sizeof(MatT<TU>) + sizeof(StreamPair<TU, TV>) * PAIR_SLOTS * STREAM_WARPS;
+}
+
+template <typename TU, typename TV, bool EDGE>
+struct StreamIo {
+  using U2 = Vec2<TU>;
+  static constexpr bool TRACK = false;
+  const MatT<TU>* mats;
+  StreamPair<TU, TV>* ring;
+  const TU *ux, *uy;
+  TU *uxo, *uyo;
+  TV *vx, *vy;
+  const uint8_t* mask;
+  int nx, ny, pitch, strip, i, jA, jB, npairs;
+  bool own;
+  int mk_c = 0;     // mask byte of the last row of the previous step
+  int mk_a = 0, mk_b = 0;
+  int slot = PAIR_SLOTS - 1;  // slot of the pair read at this step
+
+  // row pair k (rows jA - 2 + 2k and the next) into its slot: lane's half of the warp copies one
+  // row's 16 pairs of columns of each array (16 bytes; V as float 8), and the mask's words
+  __device__ __forceinline__ void issue(int k, int s) {
+    StreamPair<TU, TV>& d = ring[s];
+    const int lane = threadIdx.x & 31, r = lane >> 4, c = lane & 15;
+    const int row = jA - 2 + 2 * k + r, col = STREAM_COLS * strip - 2 + 2 * c;
+    const bool in = !EDGE || (col >= 0 && col < pitch && row >= 0);
+    const bool okx = in && (!EDGE || row < ny), oky = in && (!EDGE || row <= ny);
+    const int q = row * pitch + col;
+    auto at = [](auto* b, uint32_t k) {
+      return reinterpret_cast<decltype(b)>(reinterpret_cast<const char*>(b) + (uint32_t)(k * (uint32_t)sizeof(*b)));
+    };
+    cp_async_pair_zfill<TU>(&d.ux[r][2 * c], at(ux, okx ? q : 0), okx);
+    cp_async_pair_zfill<TU>(&d.uy[r][2 * c], at(uy, oky ? q : 0), oky);
+    cp_async_pair_zfill<TV>(&d.vx[r][2 * c], at((const TV*)vx, okx ? q : 0), okx);
+    cp_async_pair_zfill<TV>(&d.vy[r][2 * c], at((const TV*)vy, oky ? q : 0), oky);
+    if (c < 9) {
+      const int mc = STREAM_COLS * strip - 4 + 4 * c;
+      const bool okm = !EDGE || (mc >= 0 && mc < pitch && row >= 0 && row < ny);
+      cp_async_zfill<4>(&d.m[r][c], mask + (okm ? row * pitch + mc : 0), okm);
+    }
+  }
+  __device__ __forceinline__ int mask_byte(const StreamPair<TU, TV>& d, int r, int row) const {
+    const int lane = threadIdx.x & 31;
+    const int m = reinterpret_cast<const uint8_t*>(d.m[r])[lane + 2];
+    if (!EDGE) return m;
+    // a node outside the grid counts as a pore node, a corner outside it as a pore corner
+    const bool node = i >= 0 && i < nx && row >= 0 && row < ny;
+    const bool corner = i >= 0 && i < nx - 1 && row >= 0 && row < ny - 1;
+    return node ? (corner ? m : (m | M_CORNER)) : (int)(M_NODE | M_CORNER);
+  }
+  template <int STAGE>
+  __device__ __forceinline__ void begin(int p) {
+    cp_async_wait<PAIR_DEPTH - 1>();  // this lane's copies of pair p have landed
+    __syncwarp();                      // ... and every lane's; and all have read pair p - 2
+    slot = slot + 1 == PAIR_SLOTS ? 0 : slot + 1;
+    const int refill = slot + PAIR_DEPTH >= PAIR_SLOTS ? slot + PAIR_DEPTH - PAIR_SLOTS : slot + PAIR_DEPTH;
+    if (p + PAIR_DEPTH <= npairs + 1) issue(p + PAIR_DEPTH, refill);
+    cp_async_commit();  // an empty group keeps the count uniform
+    const StreamPair<TU, TV>& d = ring[slot];
+    mk_c = mk_b;
+    mk_a = mask_byte(d, 0, jA - 2 + 2 * p);
+    mk_b = mask_byte(d, 1, jA - 1 + 2 * p);
+  }
+  __device__ __forceinline__ void rows(int, U2& ua, U2& uar, U2& ub, U2& ubr) const {
+    const StreamPair<TU, TV>& d = ring[slot];
+    const int lane = threadIdx.x & 31, ln1 = min(lane + 1, 31);
+    ua.x = d.ux[0][lane];
+    ua.y = d.uy[0][lane];
+    uar.x = d.ux[0][ln1];
+    uar.y = d.uy[0][ln1];
+    ub.x = d.ux[1][lane];
+    ub.y = d.uy[1][lane];
+    ubr.x = d.ux[1][ln1];
+    ubr.y = d.uy[1][ln1];
+  }
+  __device__ __forceinline__ const MatT<TU>& mat(int, int r) const {
+    const int m = r ? mk_a : mk_c, up = r ? mk_b : mk_a;
+    return mats[(m & (M_MAT | M_NODE)) | (corner_index(m, up) << 2)];
+  }
+  __device__ __forceinline__ void old(int, U2& u0, U2& u1, TV (&v)[4]) const {
+    const StreamPair<TU, TV>& d = ring[slot ? slot - 1 : PAIR_SLOTS - 1];
+    const int lane = threadIdx.x & 31;
+    u0.x = d.ux[0][lane];
+    u0.y = d.uy[0][lane];
+    u1.x = d.ux[1][lane];
+    u1.y = d.uy[1][lane];
+    v[0] = d.vx[0][lane];
+    v[1] = d.vy[0][lane];
+    v[2] = d.vx[1][lane];
+    v[3] = d.vy[1][lane];
+  }
+  __device__ __forceinline__ void store(int p, const U2& u0, const U2& u1, const TV (&v)[4]) const {
+    const int j = jA + 2 * p - 4;
+    const uint32_t q = (uint32_t)(j * pitch + i), q1 = q + pitch;
+    auto at = [](auto* b, uint32_t k) -> auto& {
+      return *reinterpret_cast<decltype(b)>(reinterpret_cast<char*>(b) + (uint32_t)(k * (uint32_t)sizeof(*b)));
+    };
+    if (own) {
+      at(vx, q) = v[0];
+      at(vy, q) = v[1];
+      at(uxo, q) = u0.x;
+      at(uyo, q) = u0.y;
+    }
+    if (own && j + 1 < jB) {
+      at(vx, q1) = v[2];
+      at(vy, q1) = v[3];
+      at(uxo, q1) = u1.x;
+      at(uyo, q1) = u1.y;
+    }
+  }
+  __device__ __forceinline__ void yields(int, bool, bool, bool, bool) const {}
+};
+
+// One plain iteration of one RVE: warp w of CTA b handles task b * STREAM_WARPS + w =
+// (strip, segment), as k_iter_stream does.
+template <bool PLASTIC, typename TU, typename TV>
+__global__ void __launch_bounds__(32 * STREAM_WARPS, 4) k_iter_pairs(const __grid_constant__ Geo g,
+                                                                     const __grid_constant__ Fields f, int src,
+                                                                     int nstrips, int nsegs, int seg_h) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  MatT<TU>* mats = reinterpret_cast<MatT<TU>*>(smem_raw);
+  StreamPair<TU, TV>* ring =
+      reinterpret_cast<StreamPair<TU, TV>*>(smem_raw + N_MATS * sizeof(MatT<TU>)) + (threadIdx.x >> 5) * PAIR_SLOTS;
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  for (int t = threadIdx.x; t < N_MATS; t += blockDim.x) mats[t] = mat_entry<TU>(g, t);
+  __syncthreads();
+  const int task = blockIdx.x * STREAM_WARPS + (threadIdx.x >> 5);
+  if (task >= nstrips * nsegs) return;  // whole warp
+  const int strip = task % nstrips, jA = task / nstrips * seg_h, jB = min(jA + seg_h, g.ny);
+  const int lane = threadIdx.x & 31, i = STREAM_COLS * strip - 2 + lane;
+  // the previous iteration's grid has completed and its stores are visible
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  auto run = [&](auto edge_c) {
+    constexpr bool EDGE = decltype(edge_c)::value;
+    StreamIo<TU, TV, EDGE> io;
+    io.mats = mats;
+    io.ring = ring;
+    io.ux = u_field<TU>(f, false, src);
+    io.uy = u_field<TU>(f, true, src);
+    io.uxo = u_field<TU>(f, false, src ^ 1);
+    io.uyo = u_field<TU>(f, true, src ^ 1);
+    io.vx = static_cast<TV*>(f.vx);
+    io.vy = static_cast<TV*>(f.vy);
+    io.mask = f.mask;
+    io.nx = g.nx;
+    io.ny = g.ny;
+    io.pitch = g.pitch;
+    io.strip = strip;
+    io.i = i;
+    io.jA = jA;
+    io.jB = jB;
+    io.npairs = (jB - jA + 1) / 2;
+    io.own = lane >= 2 && lane < 2 + STREAM_COLS && (!EDGE || i < g.nx);
+#pragma unroll 1
+    for (int k = 0; k < PAIR_DEPTH; k++) {
+      if (k <= io.npairs + 1) io.issue(k, k);
+      cp_async_commit();
+    }
+    // FP32 has the registers for two steps per turn (2048^2 40.4 -> 34.5 us); FP64 gains nothing
+    constexpr int UNROLL = sizeof(TU) == 4 ? 2 : 1;
+    pair_march<TU, TV, PLASTIC, EDGE, 0, false, UNROLL>(g, io, io.npairs, i, jA);
+  };
+  if (stream_interior(g.nx, g.ny, strip, jA, jB + 1)) run(std::false_type{});
+  else run(std::true_type{});
 }
 
 }  // namespace ep2d

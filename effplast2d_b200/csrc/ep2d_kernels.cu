@@ -118,22 +118,24 @@ int occupancy_ty(bool record) {
   return e == cudaSuccess && n > 0 ? n : 1;
 }
 
-template <int PLASTIC, int JOBS, typename TV, bool TRACK = false>
+template <int PLASTIC, int JOBS, typename T, typename TV, bool TRACK = false>
 cudaError_t set_chip_attr() {
-  return cudaFuncSetAttribute(k_iter_chip<PLASTIC, JOBS, TV, TRACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, CHIP_SMEM);
+  return cudaFuncSetAttribute(k_iter_chip<PLASTIC, JOBS, T, TV, TRACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, CHIP_SMEM);
 }
 
 template <typename TV>
 cudaError_t set_chip_attrs() {
   cudaError_t e;
-  if ((e = set_chip_attr<0, 1, TV>()) != cudaSuccess) return e;
-  if ((e = set_chip_attr<1, 1, TV>()) != cudaSuccess) return e;
-  if ((e = set_chip_attr<1, 1, TV, true>()) != cudaSuccess) return e;
-  return set_chip_attr<2, CHIP_JOBS, TV>();
+  if ((e = set_chip_attr<0, 1, double, TV>()) != cudaSuccess) return e;
+  if ((e = set_chip_attr<1, 1, double, TV>()) != cudaSuccess) return e;
+  if ((e = set_chip_attr<1, 1, double, TV, true>()) != cudaSuccess) return e;
+  return set_chip_attr<2, CHIP_JOBS, double, TV>();
 }
 
 cudaError_t prepare_kernels_impl() {
   cudaError_t e;
+  if ((e = set_chip_attr<0, 1, float, float>()) != cudaSuccess) return e;
+  if ((e = set_chip_attr<1, 1, float, float>()) != cudaSuccess) return e;
   if ((e = set_chip_attrs<double>()) != cudaSuccess) return e;
   if ((e = set_chip_attrs<float>()) != cudaSuccess) return e;
   if ((e = set_attrs_ty<8, double>()) != cudaSuccess) return e;
@@ -172,6 +174,12 @@ cudaError_t launch_stream_tv(const Geo& g, const Fields& f, int src, bool plasti
   const int blocks = (nstrips * nsegs + STREAM_WARPS - 1) / STREAM_WARPS;
   const int threads = 32 * STREAM_WARPS;
   const size_t sm = stream_smem_bytes<TU, TV>();
+  // plain launches take the pair march; its offsets are 32-bit bytes
+  if (!record && !(track && plastic) && (uint64_t)g.pitch * (g.ny + 1) * sizeof(TU) < ((uint64_t)1 << 32)) {
+    const size_t sp = stream_pair_smem_bytes<TU, TV>();
+    if (plastic) return launch_overlapped(k_iter_pairs<true, TU, TV>, blocks, threads, sp, stream, g, f, src, nstrips, nsegs, seg_h);
+    return launch_overlapped(k_iter_pairs<false, TU, TV>, blocks, threads, sp, stream, g, f, src, nstrips, nsegs, seg_h);
+  }
   if constexpr (std::is_same<TU, double>::value) {
     if (track && plastic) {
       if (record)
@@ -294,7 +302,7 @@ ChipShape chip_shape(int nx, int ny) {
 
 size_t chip_rim_bytes(int nx, int ny, int warps, int rows) {
   const size_t ncx = (nx + STREAM_COLS - 1) / STREAM_COLS, ncy = (ny + warps * rows - 1) / (warps * rows);
-  return 2 * RIM_BYTES * ncx * ncy * (4 * (size_t)warps * rows + 4 * STREAM_COLS);
+  return 2 * RimRecord<double>::BYTES * ncx * ncy * (4 * (size_t)warps * rows + 4 * STREAM_COLS);
 }
 
 // 4 records per row of padded height and 4 x STREAM_COLS per tile: the shortest tiles of at
@@ -332,8 +340,8 @@ cudaError_t launch_chip_jobs(const ChipJob* jobs, int njobs, const void* kern, c
 }  // namespace
 
 cudaError_t launch_iter_chip(ChipJob* jobs, int njobs, bool mixed, const ChipShape& s, int n_iter,
-                             unsigned long long timeout_ns, cudaStream_t stream, bool track) {
-  if (njobs < 1 || njobs > CHIP_JOBS || (track && njobs > 1) || n_iter < 2 || s.warps < 1 || s.groups < 1 ||
+                             unsigned long long timeout_ns, cudaStream_t stream, bool track, bool f32) {
+  if (njobs < 1 || njobs > CHIP_JOBS || ((track || f32) && njobs > 1) || n_iter < 2 || s.warps < 1 || s.groups < 1 ||
       s.warps * s.groups > CHIP_WARPS || s.rows < 2 || s.rows > 18 || (s.rows & 1) ||
       chip_smem_bytes(s.groups, s.warps, s.rows, track) > CHIP_SMEM)
     return cudaErrorInvalidValue;
@@ -350,15 +358,19 @@ cudaError_t launch_iter_chip(ChipJob* jobs, int njobs, bool mixed, const ChipSha
   }
   if (njobs == 1) {
     const bool pl = jobs[0].plastic != 0;
+    if (f32)
+      return launch_chip_jobs<1>(jobs, 1, pl ? (const void*)k_iter_chip<1, 1, float, float>
+                                             : (const void*)k_iter_chip<0, 1, float, float>,
+                                 s, n_iter, blocks, timeout_ns, stream);
     if (track && pl)
-      return launch_chip_jobs<1>(jobs, 1, mixed ? (const void*)k_iter_chip<1, 1, float, true>
-                                                : (const void*)k_iter_chip<1, 1, double, true>,
+      return launch_chip_jobs<1>(jobs, 1, mixed ? (const void*)k_iter_chip<1, 1, double, float, true>
+                                                : (const void*)k_iter_chip<1, 1, double, double, true>,
                                  s, n_iter, blocks, timeout_ns, stream, true);
-    const void* kern = mixed ? (pl ? (const void*)k_iter_chip<1, 1, float> : (const void*)k_iter_chip<0, 1, float>)
-                             : (pl ? (const void*)k_iter_chip<1, 1, double> : (const void*)k_iter_chip<0, 1, double>);
+    const void* kern = mixed ? (pl ? (const void*)k_iter_chip<1, 1, double, float> : (const void*)k_iter_chip<0, 1, double, float>)
+                             : (pl ? (const void*)k_iter_chip<1, 1, double, double> : (const void*)k_iter_chip<0, 1, double, double>);
     return launch_chip_jobs<1>(jobs, 1, kern, s, n_iter, blocks, timeout_ns, stream);
   }
-  const void* kern = mixed ? (const void*)k_iter_chip<2, CHIP_JOBS, float> : (const void*)k_iter_chip<2, CHIP_JOBS, double>;
+  const void* kern = mixed ? (const void*)k_iter_chip<2, CHIP_JOBS, double, float> : (const void*)k_iter_chip<2, CHIP_JOBS, double, double>;
   return launch_chip_jobs<CHIP_JOBS>(jobs, njobs, kern, s, n_iter, blocks, timeout_ns, stream);
 }
 

@@ -93,11 +93,25 @@ IterShape shape_of(const ep2d_params& p, int sm_count) {
   if (p.rows == 0 && s.form == FORM_STREAM && sm_count > 0) {
     const int64_t strips = (p.nx + STREAM_COLS - 1) / STREAM_COLS, sms = sm_count;
     auto warps = [&](int rows) { return strips * ((p.ny + rows - 1) / rows); };  // one per segment
-    // Segment height: the tallest power of two from 64 down that gives 16 warps of
+    // Segment height: as many rows as fill one wave of 16 warps per SM exactly, or two or more
+    // waves where that would be above 96 rows (us per iteration, NL=3: 1200^2 24 rows 19.8, 16 rows
+    // 21.4; 1536^2 37 rows 30.6, 32 rows 37.7; 1800^2 50 rows 40.6, 64 rows 49.6; 2600^2 53 rows
+    // 89.3, 105 rows 95.1; 4096^2 86 rows 214.7, 256 rows 228.7).
+    const int64_t per_wave = 16 * sms / strips;  // segments of a strip
+    if (per_wave >= 1) {
+      int64_t waves = 1;
+      while ((p.ny + waves * per_wave - 1) / (waves * per_wave) > 96) waves++;
+      const int64_t h = (p.ny + waves * per_wave - 1) / (waves * per_wave);
+      if (h >= 16) {
+        s.rows = (int)h;
+        return s;
+      }
+    }
+    // Grids with fewer rows for it: the tallest power of two from 64 down that gives 16 warps of
     // segments per SM; below 16 rows the march's three extra rows per segment weigh more
-    // (75 % at 4 rows), so 8 rows stay while they give 9 warps per SM.  Measured, us per
-    // iteration, NL=3: 1024^2 16 rows 16.3 (8: 18.2); 768^2 8 rows 14.3 (16: 16.1);
-    // 640^2 8 rows 9.6 (4: 10.7); 576^2 8 rows 9.6 (4: 9.9); 512^2 4 rows 8.8 (8: 9.5).
+    // (75 % at 4 rows), so 8 rows stay while they give 9 warps per SM.  Measured (k_iter_stream),
+    // us per iteration, NL=3: 768^2 8 rows 14.3 (16: 16.1); 640^2 8 rows 9.6 (4: 10.7); 576^2 8
+    // rows 9.6 (4: 9.9); 512^2 4 rows 8.8 (8: 9.5).
     s.rows = 64;
     while (s.rows > SEG_MIN && warps(s.rows) < (s.rows > 8 ? 16 : 9) * sms) s.rows /= 2;
     // Too few 4-row segments to keep the SMs busy: a warp's march latency then sets the
@@ -322,9 +336,11 @@ size_t n_samples(const ep2d_params& p) {
 // the on-chip form is taken only where the parameters leave the kernel to the library
 bool chip_allowed(const ep2d_params& p) { return p.kernel == EP2D_KERNEL_AUTO && p.rows == 0; }
 // the stress arrays are contiguous, and those a recording launch writes (p to txy; with the
-// return map also txyav, j2, j2xy) hold the rim records of a run if they can
+// return map also txyav, j2, j2xy) hold the rim records of a run if they can; an FP32 run need
+// not be followed by a launch that writes them
 size_t own_rim_bytes(const ep2d_params& p) {
   const size_t need = chip_allowed(p) ? chip_rim_capacity(p.nx, p.ny) : 0;
+  if (p.precision == EP2D_F32_BULK) return align256(need);
   return need > (p.nl > 1 ? 7 : 4) * align256(field_elems(p) * sizeof(double)) ? align256(need) : 0;
 }
 
@@ -640,7 +656,8 @@ int Rve::run_chip(int64_t n, bool* done) {
     // chunks of an even length keep the parity; a chunk of one iteration cannot arise
     const int64_t chunk = n > ((int64_t)1 << 30) ? (int64_t)1 << 29 : n;
     ChipJob job = chip_job(f.gbar + 2);
-    const cudaError_t e = launch_iter_chip(&job, 1, mixed(), chip, (int)chunk, CHIP_TIMEOUT_NS, stream, track);
+    const cudaError_t e = launch_iter_chip(&job, 1, mixed(), chip, (int)chunk, CHIP_TIMEOUT_NS, stream,
+                                           track && !f32, f32);
     if (e == cudaErrorCooperativeLaunchTooLarge) {
       cudaGetLastError();
       chip = ChipShape{};
@@ -658,8 +675,8 @@ int Rve::run_chip(int64_t n, bool* done) {
 }
 
 int Rve::run_plain(int64_t n) {
-  if (chip.warps && n >= CHIP_MIN_RUN && !f32 &&
-      (!track || chip_smem(chip.groups, chip.warps, chip.rows, true) <= CHIP_SMEM)) {
+  if (chip.warps && n >= CHIP_MIN_RUN &&
+      (!track || f32 || chip_smem(chip.groups, chip.warps, chip.rows, true) <= CHIP_SMEM)) {
     bool done = false;
     const int rc = run_chip(n, &done);
     if (rc || done) return rc;

@@ -147,9 +147,11 @@ size_t chip_smem(int groups, int warps, int rows, bool track = false);
 // n_iter >= 2 plain iterations of the jobs' RVEs in one cooperative launch: CTAs of s.groups tiles of
 // s.warps x s.rows (s.ncx, s.ncy unused); fills in the jobs' tiles and CTAs.  Each wait gives up
 // after timeout_ns, which sets the job's flag
-// (track: also mark what yields, as launch_iter does; one job)
+// (track: also mark what yields, as launch_iter does; f32: the FP32 bulk's iterations, on
+// f.ux32/uy32; one job each)
 cudaError_t launch_iter_chip(ChipJob* jobs, int njobs, bool mixed, const ChipShape& s, int n_iter,
-                             unsigned long long timeout_ns, cudaStream_t stream, bool track = false);
+                             unsigned long long timeout_ns, cudaStream_t stream, bool track = false,
+                             bool f32 = false);
 // clear the M_YN / M_YC bits of every node
 cudaError_t launch_clear_track(const Geo& g, uint8_t* mask, cudaStream_t stream);
 // one iteration of the FP32 bulk (stream form, segments of seg_h rows): u' and V in

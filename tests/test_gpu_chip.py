@@ -76,6 +76,41 @@ def test_chip_tracking_matches_stream_tracking(nx, ny, precision):
         assert np.array_equal(out[0][k], out[1][k]), k
 
 
+@pytest.mark.parametrize("rows", [4, 5, 19, 37, 200])
+@pytest.mark.parametrize("nl,precision", [(1, ep.FP64), (3, ep.FP64), (2, ep.MIXED)], ids=["elastic", "plastic", "mixed"])
+def test_stream_pairs_match_tile_form(rows, nl, precision):
+    # the stream form's plain launches march two rows per step: odd and even segments, the last
+    # one cut short, interior and edge segments, a ragged last strip
+    nx, ny = 203, 181
+    pa = _pa(nx, ny, n_pores=3, porosity=0.03, yield_stress=1e-5)
+    st = _random_state(nx, ny, 43)
+    a, _ = _run(nx, ny, pa, nl, st, (70, 2), precision, kernel=ep.KERNEL_TILE, rows=16)
+    b, _ = _run(nx, ny, pa, nl, st, (70, 2), precision, kernel=ep.KERNEL_STREAM, rows=rows)
+    for f in a:
+        assert np.array_equal(b[f], a[f]), (f, float(np.max(np.abs(b[f] - a[f]))))
+
+
+@pytest.mark.parametrize("nx,ny", [(8, 9), (57, 130), (403, 401), (1061, 1060)])
+@pytest.mark.parametrize("nl", [1, 2])
+def test_chip_f32_matches_stream_f32(nx, ny, nl):
+    # the FP32 bulk's iterations on chip against single launches of the stream form; the
+    # recorded stresses are left alone
+    pa = _pa(nx, ny, n_pores=1, porosity=0.02, yield_stress=1e-5)
+    out = []
+    for kw in (dict(kernel=ep.KERNEL_STREAM, rows=16), {}):
+        s = ep.Solver(nx, ny, pa, nl=nl, niter=40, check_every=40, precision=ep.F32_BULK, **kw)
+        s.solve_step(0, -6e-5, [1.0, 0.8, 0.3])
+        p = s.get("P")
+        for n in (41, 30):
+            s.iterate_f32(n)
+        assert np.array_equal(s.get("P"), p)
+        out.append({f: s.get(f) for f in ("Ux", "Uy", "Vx", "Vy")})
+        s.close()
+    for f in out[0]:
+        assert np.max(np.abs(out[0][f])) > 0.0
+        assert np.array_equal(out[0][f], out[1][f]), f
+
+
 def test_chip_form_two_threads():
     # on-chip launches of different handles take turns; both finish with the single-thread result
     nx = ny = 200
