@@ -253,8 +253,12 @@ struct ChipIo {
 // its neighbours have read it).  CTAs of groups of a.warps warps, a group per tile, a.rows rows per
 // warp.  rim: records [2][tile][4 H + 112 cells].  PLASTIC 0, 1: all jobs; 2: per job.
 // TRACK: also mark the nodes and corners that yield at any of the iterations (M_YN, M_YC).
-template <int PLASTIC, int JOBS, typename T, typename TV, bool TRACK = false>
-__global__ void __launch_bounds__(32 * CHIP_WARPS, 1) k_iter_chip(const __grid_constant__ ChipArgs<JOBS> a) {
+// WARPS: the most warps of a CTA.  A shape of 8 or 12 warps per SM leaves the march 255 or 168
+// registers instead of 128, and the unrolled rows overlap better (us per iteration: 128^2
+// elastic 1.63 -> 1.50, NL=3 2.28 -> 2.10 with 4 warps; 256^2 2.66 -> 2.56, 512^2 elastic 2.40 ->
+// 2.29, NL=3 4.10 -> 3.96 with 10 and 12).
+template <int PLASTIC, int JOBS, typename T, typename TV, bool TRACK = false, int WARPS = CHIP_WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_constant__ ChipArgs<JOBS> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t s_tmem;
   using U2 = Vec2<T>;

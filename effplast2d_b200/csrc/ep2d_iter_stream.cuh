@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(32 * STREAM_WARPS) k_iter_stream_batch(const B
 // ---- plain launches of one RVE: the pair march over a ring of row pairs -------------------
 // Two rows per step (ep2d_march.cuh), the rows in a per-warp ring of row pairs filled by
 // cp.async, PAIR_DEPTH pairs ahead of use: pair k is read at step k (U of its rows) and at
-// step k + 1 (old U and V of the faces), and its slot is refilled after that.  3 pairs ahead
+// step k + 1 (V of the faces), and its slot is refilled after that.  3 pairs ahead
 // measured slower (2048^2 58.6 us an iteration against 53.3: less L1 beside the larger rings).
 // Offsets into a field are 32-bit bytes from its base (fields of 4 GB and more stay with
 // k_iter_stream): a store or copy then needs no 64-bit address arithmetic (53.3 -> 52.5).
@@ -494,6 +494,7 @@ struct StreamIo {
   const uint8_t* mask;
   int nx, ny, pitch, strip, i, jA, jB, npairs;
   bool own;
+  U2 cur_a, cur_b, old_a, old_b;  // this column's U of the rows read at this step and at the one before
   int mk_c = 0;     // mask byte of the last row of the previous step
   int mk_a = 0, mk_b = 0;
   int slot = PAIR_SLOTS - 1;  // slot of the pair read at this step
@@ -542,7 +543,7 @@ struct StreamIo {
     mk_a = mask_byte(d, 0, jA - 2 + 2 * p);
     mk_b = mask_byte(d, 1, jA - 1 + 2 * p);
   }
-  __device__ __forceinline__ void rows(int, U2& ua, U2& uar, U2& ub, U2& ubr) const {
+  __device__ __forceinline__ void rows(int, U2& ua, U2& uar, U2& ub, U2& ubr) {
     const StreamPair<TU, TV>& d = ring[slot];
     const int lane = threadIdx.x & 31, ln1 = min(lane + 1, 31);
     ua.x = d.ux[0][lane];
@@ -553,6 +554,10 @@ struct StreamIo {
     ub.y = d.uy[1][lane];
     ubr.x = d.ux[1][ln1];
     ubr.y = d.uy[1][ln1];
+    old_a = cur_a;
+    old_b = cur_b;
+    cur_a = ua;
+    cur_b = ub;
   }
   __device__ __forceinline__ const MatT<TU>& mat(int, int r) const {
     const int m = r ? mk_a : mk_c, up = r ? mk_b : mk_a;
@@ -561,10 +566,8 @@ struct StreamIo {
   __device__ __forceinline__ void old(int, U2& u0, U2& u1, TV (&v)[4]) const {
     const StreamPair<TU, TV>& d = ring[slot ? slot - 1 : PAIR_SLOTS - 1];
     const int lane = threadIdx.x & 31;
-    u0.x = d.ux[0][lane];
-    u0.y = d.uy[0][lane];
-    u1.x = d.ux[1][lane];
-    u1.y = d.uy[1][lane];
+    u0 = old_a;
+    u1 = old_b;
     v[0] = d.vx[0][lane];
     v[1] = d.vy[0][lane];
     v[2] = d.vx[1][lane];

@@ -118,26 +118,21 @@ int occupancy_ty(bool record) {
   return e == cudaSuccess && n > 0 ? n : 1;
 }
 
-template <int PLASTIC, int JOBS, typename T, typename TV, bool TRACK = false>
-cudaError_t set_chip_attr() {
-  return cudaFuncSetAttribute(k_iter_chip<PLASTIC, JOBS, T, TV, TRACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, CHIP_SMEM);
-}
-
-template <typename TV>
-cudaError_t set_chip_attrs() {
-  cudaError_t e;
-  if ((e = set_chip_attr<0, 1, double, TV>()) != cudaSuccess) return e;
-  if ((e = set_chip_attr<1, 1, double, TV>()) != cudaSuccess) return e;
-  if ((e = set_chip_attr<1, 1, double, TV, true>()) != cudaSuccess) return e;
-  return set_chip_attr<2, CHIP_JOBS, double, TV>();
+const void* chip_kernel(bool plastic, bool mixed, bool track, int warps);
+cudaError_t set_chip_attr(const void* kern) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CHIP_SMEM);
 }
 
 cudaError_t prepare_kernels_impl() {
   cudaError_t e;
-  if ((e = set_chip_attr<0, 1, float, float>()) != cudaSuccess) return e;
-  if ((e = set_chip_attr<1, 1, float, float>()) != cudaSuccess) return e;
-  if ((e = set_chip_attrs<double>()) != cudaSuccess) return e;
-  if ((e = set_chip_attrs<float>()) != cudaSuccess) return e;
+  for (int warps : {8, 12, 16})
+    for (int mixed = 0; mixed < 2; mixed++)
+      for (int form = 0; form < 3; form++)  // elastic, plastic, plastic with tracking
+        if ((e = set_chip_attr(chip_kernel(form > 0, mixed, form == 2, warps))) != cudaSuccess) return e;
+  for (const void* kern : {(const void*)k_iter_chip<0, 1, float, float>, (const void*)k_iter_chip<1, 1, float, float>,
+                           (const void*)k_iter_chip<2, CHIP_JOBS, double, float>,
+                           (const void*)k_iter_chip<2, CHIP_JOBS, double, double>})
+    if ((e = set_chip_attr(kern)) != cudaSuccess) return e;
   if ((e = set_attrs_ty<8, double>()) != cudaSuccess) return e;
   if ((e = set_attrs_ty<16, double>()) != cudaSuccess) return e;
   if ((e = set_attrs_ty<32, double>()) != cudaSuccess) return e;
@@ -323,6 +318,22 @@ int chip_ctas(int nx, int ny, int groups, int warps, int rows) {
 size_t chip_smem(int groups, int warps, int rows, bool track) { return chip_smem_bytes(groups, warps, rows, track); }
 
 namespace {
+template <typename TV, bool TRACK>
+const void* chip_kernel_of(bool plastic, int warps) {
+  if (TRACK || plastic)
+    return warps <= 8    ? (const void*)k_iter_chip<1, 1, double, TV, TRACK, 8>
+           : warps <= 12 ? (const void*)k_iter_chip<1, 1, double, TV, TRACK, 12>
+                         : (const void*)k_iter_chip<1, 1, double, TV, TRACK>;
+  return warps <= 8    ? (const void*)k_iter_chip<0, 1, double, TV, false, 8>
+         : warps <= 12 ? (const void*)k_iter_chip<0, 1, double, TV, false, 12>
+                       : (const void*)k_iter_chip<0, 1, double, TV>;
+}
+// the FP64 (mixed: FP32 velocities) kernel of one RVE for a shape of `warps` warps per CTA
+const void* chip_kernel(bool plastic, bool mixed, bool track, int warps) {
+  if (track) return mixed ? chip_kernel_of<float, true>(true, warps) : chip_kernel_of<double, true>(true, warps);
+  return mixed ? chip_kernel_of<float, false>(plastic, warps) : chip_kernel_of<double, false>(plastic, warps);
+}
+
 template <int JOBS>
 cudaError_t launch_chip_jobs(const ChipJob* jobs, int njobs, const void* kern, const ChipShape& s, int n_iter, int blocks,
                              unsigned long long timeout_ns, cudaStream_t stream, bool track = false) {
@@ -358,17 +369,9 @@ cudaError_t launch_iter_chip(ChipJob* jobs, int njobs, bool mixed, const ChipSha
   }
   if (njobs == 1) {
     const bool pl = jobs[0].plastic != 0;
-    if (f32)
-      return launch_chip_jobs<1>(jobs, 1, pl ? (const void*)k_iter_chip<1, 1, float, float>
-                                             : (const void*)k_iter_chip<0, 1, float, float>,
-                                 s, n_iter, blocks, timeout_ns, stream);
-    if (track && pl)
-      return launch_chip_jobs<1>(jobs, 1, mixed ? (const void*)k_iter_chip<1, 1, double, float, true>
-                                                : (const void*)k_iter_chip<1, 1, double, double, true>,
-                                 s, n_iter, blocks, timeout_ns, stream, true);
-    const void* kern = mixed ? (pl ? (const void*)k_iter_chip<1, 1, double, float> : (const void*)k_iter_chip<0, 1, double, float>)
-                             : (pl ? (const void*)k_iter_chip<1, 1, double, double> : (const void*)k_iter_chip<0, 1, double, double>);
-    return launch_chip_jobs<1>(jobs, 1, kern, s, n_iter, blocks, timeout_ns, stream);
+    const void* kern = f32 ? (pl ? (const void*)k_iter_chip<1, 1, float, float> : (const void*)k_iter_chip<0, 1, float, float>)
+                           : chip_kernel(pl, mixed, track && pl, s.warps * s.groups);
+    return launch_chip_jobs<1>(jobs, 1, kern, s, n_iter, blocks, timeout_ns, stream, track && pl && !f32);
   }
   const void* kern = mixed ? (const void*)k_iter_chip<2, CHIP_JOBS, double, float> : (const void*)k_iter_chip<2, CHIP_JOBS, double, double>;
   return launch_chip_jobs<CHIP_JOBS>(jobs, njobs, kern, s, n_iter, blocks, timeout_ns, stream);
