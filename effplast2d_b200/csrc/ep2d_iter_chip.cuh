@@ -296,11 +296,14 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_consta
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  // the recording launch that follows folds max|V| into the pair
+  if ((int)blockIdx.x == job.cta0 && threadIdx.x < 2) f.vmax[threadIdx.x] = 0;
   for (int t = threadIdx.x; t < N_MATS; t += blockDim.x) mats[t] = mat_entry<T>(g, t);
   __syncthreads();
   if (!idle) {
     const int i = x0 - 2 + lane;
     const int jA = y0 + w * rows;
+#pragma unroll 4
     for (int r = w; r < H + 3; r += nw) idx[r * 32 + lane] = (uint8_t)chip_index(g, f.mask, i, y0 - 2 + r);
 
     // U of the tile and its halo, both copies of the double-buffered rows (faces outside the
@@ -316,6 +319,7 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_consta
     char* own = urows + w * ppw * PAIR;
     if (TRACK)
       for (int r = 0; r < rows; r++) yielded[r * 32 + lane] = 0;
+#pragma unroll 4
     for (int r = 0; r < rows; r++) {
       const U2 u = load_u(jA + r);
       for (int par = 0; par < 2; par++)

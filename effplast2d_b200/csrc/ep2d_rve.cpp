@@ -650,7 +650,7 @@ ChipJob Rve::chip_job(unsigned* flag) const {
 // n plain iterations in one launch of the on-chip form; *done = false where the device has no
 // room for its CTAs (the other forms take over for good).
 int Rve::run_chip(int64_t n, bool* done) {
-  std::lock_guard<std::mutex> turn(chip_turn(device));
+  if (!turn_.owns_lock()) turn_ = std::unique_lock<std::mutex>(chip_turn(device));
   *done = true;
   while (n > 0) {
     // chunks of an even length keep the parity; a chunk of one iteration cannot arise
@@ -670,8 +670,18 @@ int Rve::run_chip(int64_t n, bool* done) {
     resident_launches++;
     n -= chunk;
   }
-  EP2D_CK(cudaStreamSynchronize(stream));
+  vmax_zero_ = true;
   return EP2D_OK;
+}
+
+// the stream is idle: another handle may have the turn
+void Rve::end_turn() {
+  if (turn_.owns_lock()) turn_.unlock();
+}
+Rve::TurnScope::~TurnScope() {
+  if (!r.turn_.owns_lock()) return;
+  cudaStreamSynchronize(r.stream);  // an error shows again at the next call
+  r.turn_.unlock();
 }
 
 int Rve::run_plain(int64_t n) {
@@ -712,6 +722,10 @@ int Rve::run_plain(int64_t n) {
 }
 
 int Rve::reset_vmax() {
+  if (vmax_zero_) {
+    vmax_zero_ = false;
+    return EP2D_OK;
+  }
   EP2D_CK(cudaMemsetAsync(f.vmax, 0, 2 * sizeof(unsigned long long), stream));
   return EP2D_OK;
 }
@@ -719,6 +733,7 @@ int Rve::reset_vmax() {
 int Rve::iterate(int64_t n, bool record_last) {
   if (n <= 0) return EP2D_OK;
   DeviceScope ds(device);
+  TurnScope ts{*this};
   EP2D_CK(cudaEventRecord(ev_[0], stream));
   int rc = run_plain(record_last ? n - 1 : n);
   if (rc) return rc;
@@ -729,13 +744,17 @@ int Rve::iterate(int64_t n, bool record_last) {
     if (rc) return rc;
     launches++;
   }
+  vmax_zero_ = false;
   EP2D_CK(cudaEventRecord(ev_[1], stream));
+  rc = check_resident();  // waits for the stream, if it has a flag to read
+  if (rc) return rc;
   EP2D_CK(cudaEventSynchronize(ev_[1]));
+  end_turn();
   float ms = 0.0f;
   EP2D_CK(cudaEventElapsedTime(&ms, ev_[0], ev_[1]));
   kernel_ms += ms;
   cell_updates += n * (int64_t)prm.nx * prm.ny;
-  return check_resident();
+  return EP2D_OK;
 }
 
 double Rve::error_from_vmax(double vmx, double vmy) const {
@@ -745,6 +764,10 @@ double Rve::error_from_vmax(double vmx, double vmy) const {
   return (vmx / (d.dX * (prm.nx - 1)) + vmy / (d.dY * (prm.ny - 1))) * d.dT / std::max(a, b);
 }
 
+static int failed_wait() {
+  return fail(EP2D_ERR_CUDA, "resident or on-chip form: a wait for another CTA ran out; the RVE's state is invalid");
+}
+
 // The error flag of the forms whose CTAs wait on one another (sticky), read back; EP2D_OK if
 // the RVE never ran one.
 int Rve::check_resident() {
@@ -752,20 +775,16 @@ int Rve::check_resident() {
   unsigned* hf = reinterpret_cast<unsigned*>(h_pin + 2 * NAVG + holes.size() + 2);
   EP2D_CK(cudaMemcpyAsync(hf, f.gbar + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
   EP2D_CK(cudaStreamSynchronize(stream));
-  if (*hf)
-    return fail(EP2D_ERR_CUDA,
-                "resident or on-chip form: a wait for another CTA ran out; the RVE's state is invalid");
-  return EP2D_OK;
+  return *hf ? failed_wait() : EP2D_OK;
 }
 
 int Rve::read_error(double* error) {
+  // the max|V| pair and, right behind it, the barrier words with the error flag (check_resident)
   unsigned long long* hv = reinterpret_cast<unsigned long long*>(h_pin + 2 * NAVG + holes.size());
-  EP2D_CK(cudaMemcpyAsync(hv, f.vmax, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
+  EP2D_CK(cudaMemcpyAsync(hv, f.vmax, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
   EP2D_CK(cudaStreamSynchronize(stream));
-  {
-    const int rc = check_resident();
-    if (rc) return rc;
-  }
+  end_turn();
+  if (resident_launches && reinterpret_cast<unsigned*>(hv + 3)[0]) return failed_wait();
   double vmx, vmy;
   std::memcpy(&vmx, &hv[0], sizeof(double));
   std::memcpy(&vmy, &hv[1], sizeof(double));
@@ -869,6 +888,7 @@ void Rve::finish_chain(int n_time_steps, ep2d_result* out) {
 int Rve::solve_step(int step, double lsv, const double lt[3], int n_time_steps) {
   if (!lt) return fail(EP2D_ERR_ARG, "load_type is null");
   DeviceScope ds(device);
+  TurnScope ts{*this};
   int rc0 = begin_step(step, n_time_steps);
   if (rc0) return rc0;
   const int64_t ce = prm.check_every;
@@ -886,6 +906,7 @@ int Rve::solve_step(int step, double lsv, const double lt[3], int n_time_steps) 
     double error = 0.0;
     int64_t iter = 0, iters = prm.niter;
     int converged = 0;
+    bool flag_read = false;  // the last interval ended with a checkpoint, which read the error flag
     EP2D_CK(cudaEventRecord(ev_[0], stream));
     while (iter < prm.niter) {
       const int64_t block_end = std::min<int64_t>(prm.niter, (iter / ce + 1) * ce);
@@ -904,9 +925,11 @@ int Rve::solve_step(int step, double lsv, const double lt[3], int n_time_steps) 
       launches++;
       if (in_f32) f32_iterations += block_end - iter;
       iter = block_end;
+      flag_read = false;
       if (iter % ce == 0) {
         rc = read_error(&error);
         if (rc) return rc;
+        flag_read = true;
         checks[step][it].push_back(error);
         r.n_checks++;
         if (in_f32) {
@@ -938,8 +961,9 @@ int Rve::solve_step(int step, double lsv, const double lt[3], int n_time_steps) 
     EP2D_CK(cudaEventElapsedTime(&ms, ev_[0], ev_[1]));
     kernel_ms += ms;
     cell_updates += iters * (int64_t)prm.nx * prm.ny;
-    rc = check_resident();  // the last interval may end without a checkpoint
+    if (!flag_read) rc = check_resident();
     if (rc) return rc;
+    end_turn();
     r.iterations = iters;
     r.converged = converged;
     r.error = error;

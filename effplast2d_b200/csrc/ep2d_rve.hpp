@@ -184,6 +184,15 @@ class Rve {
  private:
   int run_plain(int64_t n);
   int run_chip(int64_t n, bool* done);
+  // this handle's turn for on-chip launches (chip_turn): taken by run_chip, given back once the
+  // stream has been waited for -- by end_turn at the latest when iterate or solve_step returns
+  std::unique_lock<std::mutex> turn_;
+  void end_turn();
+  struct TurnScope {
+    Rve& r;
+    ~TurnScope();
+  };
+  bool vmax_zero_ = false;  // an on-chip launch has just zeroed the max|V| pair
   int capture(int parity);
   cudaGraphExec_t gexec_[2] = {nullptr, nullptr};
   cudaGraphExec_t gexec32_[2] = {nullptr, nullptr};  // FP32 bulk (hold the affine strains)
