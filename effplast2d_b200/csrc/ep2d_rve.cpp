@@ -395,13 +395,37 @@ void Rve::release() {
         ev = nullptr;
       }
     if (stream) cudaStreamSynchronize(stream);
+    if (scratch_) cudaFree(scratch_);
     if (dmem) cudaFree(dmem);
     if (h_pin) cudaFreeHost(h_pin);
     if (own_stream && stream) cudaStreamDestroy(stream);
   }
+  scratch_ = nullptr;
+  scratch_bytes_ = 0;
   dmem = nullptr;
   h_pin = nullptr;
   stream = nullptr;
+}
+
+cudaError_t Rve::scratch_get(size_t bytes, double** p) {
+  *p = nullptr;
+  if (bytes > kKeepScratch) return cudaMallocAsync(reinterpret_cast<void**>(p), bytes, stream);
+  if (scratch_bytes_ < bytes) {
+    if (scratch_) cudaFree(scratch_);  // waits for the work that uses it
+    scratch_ = nullptr;
+    scratch_bytes_ = 0;
+    const cudaError_t e = cudaMalloc(&scratch_, bytes);
+    if (e != cudaSuccess) {
+      scratch_ = nullptr;
+      return e;
+    }
+    scratch_bytes_ = bytes;
+  }
+  *p = static_cast<double*>(scratch_);
+  return cudaSuccess;
+}
+void Rve::scratch_put(double* p) {
+  if (p && p != scratch_) cudaFreeAsync(p, stream);
 }
 
 int Rve::create(const ep2d_params& p, cudaStream_t s) {
@@ -1117,12 +1141,12 @@ int Rve::static_fields(double* unu, double* j1, double* j2) {
   DeviceScope ds(device);
   const size_t nn = (size_t)prm.nx * prm.ny, nc = (size_t)(prm.nx - 1) * (prm.ny - 1);
   double* tmp = nullptr;
-  EP2D_CK(cudaMallocAsync(&tmp, (nn + 2 * nc) * sizeof(double), stream));
+  EP2D_CK(scratch_get((nn + 2 * nc) * sizeof(double), &tmp));
   cudaError_t e = launch_static_fields(g, f, cur, tmp, tmp + nn, tmp + nn + nc, stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(unu, tmp, nn * sizeof(double), cudaMemcpyDeviceToHost, stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(j1, tmp + nn, nc * sizeof(double), cudaMemcpyDeviceToHost, stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(j2, tmp + nn + nc, nc * sizeof(double), cudaMemcpyDeviceToHost, stream);
-  cudaFreeAsync(tmp, stream);
+  scratch_put(tmp);
   cudaError_t se = cudaStreamSynchronize(stream);
   if (e != cudaSuccess || se != cudaSuccess)
     return fail(EP2D_ERR_CUDA, std::string("static fields: ") + cudaGetErrorString(e != cudaSuccess ? e : se));
@@ -1136,14 +1160,14 @@ int Rve::polar_fields(double load_value, double* snrr, double* snff, double* sar
   // sign(loadValue), get_sigma_2D.m:175 (MATLAB sign: 0 for 0)
   const double sgn = load_value > 0.0 ? 1.0 : (load_value < 0.0 ? -1.0 : 0.0);
   double* tmp = nullptr;
-  EP2D_CK(cudaMallocAsync(&tmp, 4 * nn * sizeof(double) + nn, stream));
+  EP2D_CK(scratch_get(4 * nn * sizeof(double) + nn, &tmp));
   uint8_t* pl = reinterpret_cast<uint8_t*>(tmp + 4 * nn);
   cudaError_t e = launch_polar_fields(g, f, sgn, tmp, tmp + nn, tmp + 2 * nn, tmp + 3 * nn, pl, tracked, stream);
   double* outs[4] = {snrr, snff, sarr, saff};
   for (int k = 0; k < 4 && e == cudaSuccess; k++)
     e = cudaMemcpyAsync(outs[k], tmp + k * nn, nn * sizeof(double), cudaMemcpyDeviceToHost, stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(plast, pl, nn, cudaMemcpyDeviceToHost, stream);
-  cudaFreeAsync(tmp, stream);
+  scratch_put(tmp);
   cudaError_t se = cudaStreamSynchronize(stream);
   if (e != cudaSuccess || se != cudaSuccess)
     return fail(EP2D_ERR_CUDA, std::string("polar fields: ") + cudaGetErrorString(e != cudaSuccess ? e : se));
@@ -1178,7 +1202,7 @@ int Rve::analytic_fields(double deltaP, double tauInfty, double* uan, double* eu
   const size_t nn = (size_t)prm.nx * prm.ny, nc = (size_t)(prm.nx - 1) * (prm.ny - 1);
   const size_t nst = (size_t)ANALYTIC_BLOCKS * 8;
   double* tmp = nullptr;
-  EP2D_CK(cudaMallocAsync(&tmp, (3 * nn + 6 * nc + nst) * sizeof(double), stream));
+  EP2D_CK(scratch_get((3 * nn + 6 * nc + nst) * sizeof(double), &tmp));
   double* unu = tmp;
   double* j1nu = unu + nn;
   double* j2nu = j1nu + nc;
@@ -1200,7 +1224,7 @@ int Rve::analytic_fields(double deltaP, double tauInfty, double* uan, double* eu
             {st.data(), d_st, nst}};
   for (auto& c : cp)
     if (e == cudaSuccess) e = cudaMemcpyAsync(c.h, c.dd, c.n * sizeof(double), cudaMemcpyDeviceToHost, stream);
-  cudaFreeAsync(tmp, stream);
+  scratch_put(tmp);
   cudaError_t se = cudaStreamSynchronize(stream);
   if (e != cudaSuccess || se != cudaSuccess)
     return fail(EP2D_ERR_CUDA, std::string("analytic fields: ") + cudaGetErrorString(e != cudaSuccess ? e : se));

@@ -173,6 +173,14 @@ class Rve {
   int64_t aux_launches = 0;  // preload, averaging, boundary, gather, mask
   int64_t cell_updates = 0;
 
+  // temporary device memory of a post-processing call: kept with the handle up to
+  // kKeepScratch bytes, so that calls in a row do not map it anew, else for the call only
+  static constexpr size_t kKeepScratch = (size_t)24 << 20;  // 512^2 and below
+  void* scratch_ = nullptr;
+  size_t scratch_bytes_ = 0;
+  cudaError_t scratch_get(size_t bytes, double** p);
+  void scratch_put(double* p);
+
   // device scratch
   void* dmem = nullptr;
   double* d_partials = nullptr;
