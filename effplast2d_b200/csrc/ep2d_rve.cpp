@@ -9,6 +9,10 @@
 #include <limits>
 #include <mutex>
 #include <set>
+#include <thread>
+
+#include <sys/mman.h>
+#include <unistd.h>
 
 namespace ep2d {
 
@@ -1053,6 +1057,36 @@ void dims(int nx, int ny, int field, int* w, int* h) {
 }
 }  // namespace
 
+namespace {
+// Have the pages of a large output buffer present before the copy into it: the copy from the
+// device faults pages of fresh memory in one by one (2048^2, 34 MB: 7.5 ms, 1.6 ms into pages that
+// are present; 4.1 with this).  Four threads fault in a quarter each; a kernel that does not know
+// MADV_POPULATE_WRITE, or a buffer it refuses, leaves the copy to do it.  Contents are kept.
+void populate(void* p, size_t bytes) {
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+  constexpr size_t kLarge = (size_t)32 << 20;  // smaller ones come warm from the heap as a rule
+  constexpr int kThreads = 4;
+  if (bytes < kLarge) return;
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+  const uintptr_t a = ((uintptr_t)p + page - 1) & ~(page - 1), b = ((uintptr_t)p + bytes) & ~(page - 1);
+  const uintptr_t part = ((b - a) / kThreads + page - 1) & ~(page - 1);
+  auto work = [=](int k) {
+    const uintptr_t lo = a + k * part, hi = std::min(lo + part, b);
+    if (lo < hi) madvise(reinterpret_cast<void*>(lo), hi - lo, MADV_POPULATE_WRITE);
+  };
+  std::thread th[kThreads - 1];
+  int n = 0;
+  try {
+    for (; n < kThreads - 1; n++) th[n] = std::thread(work, n + 1);
+  } catch (const std::exception&) {  // no thread to be had: the copy faults the rest in
+  }
+  work(0);
+  for (int k = 0; k < n; k++) th[k].join();
+}
+}  // namespace
+
 int Rve::get_field(int field, double* host) const {
   if (!host || field < 0 || field >= EP2D_NFIELDS) return fail(EP2D_ERR_ARG, "bad field or null buffer");
   DeviceScope ds(device);
@@ -1092,6 +1126,7 @@ int Rve::get_field(int field, double* host) const {
     for (size_t k = 0; k < tmp.size(); k++) host[k] = tmp[k];
     return EP2D_OK;
   }
+  populate(host, (size_t)w * h * sizeof(double));
   EP2D_CK(cudaMemcpy2DAsync(host, (size_t)w * sizeof(double), src, pb, (size_t)w * sizeof(double), h,
                             cudaMemcpyDeviceToHost, stream));
   EP2D_CK(cudaStreamSynchronize(stream));
