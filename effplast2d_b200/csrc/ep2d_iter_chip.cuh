@@ -176,9 +176,6 @@ struct RimRecord<float> {
                  : "memory");
   }
 };
-// records a lane has in flight while it polls: 2 (3 and 4 cost the march registers, 128 being
-// all there are: 1024^2 9.85 -> 10.6 us an iteration)
-constexpr int kRimInFlight = 2;
 // where a warp's row pairs lie: pair q of its rows/2, copy `par` of the double-buffered ones
 template <typename T>
 __device__ __forceinline__ uint32_t chip_pair_off(int q, int npairs, int par) {
@@ -257,7 +254,11 @@ struct ChipIo {
 // registers instead of 128, and the unrolled rows overlap better (us per iteration: 128^2
 // elastic 1.63 -> 1.50, NL=3 2.28 -> 2.10 with 4 warps; 256^2 2.66 -> 2.56, 512^2 elastic 2.40 ->
 // 2.29, NL=3 4.10 -> 3.96 with 10 and 12).
-template <int PLASTIC, int JOBS, typename T, typename TV, bool TRACK = false, int WARPS = CHIP_WARPS>
+// FLY: records a lane has in flight while it polls.  Tiles of 10 rows per warp and more have
+// three per lane; in one go they cost one round trip (1024^2 10.08 -> 9.93 us an iteration; elastic RVEs
+// gain nothing: 5.82, 5.91).  Where
+// two do, a third costs 2 %, and a fourth spills the march.
+template <int PLASTIC, int JOBS, typename T, typename TV, bool TRACK = false, int WARPS = CHIP_WARPS, int FLY = 3>
 __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_constant__ ChipArgs<JOBS> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t s_tmem;
@@ -448,12 +449,12 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_consta
             if (lane < STREAM_COLS) put(4 * H + (2 + r) * STREAM_COLS + lane, rows - 2 + r, 2 + lane);
       }
       int failed = 0;
-      for (int t0 = 0; t0 < npoll && !failed; t0 += kRimInFlight) {
-        uint2 e[kRimInFlight];
-        RimRecord<T> rec[kRimInFlight];
-        bool wait[kRimInFlight];
+      for (int t0 = 0; t0 < npoll && !failed; t0 += FLY) {
+        uint2 e[FLY];
+        RimRecord<T> rec[FLY];
+        bool wait[FLY];
 #pragma unroll
-        for (int k = 0; k < kRimInFlight; k++) {
+        for (int k = 0; k < FLY; k++) {
           e[k].x = 0xffffffffu;
           if (t0 + k < npoll) e[k] = polls[(w * npoll + t0 + k) * 32 + lane];
           wait[k] = e[k].x != 0xffffffffu;
@@ -463,10 +464,10 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_consta
         for (;;) {
           bool any = false;
 #pragma unroll
-          for (int k = 0; k < kRimInFlight; k++)
+          for (int k = 0; k < FLY; k++)
             if (wait[k]) rec[k].get(in + (size_t)e[k].x * RIM_BYTES);
 #pragma unroll
-          for (int k = 0; k < kRimInFlight; k++) {
+          for (int k = 0; k < FLY; k++) {
             if (wait[k]) wait[k] = !rec[k].ready(tag);
             any |= wait[k];
           }
@@ -482,7 +483,7 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_consta
           }
         }
 #pragma unroll
-        for (int k = 0; k < kRimInFlight; k++) {
+        for (int k = 0; k < FLY; k++) {
           if (e[k].x == 0xffffffffu) continue;
           const uint32_t off = (e[k].y & ~1u) + ((e[k].y & 1u) ? (uint32_t)(par ^ 1) * PAIR : 0u);
           *reinterpret_cast<U2*>(urows + off) = rec[k].value();

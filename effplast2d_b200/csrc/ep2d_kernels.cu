@@ -118,7 +118,7 @@ int occupancy_ty(bool record) {
   return e == cudaSuccess && n > 0 ? n : 1;
 }
 
-const void* chip_kernel(bool plastic, bool mixed, bool track, int warps);
+const void* chip_kernel(bool plastic, bool mixed, bool track, int warps, int rows);
 cudaError_t set_chip_attr(const void* kern) {
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CHIP_SMEM);
 }
@@ -126,9 +126,10 @@ cudaError_t set_chip_attr(const void* kern) {
 cudaError_t prepare_kernels_impl() {
   cudaError_t e;
   for (int warps : {8, 12, 16})
-    for (int mixed = 0; mixed < 2; mixed++)
-      for (int form = 0; form < 3; form++)  // elastic, plastic, plastic with tracking
-        if ((e = set_chip_attr(chip_kernel(form > 0, mixed, form == 2, warps))) != cudaSuccess) return e;
+    for (int rows : {2, 16})
+      for (int mixed = 0; mixed < 2; mixed++)
+        for (int form = 0; form < 3; form++)  // elastic, plastic, plastic with tracking
+          if ((e = set_chip_attr(chip_kernel(form > 0, mixed, form == 2, warps, rows))) != cudaSuccess) return e;
   for (const void* kern : {(const void*)k_iter_chip<0, 1, float, float>, (const void*)k_iter_chip<1, 1, float, float>,
                            (const void*)k_iter_chip<2, CHIP_JOBS, double, float>,
                            (const void*)k_iter_chip<2, CHIP_JOBS, double, double>})
@@ -318,20 +319,19 @@ int chip_ctas(int nx, int ny, int groups, int warps, int rows) {
 size_t chip_smem(int groups, int warps, int rows, bool track) { return chip_smem_bytes(groups, warps, rows, track); }
 
 namespace {
-template <typename TV, bool TRACK>
-const void* chip_kernel_of(bool plastic, int warps) {
-  if (TRACK || plastic)
-    return warps <= 8    ? (const void*)k_iter_chip<1, 1, double, TV, TRACK, 8>
-           : warps <= 12 ? (const void*)k_iter_chip<1, 1, double, TV, TRACK, 12>
-                         : (const void*)k_iter_chip<1, 1, double, TV, TRACK>;
-  return warps <= 8    ? (const void*)k_iter_chip<0, 1, double, TV, false, 8>
-         : warps <= 12 ? (const void*)k_iter_chip<0, 1, double, TV, false, 12>
-                       : (const void*)k_iter_chip<0, 1, double, TV>;
+template <int PLASTIC, typename TV, bool TRACK>
+const void* chip_kernel_of(int warps, int rows) {
+  if (warps <= 8) return (const void*)k_iter_chip<PLASTIC, 1, double, TV, TRACK, 8, 2>;
+  if (warps <= 12) return (const void*)k_iter_chip<PLASTIC, 1, double, TV, TRACK, 12, 2>;
+  if constexpr (PLASTIC == 1)
+    if (rows >= 10) return (const void*)k_iter_chip<PLASTIC, 1, double, TV, TRACK, 16, 3>;
+  return (const void*)k_iter_chip<PLASTIC, 1, double, TV, TRACK, 16, 2>;
 }
 // the FP64 (mixed: FP32 velocities) kernel of one RVE for a shape of `warps` warps per CTA
-const void* chip_kernel(bool plastic, bool mixed, bool track, int warps) {
-  if (track) return mixed ? chip_kernel_of<float, true>(true, warps) : chip_kernel_of<double, true>(true, warps);
-  return mixed ? chip_kernel_of<float, false>(plastic, warps) : chip_kernel_of<double, false>(plastic, warps);
+const void* chip_kernel(bool plastic, bool mixed, bool track, int warps, int rows) {
+  if (track) return mixed ? chip_kernel_of<1, float, true>(warps, rows) : chip_kernel_of<1, double, true>(warps, rows);
+  if (plastic) return mixed ? chip_kernel_of<1, float, false>(warps, rows) : chip_kernel_of<1, double, false>(warps, rows);
+  return mixed ? chip_kernel_of<0, float, false>(warps, rows) : chip_kernel_of<0, double, false>(warps, rows);
 }
 
 template <int JOBS>
@@ -370,7 +370,7 @@ cudaError_t launch_iter_chip(ChipJob* jobs, int njobs, bool mixed, const ChipSha
   if (njobs == 1) {
     const bool pl = jobs[0].plastic != 0;
     const void* kern = f32 ? (pl ? (const void*)k_iter_chip<1, 1, float, float> : (const void*)k_iter_chip<0, 1, float, float>)
-                           : chip_kernel(pl, mixed, track && pl, s.warps * s.groups);
+                           : chip_kernel(pl, mixed, track && pl, s.warps * s.groups, s.rows);
     return launch_chip_jobs<1>(jobs, 1, kern, s, n_iter, blocks, timeout_ns, stream, track && pl && !f32);
   }
   const void* kern = mixed ? (const void*)k_iter_chip<2, CHIP_JOBS, double, float> : (const void*)k_iter_chip<2, CHIP_JOBS, double, double>;
