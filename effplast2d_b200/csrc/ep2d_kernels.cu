@@ -345,8 +345,8 @@ cudaError_t launch_chip_jobs(const ChipJob* jobs, int njobs, const void* kern, c
   a.timeout_ns = timeout_ns;
   std::copy(jobs, jobs + njobs, a.job);
   void* args[] = {&a};
-  return cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(32 * s.warps * s.groups), args,
-                                     chip_smem_bytes(s.groups, s.warps, s.rows, track), stream);
+  const size_t sm = std::max(chip_smem_bytes(s.groups, s.warps, s.rows, track), (size_t)CHIP_SMEM_MIN);
+  return cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(32 * s.warps * s.groups), args, sm, stream);
 }
 }  // namespace
 

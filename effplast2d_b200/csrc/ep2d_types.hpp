@@ -117,6 +117,9 @@ struct ChipShape {
 constexpr int CHIP_SMS = 148;    // SMs of a B200
 constexpr int CHIP_WARPS = 16;   // warps per CTA: 128 registers per thread
 constexpr int CHIP_SMEM = 226 * 1024;
+// every CTA takes at least this much, of which no two fit an SM: a second CTA there would wait for the
+// first one's tensor memory, and the first for the second's rim
+constexpr int CHIP_SMEM_MIN = 116 * 1024;
 constexpr unsigned long long CHIP_TIMEOUT_NS = 10000000000ull;  // 10 s per wait
 constexpr int CHIP_MIN_RUN = 8;  // shorter runs of plain iterations are launched one by one
 ChipShape chip_shape(int nx, int ny);

@@ -151,3 +151,27 @@ def test_batch_waves_match_stream_batch(sides, precision):
             for m in ("kphi", "kd", "g"):
                 u, v = x[kind][m], y[kind][m]
                 assert u == v or (np.isnan(u) and np.isnan(v)), (kind, m, u, v)
+
+
+@pytest.mark.parametrize("kw,n", [(dict(kernel=ep.KERNEL_STREAM, rows=16), 1200)], ids=["stream"])
+def test_chip_form_beside_another_handle(kw, n):
+    # a small grid's CTAs (few warps, little shared memory) find their SMs while another thread's
+    # launches come and go, or another form's CTAs wait on one another; both results as alone
+    cases = [(64, {}, (500,) * 6), (n, kw, (300,) * 3)]
+    ins = [(m, m, _pa(m, m, n_pores=3, porosity=0.02, yield_stress=1e-5), 3, _random_state(m, m, 70), counts, ep.FP64, k)
+           for m, k, counts in cases]
+    want = [_run(*a, **k)[0] for *a, k in ins]
+    got = [None, None]
+
+    def work(k):
+        *a, opt = ins[k]
+        got[k] = _run(*a, **opt)[0]
+
+    ths = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in ths:
+        t.start()
+    for t in ths:
+        t.join()
+    for k in range(2):
+        for f in ("Ux", "Uy", "Vx", "Vy"):
+            assert np.array_equal(got[k][f], want[k][f]), (k, f)
