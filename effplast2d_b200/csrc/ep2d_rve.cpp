@@ -678,7 +678,7 @@ ChipJob Rve::chip_job(unsigned* flag) const {
 // n plain iterations in one launch of the on-chip form; *done = false where the device has no
 // room for its CTAs (the other forms take over for good).
 int Rve::run_chip(int64_t n, bool* done) {
-  if (!turn_.owns_lock()) turn_ = std::unique_lock<std::mutex>(chip_turn(device));
+  take_turn();
   *done = true;
   while (n > 0) {
     // chunks of an even length keep the parity; a chunk of one iteration cannot arise
@@ -702,6 +702,9 @@ int Rve::run_chip(int64_t n, bool* done) {
   return EP2D_OK;
 }
 
+void Rve::take_turn() {
+  if (!turn_.owns_lock()) turn_ = std::unique_lock<std::mutex>(chip_turn(device));
+}
 // the stream is idle: another handle may have the turn
 void Rve::end_turn() {
   if (turn_.owns_lock()) turn_.unlock();
@@ -722,6 +725,7 @@ int Rve::run_plain(int64_t n) {
   if (shape.form == FORM_RESIDENT && !f32 && !track) {
     // one cooperative launch for all n iterations (n == 1: an ordinary tile launch)
     if (n > 1) {
+      take_turn();
       EP2D_CK(launch_iter_resident(g, f, cur, prm.nl > 1, mixed(), shape.rows, n, RESIDENT_TIMEOUT_NS, stream));
       cur ^= (int)(n & 1);
       launches++;

@@ -63,8 +63,8 @@ IterShape shape_of(const ep2d_params& p, int sm_count = 0);
 // Device row pitch (elements) for an nx-wide grid.
 int row_pitch(int nx);
 
-// On-chip launches of different handles take turns on a device: their CTAs wait on one
-// another, so two such grids that each found room for only part of their CTAs would wait for
+// On-chip and resident-form launches of different handles take turns on a device: their CTAs wait on
+// one another, so two such grids that each found room for only part of their CTAs would wait for
 // each other until their waits ran out.  Held from the launch to its completion.
 std::mutex& chip_turn(int dev);
 
@@ -192,9 +192,10 @@ class Rve {
  private:
   int run_plain(int64_t n);
   int run_chip(int64_t n, bool* done);
-  // this handle's turn for on-chip launches (chip_turn): taken by run_chip, given back once the
+  // this handle's turn for launches whose CTAs wait on one another (chip_turn): given back once the
   // stream has been waited for -- by end_turn at the latest when iterate or solve_step returns
   std::unique_lock<std::mutex> turn_;
+  void take_turn();
   void end_turn();
   struct TurnScope {
     Rve& r;

@@ -153,7 +153,8 @@ def test_batch_waves_match_stream_batch(sides, precision):
                 assert u == v or (np.isnan(u) and np.isnan(v)), (kind, m, u, v)
 
 
-@pytest.mark.parametrize("kw,n", [(dict(kernel=ep.KERNEL_STREAM, rows=16), 1200)], ids=["stream"])
+@pytest.mark.parametrize("kw,n", [(dict(kernel=ep.KERNEL_STREAM, rows=16), 1200), (dict(kernel=ep.KERNEL_RESIDENT, rows=8), 160)],
+                         ids=["stream", "resident"])
 def test_chip_form_beside_another_handle(kw, n):
     # a small grid's CTAs (few warps, little shared memory) find their SMs while another thread's
     # launches come and go, or another form's CTAs wait on one another; both results as alone
