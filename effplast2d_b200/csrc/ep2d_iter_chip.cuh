@@ -14,8 +14,8 @@
 // The rim goes to the neighbouring CTAs through L2 as 16-byte records {lo, tag, hi, tag}
 // of a double, tag = the iteration: a reader polls the record itself until both tags are
 // the iteration's, so one L2 round trip both carries the value and synchronises, with no
-// fence, flag or grid-wide barrier (each 8-byte half {word, tag} is written by one
-// vector store and is valid on its own).  Records are double-buffered by iteration parity: a CTA
+// fence, flag or grid-wide barrier (each 64-bit {word, tag} is an element of one vector
+// store and valid on its own).  Records are double-buffered by iteration parity: a CTA
 // overwrites iteration t's records in iteration t + 2, after it has read its neighbours'
 // records of t + 1, which they wrote after reading all of t's.  Waits are bounded: a CTA that
 // waits longer than timeout_ns sets its RVE's error flag and leaves, the others
@@ -135,7 +135,9 @@ struct VPair<float> {
 
 // ---- rim records ------------------------------------------------------------------------
 // Record of a cell: {lo, tag, hi, tag} of Ux and of Uy, one 256-bit access; for float
-// displacements {Ux, tag, Uy, tag}, one 128-bit access.
+// displacements {Ux, tag, Uy, tag}, one 128-bit access.  The accesses' elements are the 64-bit
+// {word, tag}, so no element shows a tag without its word; they are taken apart inside the
+// statement (packed with shifts outside it 1024^2 took 3 % longer).
 template <typename T>
 struct RimRecord;
 template <>
@@ -147,15 +149,19 @@ struct RimRecord<double> {
     return make_double2(__hiloint2double((int)w[2], (int)w[0]), __hiloint2double((int)w[6], (int)w[4]));
   }
   __device__ void get(const char* rec) {
-    asm volatile("ld.relaxed.gpu.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+    asm volatile(
+        "{\n .reg .b64 a, b, c, d;\n ld.relaxed.gpu.global.v4.b64 {a,b,c,d}, [%8];\n mov.b64 {%0,%1}, a;\n"
+        " mov.b64 {%2,%3}, b;\n mov.b64 {%4,%5}, c;\n mov.b64 {%6,%7}, d;\n}"
                  : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
                  : "l"(rec)
                  : "memory");
   }
   static __device__ void put(char* rec, const double2& u, uint32_t tag) {
-    asm volatile("st.relaxed.gpu.global.v8.b32 [%0], {%1,%5,%2,%5,%3,%5,%4,%5};" ::"l"(rec), "r"(__double2loint(u.x)),
-                 "r"(__double2hiint(u.x)), "r"(__double2loint(u.y)), "r"(__double2hiint(u.y)), "r"(tag)
-                 : "memory");
+    asm volatile(
+        "{\n .reg .b64 a, b, c, d;\n mov.b64 a, {%1,%5};\n mov.b64 b, {%2,%5};\n mov.b64 c, {%3,%5};\n"
+        " mov.b64 d, {%4,%5};\n st.relaxed.gpu.global.v4.b64 [%0], {a,b,c,d};\n}" ::"l"(rec),
+        "r"(__double2loint(u.x)), "r"(__double2hiint(u.x)), "r"(__double2loint(u.y)), "r"(__double2hiint(u.y)), "r"(tag)
+        : "memory");
   }
 };
 template <>
@@ -165,15 +171,18 @@ struct RimRecord<float> {
   __device__ bool ready(uint32_t tag) const { return ((w[1] ^ tag) | (w[3] ^ tag)) == 0; }
   __device__ float2 value() const { return make_float2(__uint_as_float(w[0]), __uint_as_float(w[2])); }
   __device__ void get(const char* rec) {
-    asm volatile("ld.relaxed.gpu.global.v4.b32 {%0,%1,%2,%3}, [%4];"
+    asm volatile(
+        "{\n .reg .b64 a, b;\n ld.relaxed.gpu.global.v2.b64 {a,b}, [%4];\n mov.b64 {%0,%1}, a;\n mov.b64 {%2,%3}, b;\n}"
                  : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
                  : "l"(rec)
                  : "memory");
   }
   static __device__ void put(char* rec, const float2& u, uint32_t tag) {
-    asm volatile("st.relaxed.gpu.global.v4.b32 [%0], {%1,%3,%2,%3};" ::"l"(rec), "r"(__float_as_uint(u.x)),
-                 "r"(__float_as_uint(u.y)), "r"(tag)
-                 : "memory");
+    asm volatile(
+        "{\n .reg .b64 a, b;\n mov.b64 a, {%1,%3};\n mov.b64 b, {%2,%3};\n st.relaxed.gpu.global.v2.b64 [%0], {a,b};\n}" ::
+            "l"(rec),
+        "r"(__float_as_uint(u.x)), "r"(__float_as_uint(u.y)), "r"(tag)
+        : "memory");
   }
 };
 // where a warp's row pairs lie: pair q of its rows/2, copy `par` of the double-buffered ones
