@@ -468,6 +468,10 @@ __global__ void __launch_bounds__(32 * STREAM_WARPS) k_iter_stream_batch(const B
 // cycles) together with HBM.
 constexpr int PAIR_DEPTH = 2;
 constexpr int PAIR_SLOTS = PAIR_DEPTH + 2;
+// U's two buffers and V from which marches alternate in direction.  Below it L2 holds them and the march
+// down's addresses only cost (us: 1200^2, 68 MiB, 18.1 up, 18.25 in turn; FP32 2048^2, 99 MiB, 32.5, 33.3);
+// 1536^2, 110.3 MiB, is even.
+constexpr size_t PAIR_TURN_BYTES = (size_t)110 << 20;
 
 template <typename TU, typename TV>
 struct __align__(16) StreamPair {
@@ -482,7 +486,7 @@ constexpr size_t stream_pair_smem_bytes() {
   return N_MATS * sizeof(MatT<TU>) + sizeof(StreamPair<TU, TV>) * PAIR_SLOTS * STREAM_WARPS;
 }
 
-template <typename TU, typename TV, bool EDGE>
+template <typename TU, typename TV, bool EDGE, bool DOWN>
 struct StreamIo {
   using U2 = Vec2<TU>;
   static constexpr bool TRACK = false;
@@ -507,18 +511,18 @@ struct StreamIo {
     const int row = jA - 2 + 2 * k + r, col = STREAM_COLS * strip - 2 + 2 * c;
     const bool in = !EDGE || (col >= 0 && col < pitch && row >= 0);
     const bool okx = in && (!EDGE || row < ny), oky = in && (!EDGE || row <= ny);
-    const int q = row * pitch + col;
+    const int qx = (DOWN ? ny - 1 - row : row) * pitch + col, qy = DOWN ? qx + pitch : qx;
     auto at = [](auto* b, uint32_t k) {
       return reinterpret_cast<decltype(b)>(reinterpret_cast<const char*>(b) + (uint32_t)(k * (uint32_t)sizeof(*b)));
     };
-    cp_async_pair_zfill<TU>(&d.ux[r][2 * c], at(ux, okx ? q : 0), okx);
-    cp_async_pair_zfill<TU>(&d.uy[r][2 * c], at(uy, oky ? q : 0), oky);
-    cp_async_pair_zfill<TV>(&d.vx[r][2 * c], at((const TV*)vx, okx ? q : 0), okx);
-    cp_async_pair_zfill<TV>(&d.vy[r][2 * c], at((const TV*)vy, oky ? q : 0), oky);
+    cp_async_pair_zfill<TU>(&d.ux[r][2 * c], at(ux, okx ? qx : 0), okx);
+    cp_async_pair_zfill<TU>(&d.uy[r][2 * c], at(uy, oky ? qy : 0), oky);
+    cp_async_pair_zfill<TV>(&d.vx[r][2 * c], at((const TV*)vx, okx ? qx : 0), okx);
+    cp_async_pair_zfill<TV>(&d.vy[r][2 * c], at((const TV*)vy, oky ? qy : 0), oky);
     if (c < 9) {
       const int mc = STREAM_COLS * strip - 4 + 4 * c;
       const bool okm = !EDGE || (mc >= 0 && mc < pitch && row >= 0 && row < ny);
-      cp_async_zfill<4>(&d.m[r][c], mask + (okm ? row * pitch + mc : 0), okm);
+      cp_async_zfill<4>(&d.m[r][c], mask + (okm ? (DOWN ? ny - 1 - row : row) * pitch + mc : 0), okm);
     }
   }
   __device__ __forceinline__ int mask_byte(const StreamPair<TU, TV>& d, int r, int row) const {
@@ -527,7 +531,7 @@ struct StreamIo {
     if (!EDGE) return m;
     // a node outside the grid counts as a pore node, a corner outside it as a pore corner
     const bool node = i >= 0 && i < nx && row >= 0 && row < ny;
-    const bool corner = i >= 0 && i < nx - 1 && row >= 0 && row < ny - 1;
+    const bool corner = i >= 0 && i < nx - 1 && (DOWN ? row >= 1 && row < ny : row >= 0 && row < ny - 1);
     return node ? (corner ? m : (m | M_CORNER)) : (int)(M_NODE | M_CORNER);
   }
   template <int STAGE>
@@ -561,7 +565,8 @@ struct StreamIo {
   }
   __device__ __forceinline__ const MatT<TU>& mat(int, int r) const {
     const int m = r ? mk_a : mk_c, up = r ? mk_b : mk_a;
-    return mats[(m & (M_MAT | M_NODE)) | (corner_index(m, up) << 2)];
+    // (the corner's lower row of nodes is the next one of the march down)
+    return mats[(m & (M_MAT | M_NODE)) | ((DOWN ? corner_index(up, m) : corner_index(m, up)) << 2)];
   }
   __device__ __forceinline__ void old(int, U2& u0, U2& u1, TV (&v)[4]) const {
     const StreamPair<TU, TV>& d = ring[slot ? slot - 1 : PAIR_SLOTS - 1];
@@ -575,29 +580,37 @@ struct StreamIo {
   }
   __device__ __forceinline__ void store(int p, const U2& u0, const U2& u1, const TV (&v)[4]) const {
     const int j = jA + 2 * p - 4;
-    const uint32_t q = (uint32_t)(j * pitch + i), q1 = q + pitch;
+    // rows of Ux and Vx, of Uy and Vy
+    const uint32_t x0 = (uint32_t)((DOWN ? ny - 1 - j : j) * pitch + i), x1 = DOWN ? x0 - pitch : x0 + pitch;
+    const uint32_t y0 = DOWN ? x0 + pitch : x0, y1 = DOWN ? x0 : x1;
     auto at = [](auto* b, uint32_t k) -> auto& {
       return *reinterpret_cast<decltype(b)>(reinterpret_cast<char*>(b) + (uint32_t)(k * (uint32_t)sizeof(*b)));
     };
     if (own) {
-      at(vx, q) = v[0];
-      at(vy, q) = v[1];
-      at(uxo, q) = u0.x;
-      at(uyo, q) = u0.y;
+      at(vx, x0) = v[0];
+      at(uxo, x0) = u0.x;
+      if (!EDGE || !DOWN || j > 0) {  // row ny of Uy never changes
+        at(vy, y0) = v[1];
+        at(uyo, y0) = u0.y;
+      }
     }
     if (own && j + 1 < jB) {
-      at(vx, q1) = v[2];
-      at(vy, q1) = v[3];
-      at(uxo, q1) = u1.x;
-      at(uyo, q1) = u1.y;
+      at(vx, x1) = v[2];
+      at(vy, y1) = v[3];
+      at(uxo, x1) = u1.x;
+      at(uyo, y1) = u1.y;
     }
   }
   __device__ __forceinline__ void yields(int, bool, bool, bool, bool) const {}
 };
 
 // One plain iteration of one RVE: warp w of CTA b handles task b * STREAM_WARPS + w =
-// (strip, segment), as k_iter_stream does.
-template <bool PLASTIC, typename TU, typename TV>
+// (strip, segment), as k_iter_stream does.  DOWN: segments and rows counted from the top, the
+// march down.  Launches on a state above PAIR_TURN_BYTES alternate (by the buffer that holds U), so that an
+// iteration begins with the rows the one before it ended with, which L2 still holds.  us per iteration,
+// one direction / in turn: 2048^2 NL=3 54.6 / 53.6, elastic 50.0 / 46.3, mixed 52.2 / 50.6; 2600^2 90.3 /
+// 88.3; 1600^2 elastic 28.7 / 27.3; 4096^2 (several waves) 212.4 / 211.5; FP32 2600^2 54.2 / 51.6.
+template <bool PLASTIC, typename TU, typename TV, bool DOWN>
 __global__ void __launch_bounds__(32 * STREAM_WARPS, 4) k_iter_pairs(const __grid_constant__ Geo g,
                                                                      const __grid_constant__ Fields f, int src,
                                                                      int nstrips, int nsegs, int seg_h) {
@@ -616,7 +629,7 @@ __global__ void __launch_bounds__(32 * STREAM_WARPS, 4) k_iter_pairs(const __gri
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   auto run = [&](auto edge_c) {
     constexpr bool EDGE = decltype(edge_c)::value;
-    StreamIo<TU, TV, EDGE> io;
+    StreamIo<TU, TV, EDGE, DOWN> io;
     io.mats = mats;
     io.ring = ring;
     io.ux = u_field<TU>(f, false, src);
@@ -642,7 +655,9 @@ __global__ void __launch_bounds__(32 * STREAM_WARPS, 4) k_iter_pairs(const __gri
     }
     // FP32 has the registers for two steps per turn (2048^2 40.4 -> 34.5 us); FP64 gains nothing
     constexpr int UNROLL = sizeof(TU) == 4 ? 2 : 1;
-    pair_march<TU, TV, PLASTIC, EDGE, 0, false, UNROLL>(g, io, io.npairs, i, jA);
+    pair_march<TU, TV, PLASTIC, EDGE, 0, false, UNROLL, DOWN>(g, io, io.npairs, i, jA);
+    // row 0 of Uy, row ny of the march down, moves with the velocity it has
+    if (EDGE && DOWN && jB == g.ny && io.own) io.uyo[i] = advance(io.uy[i], (TU)io.vy[i], (TU)g.dT);
   };
   if (stream_interior(g.nx, g.ny, strip, jA, jB + 1)) run(std::false_type{});
   else run(std::true_type{});

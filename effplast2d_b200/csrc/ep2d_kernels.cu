@@ -173,8 +173,13 @@ cudaError_t launch_stream_tv(const Geo& g, const Fields& f, int src, bool plasti
   // plain launches take the pair march; its offsets are 32-bit bytes
   if (!record && !(track && plastic) && (uint64_t)g.pitch * (g.ny + 1) * sizeof(TU) < ((uint64_t)1 << 32)) {
     const size_t sp = stream_pair_smem_bytes<TU, TV>();
-    if (plastic) return launch_overlapped(k_iter_pairs<true, TU, TV>, blocks, threads, sp, stream, g, f, src, nstrips, nsegs, seg_h);
-    return launch_overlapped(k_iter_pairs<false, TU, TV>, blocks, threads, sp, stream, g, f, src, nstrips, nsegs, seg_h);
+    auto go = [&](auto kern) {
+      return launch_overlapped(kern, blocks, threads, sp, stream, g, f, src, nstrips, nsegs, seg_h);
+    };
+    // marches up and down in turn where U's two buffers and V exceed what L2 keeps of them (k_iter_pairs)
+    const size_t state = (size_t)g.pitch * (g.ny + 1) * (4 * sizeof(TU) + 2 * sizeof(TV));
+    if ((src & 1) && state > PAIR_TURN_BYTES) return plastic ? go(k_iter_pairs<true, TU, TV, true>) : go(k_iter_pairs<false, TU, TV, true>);
+    return plastic ? go(k_iter_pairs<true, TU, TV, false>) : go(k_iter_pairs<false, TU, TV, false>);
   }
   if constexpr (std::is_same<TU, double>::value) {
     if (track && plastic) {

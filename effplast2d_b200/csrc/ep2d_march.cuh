@@ -98,9 +98,13 @@ __device__ __forceinline__ float rsqrt_of(float x) { return rsqrtf(x); }
 //   old(p, u0, u1, v)               U and V = {vx, vy of the lower row, of the upper} of own pair p - 2
 //   store(p, u0, u1, v)             their new values
 //   yields(p, n0, n1, c0, c1)       TRACK: own pair p - 2's nodes and corners that yield
+// DOWN: the rows are counted from the top: row j here is row ny - 1 - j of the nodes, Ux and Vx, row
+// ny - j of Uy and Vy, corner row ny - 2 - j.  Differences along y then have their operands in the
+// other order, and every value is formed from the same operands as in the march up.
 // T: arithmetic and displacement type, TV: velocity storage.  T = float: the FP32 bulk's
 // perturbations about the affine field.
-template <typename T, typename TV, bool PLASTIC, bool EDGE, int NP, bool TRACK, int UNROLL, typename Io>
+template <typename T, typename TV, bool PLASTIC, bool EDGE, int NP, bool TRACK, int UNROLL, bool DOWN = false,
+          typename Io>
 __device__ __forceinline__ void pair_march(const Geo& g, Io& io, int npairs_in, int i, int jA) {
   using U2 = Vec2<T>;
   const int npairs = NP ? NP : npairs_in;
@@ -122,13 +126,14 @@ __device__ __forceinline__ void pair_march(const Geo& g, Io& io, int npairs_in, 
   T hz = 0, h0 = 0, h1 = 0;         // corner pair sums of the last three rows
   T syq = 0, cq = 0, cq_l = 0;      // returned: total syy, corner of the row below
 
+  auto diff_y = [](T upper, T lower) { return DOWN ? sub_rn(lower, upper) : sub_rn(upper, lower); };
   auto trial = [&](const MatT<T>& m, T ux, T ux_r, T uy, T ux1_r, T uy1, T uy1_r, T& p, T& x, T& y, T& c) {
     if constexpr (std::is_same<T, float>::value) {
-      node_trial(sub_rn(ux_r, ux), sub_rn(uy1, uy), exx0, eyy0, m.k, m.g2, rdX, rdY, third, p, x, y);
-      c = corner_trial(m.g4, sub_rn(ux1_r, ux_r), sub_rn(uy1_r, uy1), exy0, rdX, rdY);
+      node_trial(sub_rn(ux_r, ux), diff_y(uy1, uy), exx0, eyy0, m.k, m.g2, rdX, rdY, third, p, x, y);
+      c = corner_trial(m.g4, diff_y(ux1_r, ux_r), sub_rn(uy1_r, uy1), exy0, rdX, rdY);
     } else {
-      node_trial(sub_rn(ux_r, ux), sub_rn(uy1, uy), m.k, m.g2, rdX, rdY, third, p, x, y);
-      c = corner_trial(m.g4, sub_rn(ux1_r, ux_r), sub_rn(uy1_r, uy1), rdX, rdY);
+      node_trial(sub_rn(ux_r, ux), diff_y(uy1, uy), m.k, m.g2, rdX, rdY, third, p, x, y);
+      c = corner_trial(m.g4, diff_y(ux1_r, ux_r), sub_rn(uy1_r, uy1), rdX, rdY);
     }
   };
   auto corner_pair = [&](T c) {
@@ -153,8 +158,8 @@ __device__ __forceinline__ void pair_march(const Geo& g, Io& io, int npairs_in, 
   // faces of row j: new velocities and displacements from the old ones
   auto face = [&](int j, T sx, T sx_l, T sy, T cw_l, TV& vx, TV& vy, U2& u) {
     const T vxo = (T)vx, vyo = (T)vy;
-    const TV vxs = (TV)face_velocity_s(vxo, cX, sub_rn(sx, sx_l), dtrX, sub_rn(cw_l, cq_l), dtrY);
-    const TV vys = (TV)face_velocity_s(vyo, cY, sub_rn(sy, syq), dtrY, sub_rn(cq, cq_l), dtrX);
+    const TV vxs = (TV)face_velocity_s(vxo, cX, sub_rn(sx, sx_l), dtrX, diff_y(cw_l, cq_l), dtrY);
+    const TV vys = (TV)face_velocity_s(vyo, cY, diff_y(sy, syq), dtrY, sub_rn(cq, cq_l), dtrX);
     if (EDGE) {  // a face the reference leaves alone keeps its velocity
       if (i > 0 && j > 0 && j < ny - 1) vx = vxs;
       if (i > 0 && i < nx - 1 && j > 0) vy = vys;
