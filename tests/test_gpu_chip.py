@@ -90,6 +90,42 @@ def test_stream_pairs_match_tile_form(rows, nl, precision):
         assert np.array_equal(b[f], a[f]), (f, float(np.max(np.abs(b[f] - a[f]))))
 
 
+# states above PAIR_TURN_BYTES, whose marches go up and down in turn: the library's segments and odd
+# and even ones, tall and wide grids of a ragged last strip and segment
+@pytest.mark.parametrize("nx,ny,rows", [(1801, 1699, 0), (203, 15001, 37), (15001, 201, 6)])
+@pytest.mark.parametrize("nl,precision", [(1, ep.FP64), (3, ep.FP64), (2, ep.MIXED)], ids=["elastic", "plastic", "mixed"])
+def test_marches_in_turn_match_tile_form(nx, ny, rows, nl, precision):
+    pa = _pa(nx, ny, n_pores=3, porosity=0.03, yield_stress=1e-5)
+    st = _random_state(nx, ny, 47)
+    rng = np.random.default_rng(48)
+    st["Vy"][0] = 1e-7 * rng.standard_normal(nx)  # row 0 of Uy moves with its velocity, row ny never does
+    st["Vy"][-1] = 1e-7 * rng.standard_normal(nx)
+    form = dict(kernel=ep.KERNEL_STREAM, rows=rows) if rows else {}
+    a, _ = _run(nx, ny, pa, nl, st, (8, 3), precision, kernel=ep.KERNEL_TILE, rows=16)
+    b, _ = _run(nx, ny, pa, nl, st, (8, 3), precision, **form)
+    for f in a:
+        assert np.array_equal(b[f], a[f]), (f, float(np.max(np.abs(b[f] - a[f]))))
+
+
+def test_marches_in_turn_f32():
+    # FP32: the same iterations from either buffer, so each is once a march up and once a march down
+    nx, ny = 2400, 2003
+    pa = _pa(nx, ny, n_pores=3, porosity=0.03, yield_stress=1e-5)
+    st = _random_state(nx, ny, 49)
+    out = []
+    for first in (0, 1):
+        s = ep.Solver(nx, ny, pa, nl=2, precision=ep.F32_BULK)
+        s.iterate_f32(first)
+        for k, v in st.items():
+            s.set(k, v)
+        s.iterate_f32(5)
+        out.append({f: s.get(f) for f in ("Ux", "Uy", "Vx", "Vy")})
+        s.close()
+    for f in out[0]:
+        assert np.array_equal(out[0][f], out[1][f]), f
+        assert not np.array_equal(out[0][f], st[f])
+
+
 @pytest.mark.parametrize("nx,ny", [(8, 9), (57, 130), (403, 401), (1061, 1060)])
 @pytest.mark.parametrize("nl", [1, 2])
 def test_chip_f32_matches_stream_f32(nx, ny, nl):
