@@ -301,9 +301,9 @@ ChipShape chip_shape(int nx, int ny) {
   return best;
 }
 
-size_t chip_rim_bytes(int nx, int ny, int warps, int rows) {
+size_t chip_rim_bytes(int nx, int ny, int warps, int rows, bool f32) {
   const size_t ncx = (nx + STREAM_COLS - 1) / STREAM_COLS, ncy = (ny + warps * rows - 1) / (warps * rows);
-  return 2 * RimRecord<double>::BYTES * ncx * ncy * (4 * (size_t)warps * rows + 4 * STREAM_COLS);
+  return 2 * (f32 ? RimRecord<float>::BYTES : RimRecord<double>::BYTES) * ncx * ncy * (4 * (size_t)warps * rows + 4 * STREAM_COLS);
 }
 
 // 4 records per row of padded height and 4 x STREAM_COLS per tile: the shortest tiles of at
@@ -368,7 +368,7 @@ cudaError_t launch_iter_chip(ChipJob* jobs, int njobs, bool mixed, const ChipSha
     j.ncx = (j.g.nx + STREAM_COLS - 1) / STREAM_COLS;
     j.ncy = (j.g.ny + s.warps * s.rows - 1) / (s.warps * s.rows);
     j.cta0 = blocks;
-    const cudaError_t e = cudaMemsetAsync(j.rim, 0, chip_rim_bytes(j.g.nx, j.g.ny, s.warps, s.rows), stream);
+    const cudaError_t e = cudaMemsetAsync(j.rim, 0, chip_rim_bytes(j.g.nx, j.g.ny, s.warps, s.rows, f32), stream);
     if (e != cudaSuccess) return e;
     blocks += (j.ncx * j.ncy + s.groups - 1) / s.groups;
   }

@@ -340,11 +340,9 @@ size_t n_samples(const ep2d_params& p) {
 // the on-chip form is taken only where the parameters leave the kernel to the library
 bool chip_allowed(const ep2d_params& p) { return p.kernel == EP2D_KERNEL_AUTO && p.rows == 0; }
 // the stress arrays are contiguous, and those a recording launch writes (p to txy; with the
-// return map also txyav, j2, j2xy) hold the rim records of a run if they can; an FP32 run need
-// not be followed by a launch that writes them
+// return map also txyav, j2, j2xy) hold the rim records of a run if they can
 size_t own_rim_bytes(const ep2d_params& p) {
   const size_t need = chip_allowed(p) ? chip_rim_capacity(p.nx, p.ny) : 0;
-  if (p.precision == EP2D_F32_BULK) return align256(need);
   return need > (p.nl > 1 ? 7 : 4) * align256(field_elems(p) * sizeof(double)) ? align256(need) : 0;
 }
 
@@ -668,7 +666,7 @@ ChipJob Rve::chip_job(unsigned* flag) const {
   ChipJob j{};
   j.g = g;
   j.f = f;
-  j.rim = d_rim;
+  j.rim = f32 ? reinterpret_cast<char*>(f.ux[0]) : d_rim;
   j.flag = flag;
   j.src = cur;
   j.plastic = prm.nl > 1 ? 1 : 0;
@@ -698,6 +696,8 @@ int Rve::run_chip(int64_t n, bool* done) {
     resident_launches++;
     n -= chunk;
   }
+  // the padding beside the displacements is read as zeros
+  if (f32) EP2D_CK(cudaMemsetAsync(f.ux[0], 0, chip_rim_bytes(prm.nx, prm.ny, chip.warps, chip.rows, true), stream));
   vmax_zero_ = true;
   return EP2D_OK;
 }
@@ -715,9 +715,16 @@ Rve::TurnScope::~TurnScope() {
   r.turn_.unlock();
 }
 
+// The FP32 phase keeps its rim records in the FP64 displacements (four contiguous arrays), which are
+// written anew when it ends; grids of a few tiles with hardly a column or row in the last one need more
+bool Rve::chip_f32_fits() const {
+  return chip_rim_bytes(prm.nx, prm.ny, chip.warps, chip.rows, true) <=
+         4 * align256(field_elems(prm) * sizeof(double));
+}
+
 int Rve::run_plain(int64_t n) {
   if (chip.warps && n >= CHIP_MIN_RUN &&
-      (!track || f32 || chip_smem(chip.groups, chip.warps, chip.rows, true) <= CHIP_SMEM)) {
+      (f32 ? chip_f32_fits() : !track || chip_smem(chip.groups, chip.warps, chip.rows, true) <= CHIP_SMEM)) {
     bool done = false;
     const int rc = run_chip(n, &done);
     if (rc || done) return rc;

@@ -136,6 +136,7 @@ class Rve {
   ChipShape chip{};
   // its rim records: in the stress arrays, which only recording launches write and every run of
   // plain iterations is followed by one; in memory of their own where a small grid's are too small
+  // (the FP32 phase: chip_f32_fits)
   char* d_rim = nullptr;
   // velocities stored in FP32 (the mixed path, and both phases of the FP32 bulk)
   bool mixed() const { return prm.precision == EP2D_MIXED || prm.precision == EP2D_F32_BULK; }
@@ -192,6 +193,7 @@ class Rve {
  private:
   int run_plain(int64_t n);
   int run_chip(int64_t n, bool* done);
+  bool chip_f32_fits() const;
   // this handle's turn for launches whose CTAs wait on one another (chip_turn): given back once the
   // stream has been waited for -- by end_turn at the latest when iterate or solve_step returns
   std::unique_lock<std::mutex> turn_;

@@ -142,7 +142,7 @@ struct ChipArgs {
 };
 // bytes of a grid's rim records at a given warps x rows, and the most any shape may need
 // that a launch takes for it (0 for a grid that does not fit on chip)
-size_t chip_rim_bytes(int nx, int ny, int warps, int rows);
+size_t chip_rim_bytes(int nx, int ny, int warps, int rows, bool f32 = false);
 size_t chip_rim_capacity(int nx, int ny);
 // tiles and CTAs of a grid at a given warps x rows x groups
 int chip_ctas(int nx, int ny, int groups, int warps, int rows);
