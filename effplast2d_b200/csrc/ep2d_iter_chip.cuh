@@ -29,8 +29,8 @@
 // What bounds it: on grids up to ~400^2 latency, the rim exchange (1.4 us of an iteration
 // with the march left out) and one warp's march; on larger ones the issue of the march's
 // instructions.  Measured, us per iteration, the form the library took before / this one
-// (FP64): elastic 128^2 4.2 / 1.74, 512^2 6.3 / 2.53, 1024^2 15.5 / 5.7; with the return map
-// 128^2 5.8 / 2.41, 256^2 6.2 / 2.70, 512^2 8.9 / 4.27, 768^2 14.3 / 6.85, 1024^2 16.3 / 9.9.
+// (FP64): elastic 128^2 4.2 / 1.51, 1024^2 15.5 / 5.9; with the return map 128^2 5.8 / 2.05, 256^2
+// 6.2 / 2.50, 512^2 8.9 / 3.75, 768^2 14.3 / 6.83, 1024^2 16.3 / 9.96.
 #pragma once
 
 #include "ep2d_iter_f64.cuh"
@@ -198,9 +198,14 @@ __device__ __forceinline__ uint32_t chip_pair_off(int q, int npairs, int par) {
 // par ^ 1), V in tensor memory.  NP: the number of row pairs where it is known (1 to 3: the march
 // unrolled, so that its rows' chains overlap: 256^2, 2 rows, 2.70 -> 2.54 us an iteration; 448^2,
 // 4 rows, 3.76 -> 3.55; 512^2, 6 rows, 4.29 -> 4.07), else 0.
-template <typename T, typename TV, bool EDGE, int NP>
+// SEL: SELECT of the march.  The warps at the grid's edges set the pace of all, and with it their rows take
+// fewer sums (us per iteration: 128^2 2.13 -> 2.04, 256^2 2.54 -> 2.48, 512^2 3.91 -> 3.73, 601^2 4.49 ->
+// 4.36, FP32 768^2 4.60 -> 4.35).  The FP64 kernels with three records in flight have no register to
+// spare for it (768^2 6.81 -> 7.13, 1024^2 9.98 -> 10.59).
+template <typename T, typename TV, bool EDGE, int NP, bool SEL>
 struct ChipIo {
   using U2 = Vec2<T>;
+  static constexpr bool SELECT = SEL;
   static constexpr int VW = sizeof(VPair<TV>) / 4;
   const MatT<T>* mats;
   const uint8_t* idx;       // material indices of row jA - 2 on, 32 per row, this lane's column
@@ -411,7 +416,7 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_consta
             constexpr int NP = decltype(np_c)::value;
             auto run = [&](auto edge_c) {
               constexpr bool EDGE = decltype(edge_c)::value;
-              ChipIo<T, TV, EDGE, NP> io;
+              ChipIo<T, TV, EDGE, NP, FLY == 2 || sizeof(T) == 4> io;
               io.mats = mats;
               io.idx = idx + w * rows * 32 + lane;
               io.below = below;

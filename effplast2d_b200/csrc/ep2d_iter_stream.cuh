@@ -461,9 +461,9 @@ __global__ void __launch_bounds__(32 * STREAM_WARPS) k_iter_stream_batch(const B
 // Offsets into a field are 32-bit bytes from its base (fields of 4 GB and more stay with
 // k_iter_stream): a store or copy then needs no 64-bit address arithmetic (53.3 -> 52.5).
 //
-// us per iteration with the return map, k_iter_stream before / this: 2048^2 60.5 / 52.5 (5.1 TB/s of the
-// 64 B per cell, 0.78 of the measured HBM rate), 1536^2 44.5 / 30.6 and 1200^2 25.6 / 19.8 (with
-// segments that fill one wave, shape_of), 2048^2 elastic 61.7 / 49.5, FP32 bulk 41.7 / 34.5.  What bounds it
+// us per iteration with the return map, k_iter_stream before / this: 2048^2 60.5 / 52.4 (5.1 TB/s of the
+// 64 B per cell, 0.78 of the measured HBM rate), 1536^2 44.5 / 29.5 and 1200^2 25.6 / 17.7 (with
+// segments that fill one wave, shape_of), 2048^2 elastic 61.7 / 45.4, FP32 bulk 41.7 / 31.0.  What bounds it
 // at 2048^2: issue (205 warp instructions per strip row where all yields, 64 % of
 // cycles) together with HBM.
 constexpr int PAIR_DEPTH = 2;
@@ -489,7 +489,7 @@ constexpr size_t stream_pair_smem_bytes() {
 template <typename TU, typename TV, bool EDGE, bool DOWN>
 struct StreamIo {
   using U2 = Vec2<TU>;
-  static constexpr bool TRACK = false;
+  static constexpr bool SELECT = true;  // 2048^2 53.4 -> 52.4 us an iteration, FP32 32.4 -> 31.0, 1200^2 18.1 -> 17.7
   const MatT<TU>* mats;
   StreamPair<TU, TV>* ring;
   const TU *ux, *uy;

@@ -92,6 +92,7 @@ __device__ __forceinline__ double rsqrt_of(double x) { return rsqrt(x); }
 __device__ __forceinline__ float rsqrt_of(float x) { return rsqrtf(x); }
 
 // Io, the rows' source and destination:
+//   SELECT                          how the node sums at the grid's lowest and highest rows are formed
 //   begin<STAGE>(p)                 before step p's rows are read
 //   rows(p, ua, uar, ub, ubr)       (Ux, Uy) of rows ka and ka + 1, this column's and the next one's
 //   mat(p, r)                       materials of row ka - 1 (r = 0) or ka (r = 1)
@@ -139,10 +140,15 @@ __device__ __forceinline__ void pair_march(const Geo& g, Io& io, int npairs_in, 
   auto corner_pair = [&](T c) {
     return EDGE ? add_rn(shfl_idx(c, sa), shfl_idx(c, sb)) : add_rn(shfl_up1(c), c);
   };
-  // 4-corner sum of node row j from the pair sums of corner rows j - 2 .. j + 1
-  auto corner_sum = [&](int j, T hm2, T hm1, T hj, T hp1) {
-    if (EDGE) return j == 0 ? add_rn(hj, hp1) : j == ny - 1 ? add_rn(hm2, hm1) : add_rn(hm1, hj);
-    return add_rn(hm1, hj);
+  // The 4-corner sum of node row j adds the pair sums of corner rows j - 1 and j; of row 0 those of
+  // rows 0 and 1, of row ny - 1 those of rows ny - 3 and ny - 2 (EDGE).  So pair row ny - 1 takes row
+  // ny - 3's place, and row -1 that of row 1: one select on a pair sum instead of three sums to select
+  // from (Io::SELECT).
+  constexpr bool SELECT = Io::SELECT;
+  auto pair_above = [&](int row, T h, T h2) { return SELECT && EDGE && row == ny - 1 ? h2 : h; };
+  auto corner_sum = [&](int j, bool first, T hm2, T hm1, T hj, T hp1) {  // pair sums of rows j - 2 .. j + 1
+    if (EDGE && !SELECT) return j == 0 ? add_rn(hj, hp1) : j == ny - 1 ? add_rn(hm2, hm1) : add_rn(hm1, hj);
+    return add_rn(EDGE && first && j == 0 ? hp1 : hm1, hj);
   };
   // 16 J2^2 of a corner of row j from the node deviators of rows j and j + 1
   auto corner_j2 = [&](T x, T y, T c, T xn, T yn) {
@@ -179,16 +185,16 @@ __device__ __forceinline__ void pair_march(const Geo& g, Io& io, int npairs_in, 
     T p1 = 0, x1 = 0, y1 = 0, c1 = 0, p2, x2, y2, c2, hs1 = 0, hs2 = 0;
     if constexpr (STAGE >= 1) {
       trial(io.mat(p, 0), uxc, uxc_r, uyc, uar.x, ua.y, uar.y, p1, x1, y1, c1);
-      if (PLASTIC) hs1 = corner_pair(c1);
+      if (PLASTIC) hs1 = pair_above(jA + 2 * p - 3, corner_pair(c1), h0);
     }
     trial(io.mat(p, 1), ua.x, uar.x, ua.y, ubr.x, ub.y, ubr.y, p2, x2, y2, c2);
-    if (PLASTIC) hs2 = corner_pair(c2);
+    if (PLASTIC) hs2 = pair_above(jA + 2 * p - 2, corner_pair(c2), h1);
     const int ja = jA + 2 * p - 4;  // row ka - 2
     if constexpr (STAGE == 2) {
       T xr0 = xb, yr0 = yb, cw0 = cb, xr1 = x1, yr1 = y1, cw1 = c1;
       if (PLASTIC) {
-        const T n0 = node_j2sq_h(xb, yb, corner_sum(ja, hz, h0, h1, hs1));
-        const T n1 = node_j2sq_h(x1, y1, corner_sum(ja + 1, h0, h1, hs1, hs2));
+        const T n0 = node_j2sq_h(xb, yb, corner_sum(ja, true, hz, h0, h1, hs1));
+        const T n1 = node_j2sq_h(x1, y1, corner_sum(ja + 1, false, h0, h1, hs1, hs2));
         const T m0 = corner_j2(xb, yb, cb, x1, y1), m1 = corner_j2(x1, y1, c1, x2, y2);
         if (__any_sync(0xffffffffu, n0 > coh2 || n1 > coh2 || m0 > coh2x16 || m1 > coh2x16)) {
           const T f0 = factor(n0, coh2, coh), f1 = factor(n1, coh2, coh);
@@ -224,7 +230,7 @@ __device__ __forceinline__ void pair_march(const Geo& g, Io& io, int npairs_in, 
       T yr = y1;
       cq = c1;
       if (PLASTIC) {
-        yr = mul_rn(y1, factor(node_j2sq_h(x1, y1, corner_sum(ja + 1, h0, h1, hs1, hs2)), coh2, coh));
+        yr = mul_rn(y1, factor(node_j2sq_h(x1, y1, corner_sum(ja + 1, false, h0, h1, hs1, hs2)), coh2, coh));
         cq = mul_rn(c1, factor(corner_j2(x1, y1, c1, x2, y2), coh2x16, coh4));
       }
       syq = sub_rn(yr, p1);
