@@ -266,6 +266,15 @@ int ep2d_check_grid_barrier(int32_t device, int32_t blocks, int32_t missing, int
   return EP2D_OK;
 }
 
+int ep2d_check_chip_wait(ep2d_handle* h, int32_t missing, int64_t timeout_ns) {
+  if (!h) return fail(EP2D_ERR_ARG, "null handle");
+  if (missing < 0 || timeout_ns < 0 || timeout_ns > 10000000000LL)
+    return fail(EP2D_ERR_ARG, "need missing >= 0 and 0 <= timeout_ns <= 10 s");
+  h->rve.chip_waits.missing = missing;
+  h->rve.chip_waits.records_ns = (unsigned long long)timeout_ns;
+  return EP2D_OK;
+}
+
 // sizeof() of every ABI struct, for the binding's layout check
 int ep2d_abi_sizes(int64_t* out, int32_t n) {
   const int64_t s[7] = {(int64_t)sizeof(ep2d_params),      (int64_t)sizeof(ep2d_step_record),

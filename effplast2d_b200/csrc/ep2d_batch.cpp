@@ -430,7 +430,7 @@ int BatchEngine::run_waves(int64_t n, bool* done) {
       jobs.clear();
       for (int q : w.slots) jobs.push_back(slots_[q].rve->chip_job(d_flag_));
       const cudaError_t e = launch_iter_chip(jobs.data(), (int)jobs.size(), cfg.precision == EP2D_MIXED, w.shape,
-                                             (int)chunk, CHIP_TIMEOUT_NS, stream);
+                                             (int)chunk, ChipWaits{}, stream);
       if (e == cudaErrorCooperativeLaunchTooLarge && !*done) {  // no room for the CTAs here
         cudaGetLastError();
         waves_ok_ = use_waves_ = false;

@@ -341,22 +341,23 @@ const void* chip_kernel(bool plastic, bool mixed, bool track, int warps, int row
 
 template <int JOBS>
 cudaError_t launch_chip_jobs(const ChipJob* jobs, int njobs, const void* kern, const ChipShape& s, int n_iter, int blocks,
-                             unsigned long long timeout_ns, cudaStream_t stream, bool track = false) {
+                             const ChipWaits& waits, cudaStream_t stream, bool track = false) {
   ChipArgs<JOBS> a;
   a.njobs = njobs;
   a.warps = s.warps;
   a.rows = s.rows;
   a.n_iter = n_iter;
-  a.timeout_ns = timeout_ns;
+  a.timeout_ns = waits.records_ns;
   std::copy(jobs, jobs + njobs, a.job);
   void* args[] = {&a};
   const size_t sm = std::max(chip_smem_bytes(s.groups, s.warps, s.rows, track), (size_t)CHIP_SMEM_MIN);
-  return cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(32 * s.warps * s.groups), args, sm, stream);
+  return cudaLaunchCooperativeKernel(kern, dim3(std::max(blocks - waits.missing, 1)), dim3(32 * s.warps * s.groups), args,
+                                     sm, stream);
 }
 }  // namespace
 
 cudaError_t launch_iter_chip(ChipJob* jobs, int njobs, bool mixed, const ChipShape& s, int n_iter,
-                             unsigned long long timeout_ns, cudaStream_t stream, bool track, bool f32) {
+                             const ChipWaits& waits, cudaStream_t stream, bool track, bool f32) {
   if (njobs < 1 || njobs > CHIP_JOBS || ((track || f32) && njobs > 1) || n_iter < 2 || s.warps < 1 || s.groups < 1 ||
       s.warps * s.groups > CHIP_WARPS || s.rows < 2 || s.rows > 18 || (s.rows & 1) ||
       chip_smem_bytes(s.groups, s.warps, s.rows, track) > CHIP_SMEM)
@@ -376,10 +377,10 @@ cudaError_t launch_iter_chip(ChipJob* jobs, int njobs, bool mixed, const ChipSha
     const bool pl = jobs[0].plastic != 0;
     const void* kern = f32 ? (pl ? (const void*)k_iter_chip<1, 1, float, float> : (const void*)k_iter_chip<0, 1, float, float>)
                            : chip_kernel(pl, mixed, track && pl, s.warps * s.groups, s.rows);
-    return launch_chip_jobs<1>(jobs, 1, kern, s, n_iter, blocks, timeout_ns, stream, track && pl && !f32);
+    return launch_chip_jobs<1>(jobs, 1, kern, s, n_iter, blocks, waits, stream, track && pl && !f32);
   }
   const void* kern = mixed ? (const void*)k_iter_chip<2, CHIP_JOBS, double, float> : (const void*)k_iter_chip<2, CHIP_JOBS, double, double>;
-  return launch_chip_jobs<CHIP_JOBS>(jobs, njobs, kern, s, n_iter, blocks, timeout_ns, stream);
+  return launch_chip_jobs<CHIP_JOBS>(jobs, njobs, kern, s, n_iter, blocks, waits, stream);
 }
 
 cudaError_t launch_grid_barrier_check(unsigned* gbar, int blocks, int missing, int rounds,

@@ -10,6 +10,7 @@
 #include <mutex>
 #include <set>
 #include <thread>
+#include <utility>
 
 #include <sys/mman.h>
 #include <unistd.h>
@@ -682,8 +683,8 @@ int Rve::run_chip(int64_t n, bool* done) {
     // chunks of an even length keep the parity; a chunk of one iteration cannot arise
     const int64_t chunk = n > ((int64_t)1 << 30) ? (int64_t)1 << 29 : n;
     ChipJob job = chip_job(f.gbar + 2);
-    const cudaError_t e = launch_iter_chip(&job, 1, mixed(), chip, (int)chunk, CHIP_TIMEOUT_NS, stream,
-                                           track && !f32, f32);
+    const cudaError_t e = launch_iter_chip(&job, 1, mixed(), chip, (int)chunk, std::exchange(chip_waits, ChipWaits{}),
+                                           stream, track && !f32, f32);
     if (e == cudaErrorCooperativeLaunchTooLarge) {
       cudaGetLastError();
       chip = ChipShape{};

@@ -138,6 +138,7 @@ class Rve {
   // plain iterations is followed by one; in memory of their own where a small grid's are too small
   // (the FP32 phase: chip_f32_fits)
   char* d_rim = nullptr;
+  ChipWaits chip_waits;  // of the next on-chip launch
   // velocities stored in FP32 (the mixed path, and both phases of the FP32 bulk)
   bool mixed() const { return prm.precision == EP2D_MIXED || prm.precision == EP2D_F32_BULK; }
   // FP32 bulk: true while the state is in its FP32 form (u' in f.ux32/uy32)

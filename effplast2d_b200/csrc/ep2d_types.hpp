@@ -120,7 +120,12 @@ constexpr int CHIP_SMEM = 226 * 1024;
 // every CTA takes at least this much, of which no two fit an SM: a second CTA there would wait for the
 // first one's tensor memory, and the first for the second's rim
 constexpr int CHIP_SMEM_MIN = 116 * 1024;
-constexpr unsigned long long CHIP_TIMEOUT_NS = 10000000000ull;  // 10 s per wait
+// How long a launch's CTAs wait for one another; `missing` of them, the last ones, are left out
+// (ep2d_check_chip_wait).
+struct ChipWaits {
+  unsigned long long records_ns = 10000000000ull;  // for a neighbour's rim records
+  int missing = 0;
+};
 constexpr int CHIP_MIN_RUN = 8;  // shorter runs of plain iterations are launched one by one
 ChipShape chip_shape(int nx, int ny);
 // One RVE of an on-chip launch: its fields, rim records (chip_rim_bytes; zeroed by the launch),
@@ -148,13 +153,12 @@ size_t chip_rim_capacity(int nx, int ny);
 int chip_ctas(int nx, int ny, int groups, int warps, int rows);
 size_t chip_smem(int groups, int warps, int rows, bool track = false);
 // n_iter >= 2 plain iterations of the jobs' RVEs in one cooperative launch: CTAs of s.groups tiles of
-// s.warps x s.rows (s.ncx, s.ncy unused); fills in the jobs' tiles and CTAs.  Each wait gives up
-// after timeout_ns, which sets the job's flag
+// s.warps x s.rows (s.ncx, s.ncy unused); fills in the jobs' tiles and CTAs.  A wait for records that
+// gives up sets the job's flag
 // (track: also mark what yields, as launch_iter does; f32: the FP32 bulk's iterations, on
 // f.ux32/uy32; one job each)
 cudaError_t launch_iter_chip(ChipJob* jobs, int njobs, bool mixed, const ChipShape& s, int n_iter,
-                             unsigned long long timeout_ns, cudaStream_t stream, bool track = false,
-                             bool f32 = false);
+                             const ChipWaits& waits, cudaStream_t stream, bool track = false, bool f32 = false);
 // clear the M_YN / M_YC bits of every node
 cudaError_t launch_clear_track(const Geo& g, uint8_t* mask, cudaStream_t stream);
 // one iteration of the FP32 bulk (stream form, segments of seg_h rows): u' and V in

@@ -25,7 +25,7 @@ EXPORTS = (
     "ep2d_batch_solve", "ep2d_rve_footprint", "ep2d_server_create", "ep2d_server_submit", "ep2d_server_wait",
     "ep2d_server_stats", "ep2d_server_destroy", "ep2d_average_fields_noalloc", "ep2d_get_kernel_shape",
     "ep2d_compute_eff_damping", "ep2d_polar_fields", "ep2d_get_f32_iterations",
-    "ep2d_iterate_f32", "ep2d_track_plastic_zone", "ep2d_check_grid_barrier",
+    "ep2d_iterate_f32", "ep2d_track_plastic_zone", "ep2d_check_grid_barrier", "ep2d_check_chip_wait",
 )
 
 
@@ -81,6 +81,7 @@ def lib():
         L.ep2d_compute_eff_damping.argtypes = [vp, d, P(d), i32, d, P(i64)]
         L.ep2d_polar_fields.argtypes = [vp, d] + [P(d)] * 4 + [P(ctypes.c_uint8)]
         L.ep2d_check_grid_barrier.argtypes = [i32, i32, i32, i32, i64, P(i32), P(i32)]
+        L.ep2d_check_chip_wait.argtypes = [vp, i32, i64]
         _lib = L
     return _lib
 
@@ -176,6 +177,11 @@ class Solver:
 
     def iterate(self, n):
         _check(lib().ep2d_iterate(self._h, int(n)))
+
+    def check_chip_wait(self, missing, timeout_ns=2_000_000):
+        """the next on-chip launch leaves out its last `missing` CTAs and its waits give up
+        after timeout_ns (ep2d_check_chip_wait)"""
+        _check(lib().ep2d_check_chip_wait(self._h, int(missing), int(timeout_ns)))
 
     def track_plastic_zone(self, on=True):
         """get_sigma_2D.m's plastic zone: mark every node / corner that yields at any

@@ -423,6 +423,13 @@ int ep2d_get_kernel_shape(ep2d_handle* h, int32_t* kernel, int32_t* rows);
  * reference. */
 int ep2d_check_grid_barrier(int32_t device, int32_t blocks, int32_t missing, int32_t rounds, int64_t timeout_ns,
                             int32_t* passed, int32_t* flag);
+/* For checking the failure path of the on-chip form without a fault: the handle's next
+ * on-chip launch (one only) leaves out its last `missing` CTAs (one always runs), and its
+ * waits for a neighbour's values give up after timeout_ns (at most 10 s).  The neighbours of
+ * the missing CTAs then set the error flag, the others see it, the launch ends, and the
+ * handle's next checkpoint (or the end of ep2d_iterate / the time step) returns
+ * EP2D_ERR_CUDA.  No counterpart in the reference. */
+int ep2d_check_chip_wait(ep2d_handle* h, int32_t missing, int64_t timeout_ns);
 
 #ifdef __cplusplus
 }
