@@ -296,15 +296,15 @@ __global__ void __launch_bounds__(256) k_iter_batch(const BatchEntry* __restrict
 //
 // The barrier lives in device memory (`Fields::gbar`): gbar[0..1] is a 64-bit count of
 // arrivals, zeroed by the host before each launch; gbar[2] is an error flag, zero when
-// the RVE is created and never cleared.  Barrier k (k = 1, 2, ...) of a launch is passed
+// the RVE is created or reset.  Barrier k (k = 1, 2, ...) of a launch is passed
 // once the count reaches k x gridDim.x: each CTA adds 1 with release semantics after
 // its threads' stores (a CTA barrier first) and one thread polls the count with acquire
 // semantics (a CTA barrier after), the pattern of a semaphore between CTAs; the count
 // is never reset within a launch, so there is no generation to track.  Every wait is
 // bounded: a CTA that waits longer than timeout_ns sets the flag and returns, and a CTA
 // that sees the flag returns too, so a barrier that cannot complete ends the launch with
-// the flag set instead of hanging.  The flag stays set (later launches return at their
-// first barrier); the host reads it at every checkpoint and reports the RVE as failed.
+// the flag set instead of hanging.  The flag stays set until the RVE is reset (later launches return at
+// once); the host reads it at every checkpoint and reports the RVE as failed.
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;

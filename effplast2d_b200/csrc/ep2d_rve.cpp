@@ -534,7 +534,7 @@ int Rve::create(const ep2d_params& p, cudaStream_t s) {
   cp += align256(partial_elems(p) * sizeof(double));
   d_out = reinterpret_cast<double*>(cp);
   f.vmax = reinterpret_cast<unsigned long long*>(d_out + 2 * NAVG + holes.size());
-  f.gbar = reinterpret_cast<unsigned*>(d_out + 2 * NAVG + holes.size() + 2);  // zeroed above, never reset
+  f.gbar = reinterpret_cast<unsigned*>(d_out + 2 * NAVG + holes.size() + 2);
   cp += align256((2 * NAVG + n_samples(p) + 4) * sizeof(double));
   d_idx = reinterpret_cast<unsigned long long*>(cp);
   cp += align256(n_samples(p) * sizeof(unsigned long long));
@@ -565,8 +565,10 @@ int Rve::reset() {
   // the 13 field arrays are contiguous at the start of the allocation
   const size_t bytes = reinterpret_cast<char*>(const_cast<uint8_t*>(f.mask)) - static_cast<char*>(dmem);
   EP2D_CK(cudaMemsetAsync(dmem, 0, bytes, stream));
+  EP2D_CK(cudaMemsetAsync(f.gbar, 0, 4 * sizeof(unsigned), stream));  // with the error flag
   EP2D_CK(cudaStreamSynchronize(stream));
   cur = 0;
+  f32 = vmax_zero_ = false;  // a step that failed may have left them set
   nts.assign(prm.nl, 0);
   rec.assign(prm.nl, {});
   checks.assign(prm.nl, {});

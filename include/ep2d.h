@@ -234,7 +234,8 @@ int ep2d_create(const ep2d_params* params, ep2d_handle** out);
 int ep2d_destroy(ep2d_handle* h);
 /* Return a handle to the state of a freshly constructed object (EffPlast2D.cu:1585-1604:
  * every field zero, no records) without reallocating.  The reference object keeps its
- * velocities across ComputeEffModuli calls; a new object starts from rest, as this does. */
+ * velocities across ComputeEffModuli calls; a new object starts from rest, as this does.
+ * A handle whose kernel gave up a wait (EP2D_ERR_CUDA) is usable again after it. */
 int ep2d_reset(ep2d_handle* h);
 
 /* Exactly n pseudo-time iterations of the reference's kernel sequence

@@ -48,3 +48,24 @@ def test_chip_wait_arguments():
             s.check_chip_wait(**kw)
         assert e.value.status == ep.ERR_ARG
     s.close()
+
+
+@pytest.mark.parametrize("precision", [ep.FP64, ep.F32_BULK], ids=["fp64", "f32"])
+def test_reset_after_a_failed_wait_gives_a_fresh_handle(precision):
+    # (in the FP32 phase the failed step also leaves the state in its FP32 form)
+    nx, ny = 130, 96
+    kw = dict(niter=120, check_every=40, precision=precision)
+    s, _ = _solver(nx, ny, **kw)
+    s.check_chip_wait(missing=1)
+    with pytest.raises(ep.EP2DError) as e:
+        s.solve_step(0, -6e-5, [1.0, 0.8, 0.3])
+    assert e.value.status == ep.ERR_CUDA
+    s.reset()
+    r = s.solve_step(0, -6e-5, [1.0, 0.8, 0.3])[0]
+    t, _ = _solver(nx, ny, **kw)
+    q = t.solve_step(0, -6e-5, [1.0, 0.8, 0.3])[0]
+    assert r["iterations"] == q["iterations"] and r["sigma"] == q["sigma"]
+    for f in FIELDS:
+        assert np.array_equal(s.get(f), t.get(f)), f
+    s.close()
+    t.close()
