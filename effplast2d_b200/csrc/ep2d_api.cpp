@@ -270,8 +270,22 @@ int ep2d_check_chip_wait(ep2d_handle* h, int32_t missing, int64_t timeout_ns) {
   if (!h) return fail(EP2D_ERR_ARG, "null handle");
   if (missing < 0 || timeout_ns < 0 || timeout_ns > 10000000000LL)
     return fail(EP2D_ERR_ARG, "need missing >= 0 and 0 <= timeout_ns <= 10 s");
-  h->rve.chip_waits.missing = missing;
-  h->rve.chip_waits.records_ns = (unsigned long long)timeout_ns;
+  ep2d::ChipWaits w;
+  w.records_ns = (unsigned long long)timeout_ns;
+  w.missing = missing;
+  w.missing_started = true;
+  h->rve.chip_waits = w;
+  return EP2D_OK;
+}
+
+int ep2d_check_chip_start(ep2d_handle* h, int32_t missing, int64_t timeout_ns) {
+  if (!h) return fail(EP2D_ERR_ARG, "null handle");
+  if (missing < 0 || timeout_ns < 0 || timeout_ns > 10000000000LL)
+    return fail(EP2D_ERR_ARG, "need missing >= 0 and 0 <= timeout_ns <= 10 s");
+  ep2d::ChipWaits w;
+  w.start_ns = (unsigned long long)timeout_ns;
+  w.missing = missing;
+  h->rve.chip_waits = w;
   return EP2D_OK;
 }
 

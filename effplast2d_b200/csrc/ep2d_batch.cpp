@@ -11,6 +11,7 @@
 #include <mutex>
 #include <set>
 #include <thread>
+#include <utility>
 
 namespace ep2d {
 
@@ -74,9 +75,9 @@ BatchEngine::~BatchEngine() {
   cudaFree(d_tiles_);
   cudaFree(d_ntiles_);
   cudaFree(d_vmax_);
-  cudaFree(d_flag_);
+  cudaFree(d_state_);
   if (h_vmax_) cudaFreeHost(h_vmax_);
-  if (h_flag_) cudaFreeHost(h_flag_);
+  if (h_state_) cudaFreeHost(h_state_);
   cudaStreamDestroy(stream);
 }
 
@@ -100,9 +101,6 @@ int BatchEngine::init(const ep2d_batch_config& c) {
   EP2D_CK(cudaEventCreate(&ev_[0]));
   EP2D_CK(cudaEventCreate(&ev_[1]));
   EP2D_CK(cudaMalloc(&d_ntiles_, sizeof(int)));
-  EP2D_CK(cudaMalloc(&d_flag_, sizeof(unsigned)));
-  EP2D_CK(cudaMemsetAsync(d_flag_, 0, sizeof(unsigned), stream));
-  EP2D_CK(cudaMallocHost(&h_flag_, sizeof(unsigned)));
   shape.form = c.kernel == EP2D_KERNEL_TILE ? FORM_TILE : FORM_STREAM;
   shape.rows = c.rows ? c.rows : (shape.form == FORM_TILE ? TILE_Y : SEG_DEFAULT);
   tuned = c.rows != 0;
@@ -129,13 +127,19 @@ int BatchEngine::grow(int need) {
   EP2D_CK(cudaStreamSynchronize(stream));
   cudaFree(d_ents_);
   cudaFree(d_vmax_);
+  cudaFree(d_state_);
   if (h_vmax_) cudaFreeHost(h_vmax_);
+  if (h_state_) cudaFreeHost(h_state_);
   d_ents_ = nullptr;
   d_vmax_ = nullptr;
+  d_state_ = nullptr;
   h_vmax_ = nullptr;
+  h_state_ = nullptr;
   EP2D_CK(cudaMalloc(&d_ents_, cap * sizeof(BatchEntry)));
   EP2D_CK(cudaMalloc(&d_vmax_, cap * 2 * sizeof(unsigned long long)));
   EP2D_CK(cudaMallocHost(&h_vmax_, cap * 2 * sizeof(unsigned long long)));
+  EP2D_CK(cudaMalloc(&d_state_, cap * sizeof(unsigned)));
+  EP2D_CK(cudaMallocHost(&h_state_, cap * sizeof(unsigned)));
   cap_slots_ = cap;
   if (graph_) {  // the graph holds the old pointers
     cudaGraphExecDestroy(graph_);
@@ -426,11 +430,12 @@ int BatchEngine::run_waves(int64_t n, bool* done) {
   *done = false;
   while (n > 0) {  // chunks of an even length keep the parity
     const int64_t chunk = n > ((int64_t)1 << 30) ? (int64_t)1 << 29 : n;
+    EP2D_CK(cudaMemsetAsync(d_state_, 0, slots_.size() * sizeof(unsigned), stream));
     for (const Wave& w : waves_) {
       jobs.clear();
-      for (int q : w.slots) jobs.push_back(slots_[q].rve->chip_job(d_flag_));
+      for (int q : w.slots) jobs.push_back(slots_[q].rve->chip_job(d_state_ + q, 0));
       const cudaError_t e = launch_iter_chip(jobs.data(), (int)jobs.size(), cfg.precision == EP2D_MIXED, w.shape,
-                                             (int)chunk, ChipWaits{}, stream);
+                                             (int)chunk, std::exchange(chip_waits, ChipWaits{}), stream);
       if (e == cudaErrorCooperativeLaunchTooLarge && !*done) {  // no room for the CTAs here
         cudaGetLastError();
         waves_ok_ = use_waves_ = false;
@@ -441,12 +446,30 @@ int BatchEngine::run_waves(int64_t n, bool* done) {
       launches++;
       for (int q : w.slots) slots_[q].rve->cur ^= (int)(chunk & 1);
     }
+    EP2D_CK(cudaMemcpyAsync(h_state_, d_state_, slots_.size() * sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
+    EP2D_CK(cudaStreamSynchronize(stream));
+    for (const Wave& w : waves_)
+      for (int q : w.slots) {
+        if (h_state_[q] & CHIP_STALLED)
+          return fail(EP2D_ERR_CUDA, "on-chip form: a wait for another CTA ran out; the batch's state is invalid");
+        if (h_state_[q] & CHIP_GAVE_UP) {
+          waves_ok_ = use_waves_ = false;
+          slots_[q].rve->cur ^= (int)(chunk & 1);
+          const int rc = run_off_chip(q, chunk);
+          if (rc) return rc;
+        }
+      }
     n -= chunk;
   }
-  EP2D_CK(cudaMemcpyAsync(h_flag_, d_flag_, sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
-  EP2D_CK(cudaStreamSynchronize(stream));
-  if (*h_flag_) return fail(EP2D_ERR_CUDA, "on-chip form: a wait for another CTA ran out; the batch's state is invalid");
   return EP2D_OK;
+}
+
+int BatchEngine::run_off_chip(int q, int64_t n) {
+  Rve& r = *slots_[q].rve;
+  const int64_t before = r.launches;
+  const int rc = r.run_off_chip(n);
+  launches += r.launches - before;
+  return rc;
 }
 
 int BatchEngine::advance(Slot& s, double error) {
@@ -848,25 +871,15 @@ struct ep2d_server {
   ep2d::Server srv;
 };
 
-extern "C" {
-
-int64_t ep2d_rve_footprint(const ep2d_rve_spec* spec, int32_t precision) {
-  if (!spec) return -1;
-  ep2d_batch_config c{};
-  c.check_every = 2;
-  c.niter = 2;
-  c.precision = precision;
-  return (int64_t)ep2d::Rve::footprint(ep2d::params_of(c, *spec));
-}
-
-int ep2d_batch_solve(const ep2d_batch_config* cfg, const ep2d_rve_spec* specs, int32_t n, ep2d_result* results,
-                     ep2d_batch_stats* stats) {
+static int batch_solve(const ep2d_batch_config* cfg, const ep2d_rve_spec* specs, int32_t n, ep2d_result* results,
+                       ep2d_batch_stats* stats, const ep2d::ChipWaits& waits) {
   if (!cfg || (!specs && n > 0) || n < 0) return fail(EP2D_ERR_ARG, "null argument");
   try {
     const double t0 = ep2d::now_s();
     ep2d::BatchEngine eng;
     int rc = eng.init(*cfg);
     if (rc) return rc;
+    eng.chip_waits = waits;
     size_t need = 0;
     for (int k = 0; k < n; k++) {
       rc = ep2d::validate_params(ep2d::params_of(*cfg, specs[k]));
@@ -909,6 +922,32 @@ int ep2d_batch_solve(const ep2d_batch_config* cfg, const ep2d_rve_spec* specs, i
   } catch (const std::exception& ex) {
     return fail(EP2D_ERR_STATE, std::string("exception: ") + ex.what());
   }
+}
+
+extern "C" {
+
+int64_t ep2d_rve_footprint(const ep2d_rve_spec* spec, int32_t precision) {
+  if (!spec) return -1;
+  ep2d_batch_config c{};
+  c.check_every = 2;
+  c.niter = 2;
+  c.precision = precision;
+  return (int64_t)ep2d::Rve::footprint(ep2d::params_of(c, *spec));
+}
+
+int ep2d_batch_solve(const ep2d_batch_config* cfg, const ep2d_rve_spec* specs, int32_t n, ep2d_result* results,
+                     ep2d_batch_stats* stats) {
+  return batch_solve(cfg, specs, n, results, stats, ep2d::ChipWaits{});
+}
+
+int ep2d_check_batch_start(const ep2d_batch_config* cfg, const ep2d_rve_spec* specs, int32_t n, int32_t missing,
+                           int64_t timeout_ns, ep2d_result* results, ep2d_batch_stats* stats) {
+  if (missing < 0 || timeout_ns < 0 || timeout_ns > 10000000000LL)
+    return fail(EP2D_ERR_ARG, "need missing >= 0 and 0 <= timeout_ns <= 10 s");
+  ep2d::ChipWaits w;
+  w.missing = missing;
+  w.start_ns = (unsigned long long)timeout_ns;
+  return batch_solve(cfg, specs, n, results, stats, w);
 }
 
 int ep2d_server_create(const ep2d_batch_config* cfg, int64_t mem_budget_bytes, int32_t max_active, ep2d_server** out) {

@@ -68,6 +68,7 @@ class BatchEngine {
   int solo_intervals = 0;  // checkpoint intervals an RVE ran through the single-RVE path
   double tune_us[7] = {0, 0, 0, 0, 0, 0, 0};  // tile rows 8/16/32, stream rows 8/16/32/64
   void fill_stats(ep2d_batch_stats* st) const;
+  ChipWaits chip_waits;  // of the next on-chip launch (ep2d_check_batch_start)
 
  private:
   struct Slot {
@@ -92,6 +93,7 @@ class BatchEngine {
   };
   bool plan_waves(const std::vector<char>& batched);  // false: the batched launches are faster
   int run_waves(int64_t n, bool* done);               // n plain iterations of every RVE of the waves
+  int run_off_chip(int slot, int64_t n);              // ... of one RVE that an on-chip launch has left as it was
   int grow(int need);
 
   std::vector<Slot> slots_;
@@ -109,8 +111,8 @@ class BatchEngine {
   uint64_t waves_version_ = ~0ull;  // set_version_ they were planned for
   bool use_waves_ = false;
   bool waves_ok_ = true;            // false: the device has no room for their CTAs
-  unsigned* d_flag_ = nullptr;      // error flag of the on-chip launches
-  unsigned* h_flag_ = nullptr;
+  unsigned* d_state_ = nullptr;     // the slots' state words in the on-chip launches
+  unsigned* h_state_ = nullptr;
   uint64_t set_version_ = 0;    // bumped whenever an RVE joins or retires
   uint64_t tuned_version_ = 0;  // set_version_ the current shape was tuned for
   cudaGraphExec_t graph_ = nullptr;

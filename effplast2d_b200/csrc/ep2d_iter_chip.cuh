@@ -17,9 +17,11 @@
 // fence, flag or grid-wide barrier (each 64-bit {word, tag} is an element of one vector
 // store and valid on its own).  Records are double-buffered by iteration parity: a CTA
 // overwrites iteration t's records in iteration t + 2, after it has read its neighbours'
-// records of t + 1, which they wrote after reading all of t's.  Waits are bounded: a CTA that
-// waits longer than timeout_ns sets its RVE's error flag and leaves, the others
-// follow, and the host reports the RVE as failed.
+// records of t + 1, which they wrote after reading all of t's.  Waits are bounded.  Each CTA counts
+// itself in the RVE's state word as it starts; where one cannot (other work holds its SM),
+// its neighbours' waits give up after start_ns, every CTA leaves without having written the
+// state, and the host runs the iterations in another form.  A wait for a CTA that has started
+// gives up after records_ns, and the host reports the RVE as failed.
 //
 // Within a CTA the two lowest and two highest rows of a warp are read by the warps below
 // and above and are double-buffered by parity; the rows between are updated in place.
@@ -72,6 +74,39 @@ __device__ __forceinline__ bool group_barrier_or(int id, int threads, int flag) 
       : "r"(flag), "r"(id), "r"(threads)
       : "memory");
   return r != 0;
+}
+
+// Waited longer than start_ns (long_wait: than records_ns) for another CTA of the job.
+__device__ __forceinline__ void chip_give_up(const ChipJob& job, bool long_wait) {
+  unsigned w = *reinterpret_cast<volatile unsigned*>(job.state);
+  while (!(w & CHIP_FAILED)) {
+    const bool all = (w & CHIP_COUNT) == job.full;
+    if (all && !long_wait) return;
+    const unsigned old = atomicCAS(job.state, w, w | (all ? CHIP_STALLED : CHIP_GAVE_UP));
+    if (old == w) return;
+    w = old;
+  }
+}
+// The time a wait has taken in ns, looked at now and then: time between two looks counts as at most
+// 10 ms, so that time in which the GPU runs another context does not.
+struct ChipClock {
+  unsigned waited = 0, last = 0;  // in units of 1024 ns
+  __device__ __forceinline__ unsigned long long look() {
+    const unsigned now = (unsigned)(global_ns() >> 10) | 1u;
+    if (last) waited += min(now - last, 9766u);
+    last = now;
+    return (unsigned long long)waited << 10;
+  }
+};
+// Waits until all CTAs of the job have started; false if the launch has given up.  Called by whole warps.
+__device__ __forceinline__ bool chip_all_started(const ChipJob& job, unsigned long long start_ns) {
+  ChipClock clock;
+  for (unsigned tries = 1;; tries++) {
+    const unsigned w = *reinterpret_cast<volatile unsigned*>(job.state);
+    if (__any_sync(0xffffffffu, (w & CHIP_FAILED) != 0)) return false;
+    if (__all_sync(0xffffffffu, (w & CHIP_COUNT) == job.full)) return true;
+    if ((tries & 1023u) == 0 && clock.look() > start_ns) chip_give_up(job, false);
+  }
 }
 
 // index of the material constants of node (i, r) and corner (i, r): bits 0-1 the node's
@@ -295,7 +330,9 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_consta
   const int H = nw * rows, x0 = STREAM_COLS * cx, y0 = H * cy;
   const int npairs = rows / 2, ppw = chip_pairs_per_warp(rows);
   const int ncol = chip_col_polls(rows), npoll = chip_polls(nw, rows);
-  if (__syncthreads_or(*reinterpret_cast<volatile unsigned*>(job.flag) != 0)) return;  // an earlier launch failed
+  // counted before anything is published: a tile whose neighbours' records have come knows they started
+  unsigned state = 0;
+  if (threadIdx.x == 0) state = atomicAdd(job.state, 1u);
 
   MatT<T>* mats = reinterpret_cast<MatT<T>*>(smem_raw);
   char* urows = reinterpret_cast<char*>(smem_raw) + N_MATS * sizeof(MatT<T>) + group * chip_group_bytes(nw, rows, US);
@@ -314,8 +351,8 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_consta
   // the recording launch that follows folds max|V| into the pair
   if ((int)blockIdx.x == job.cta0 && threadIdx.x < 2) f.vmax[threadIdx.x] = 0;
   for (int t = threadIdx.x; t < N_MATS; t += blockDim.x) mats[t] = mat_entry<T>(g, t);
-  __syncthreads();
-  if (!idle) {
+  const bool late = __syncthreads_or((state & CHIP_FAILED) != 0);  // the others have given up
+  if (!idle && !late) {
     const int i = x0 - 2 + lane;
     const int jA = y0 + w * rows;
 #pragma unroll 4
@@ -474,7 +511,7 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_consta
           wait[k] = e[k].x != 0xffffffffu;
         }
         unsigned tries = 0;
-        unsigned long long since = 0;
+        ChipClock clock;
         for (;;) {
           bool any = false;
 #pragma unroll
@@ -486,11 +523,10 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_consta
             any |= wait[k];
           }
           if (!__any_sync(0xffffffffu, any)) break;
-          if ((++tries & 1023u) == 0) {  // bounded: look at the clock and the error flag now and then
-            const unsigned long long now = global_ns();
-            if (since == 0) since = now;
-            if (now - since > a.timeout_ns) atomicExch(job.flag, 1u);
-            if (__any_sync(0xffffffffu, *reinterpret_cast<volatile unsigned*>(job.flag) != 0)) {
+          if ((++tries & 1023u) == 0) {  // bounded: look at the clock and the state word now and then
+            const unsigned long long waited = clock.look();
+            if (waited > min(a.start_ns, a.records_ns)) chip_give_up(job, waited > a.records_ns);
+            if (__any_sync(0xffffffffu, (*reinterpret_cast<volatile unsigned*>(job.state) & CHIP_FAILED) != 0)) {
               failed = 1;
               break;
             }
@@ -506,8 +542,12 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_consta
       if (group_barrier_or(1 + group, 32 * nw, failed)) break;
     }
 
-    // back to global memory: U of the last copy written, V
-    if (jA < ny) {
+    // Back to global memory: U of the last copy written, V -- unless the launch has failed.  A tile that
+    // has gone through n iterations has records that go back to every tile up to n - 1 away, so all have
+    // started; after fewer it has to look.
+    bool write = it + 1 >= n_iter;
+    if (write && n_iter < max(ncx, ncy)) write = chip_all_started(job, a.start_ns);
+    if (write && jA < ny) {
       __syncwarp();
       T* uxo = u_field<T>(f, false, src ^ (n_iter & 1));
       T* uyo = u_field<T>(f, true, src ^ (n_iter & 1));

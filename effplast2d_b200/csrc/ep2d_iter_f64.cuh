@@ -60,7 +60,7 @@ __device__ __forceinline__ T ld_field(const T* p) {
 
 template <int TX, int TY, bool PLASTIC, bool RECORD, typename TV, bool COH = false>
 __device__ __forceinline__ void iter_tile(const Geo& g, const Fields& f, const int src, const int bx, const int by,
-                                          TileSmem<TX, TY>& s) {
+                                          TileSmem<TX, TY>& s, bool skip = false) {
   static_assert(TX == 32 && TY % 8 == 0, "the thread mapping assumes 32 x 8 threads and TX == 32");
   using S = TileSmem<TX, TY>;
   constexpr int UW = S::UW, UH = S::UH, SW = S::SW, SH = S::SH, FW = S::FW, FH = S::FH;
@@ -195,6 +195,8 @@ __device__ __forceinline__ void iter_tile(const Geo& g, const Fields& f, const i
     __syncthreads();
   }
 
+  if (skip) return;  // all threads
+
   // ---- D: damped momentum update and U += V dt on the owned faces
   const double dT = g.dT, cX = g.cX, cY = g.cY, dtrX = g.dtrX, dtrY = g.dtrY;
   double vmx = 0.0, vmy = 0.0;
@@ -255,12 +257,19 @@ __device__ __forceinline__ void iter_tile(const Geo& g, const Fields& f, const i
   }
 }
 
+// An on-chip launch has given up (CHIP_GAVE_UP): the recording launch behind it leaves the state
+// alone (U and V; the stresses it is there to write anew), and the host runs the interval again.
+__device__ __forceinline__ bool chip_failed(const Fields& f) {
+  return (*reinterpret_cast<const volatile unsigned*>(f.gbar + 3) & CHIP_FAILED) != 0;
+}
+
 // One RVE: one CTA per tile.
 template <int TX, int TY, bool PLASTIC, bool RECORD, typename TV>
 __global__ void __launch_bounds__(256) k_iter(Geo g, Fields f, int src) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  const bool skip = RECORD && chip_failed(f);
   iter_tile<TX, TY, PLASTIC, RECORD, TV>(g, f, src, blockIdx.x, blockIdx.y,
-                                         *reinterpret_cast<TileSmem<TX, TY>*>(smem_raw));
+                                         *reinterpret_cast<TileSmem<TX, TY>*>(smem_raw), skip);
 }
 
 // Many RVEs: a persistent grid walks the device-side tile list {rve, bx | by << 16}.

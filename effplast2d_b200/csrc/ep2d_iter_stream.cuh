@@ -424,6 +424,10 @@ __global__ void __launch_bounds__(32 * STREAM_WARPS) k_iter_stream(Geo g, Fields
   const int task = blockIdx.x * STREAM_WARPS + (threadIdx.x >> 5);
   if (task >= nstrips * nsegs) return;  // whole warp
   double vmx = 0.0, vmy = 0.0;
+  if (RECORD) {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    if (chip_failed(f)) return;
+  }
   stream_segment<PLASTIC, RECORD, TU, TV, TRACK>(g, f, src, task % nstrips, task / nstrips, seg_h, sm, vmx, vmy);
   stream_fold_vmax<RECORD>(vmx, vmy, f.vmax);
 }

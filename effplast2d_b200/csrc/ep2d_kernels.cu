@@ -347,12 +347,12 @@ cudaError_t launch_chip_jobs(const ChipJob* jobs, int njobs, const void* kern, c
   a.warps = s.warps;
   a.rows = s.rows;
   a.n_iter = n_iter;
-  a.timeout_ns = waits.records_ns;
+  a.start_ns = waits.start_ns;
+  a.records_ns = waits.records_ns;
   std::copy(jobs, jobs + njobs, a.job);
   void* args[] = {&a};
   const size_t sm = std::max(chip_smem_bytes(s.groups, s.warps, s.rows, track), (size_t)CHIP_SMEM_MIN);
-  return cudaLaunchCooperativeKernel(kern, dim3(std::max(blocks - waits.missing, 1)), dim3(32 * s.warps * s.groups), args,
-                                     sm, stream);
+  return cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(32 * s.warps * s.groups), args, sm, stream);
 }
 }  // namespace
 
@@ -365,14 +365,19 @@ cudaError_t launch_iter_chip(ChipJob* jobs, int njobs, bool mixed, const ChipSha
   int blocks = 0;
   for (int k = 0; k < njobs; k++) {
     ChipJob& j = jobs[k];
-    if (!j.rim || !j.flag) return cudaErrorInvalidValue;
+    if (!j.rim || !j.state) return cudaErrorInvalidValue;
     j.ncx = (j.g.nx + STREAM_COLS - 1) / STREAM_COLS;
     j.ncy = (j.g.ny + s.warps * s.rows - 1) / (s.warps * s.rows);
     j.cta0 = blocks;
     const cudaError_t e = cudaMemsetAsync(j.rim, 0, chip_rim_bytes(j.g.nx, j.g.ny, s.warps, s.rows, f32), stream);
     if (e != cudaSuccess) return e;
-    blocks += (j.ncx * j.ncy + s.groups - 1) / s.groups;
+    const int ctas = (j.ncx * j.ncy + s.groups - 1) / s.groups;
+    blocks += ctas;
+    j.full = j.count0 + ctas;
   }
+  const int missing = std::min(waits.missing, blocks - jobs[njobs - 1].cta0 - 1);  // of the last job
+  blocks -= missing;
+  if (waits.missing_started) jobs[njobs - 1].full -= missing;
   if (njobs == 1) {
     const bool pl = jobs[0].plastic != 0;
     const void* kern = f32 ? (pl ? (const void*)k_iter_chip<1, 1, float, float> : (const void*)k_iter_chip<0, 1, float, float>)

@@ -565,7 +565,8 @@ int Rve::reset() {
   // the 13 field arrays are contiguous at the start of the allocation
   const size_t bytes = reinterpret_cast<char*>(const_cast<uint8_t*>(f.mask)) - static_cast<char*>(dmem);
   EP2D_CK(cudaMemsetAsync(dmem, 0, bytes, stream));
-  EP2D_CK(cudaMemsetAsync(f.gbar, 0, 4 * sizeof(unsigned), stream));  // with the error flag
+  EP2D_CK(cudaMemsetAsync(f.gbar, 0, 4 * sizeof(unsigned), stream));  // with what a wait that ran out has set
+  chip_count = 0;
   EP2D_CK(cudaStreamSynchronize(stream));
   cur = 0;
   f32 = vmax_zero_ = false;  // a step that failed may have left them set
@@ -665,43 +666,57 @@ int Rve::capture(int parity) {
   return EP2D_OK;
 }
 
-ChipJob Rve::chip_job(unsigned* flag) const {
+ChipJob Rve::chip_job(unsigned* state, unsigned count0) const {
   ChipJob j{};
   j.g = g;
   j.f = f;
   j.rim = f32 ? reinterpret_cast<char*>(f.ux[0]) : d_rim;
-  j.flag = flag;
+  j.state = state;
+  j.count0 = count0;
   j.src = cur;
   j.plastic = prm.nl > 1 ? 1 : 0;
   return j;
 }
 
-// n plain iterations in one launch of the on-chip form; *done = false where the device has no
+// *n plain iterations in one launch of the on-chip form; *n: those left, where the device has no
 // room for its CTAs (the other forms take over for good).
-int Rve::run_chip(int64_t n, bool* done) {
+int Rve::run_chip(int64_t* n) {
   take_turn();
-  *done = true;
-  while (n > 0) {
+  const ChipShape s = chip;
+  bool launched = false;
+  while (*n > 0 && chip.warps) {
     // chunks of an even length keep the parity; a chunk of one iteration cannot arise
-    const int64_t chunk = n > ((int64_t)1 << 30) ? (int64_t)1 << 29 : n;
-    ChipJob job = chip_job(f.gbar + 2);
-    const cudaError_t e = launch_iter_chip(&job, 1, mixed(), chip, (int)chunk, std::exchange(chip_waits, ChipWaits{}),
-                                           stream, track && !f32, f32);
+    const int64_t chunk = *n > ((int64_t)1 << 30) ? (int64_t)1 << 29 : *n;
+    const bool more = chunk < *n, record = last_.record;
+    if (more) last_ = {chunk, false, cur};
+    if (chip_count > CHIP_COUNT / 2) {
+      EP2D_CK(cudaMemsetAsync(f.gbar + 3, 0, sizeof(unsigned), stream));
+      chip_count = 0;
+    }
+    ChipJob job = chip_job(f.gbar + 3, chip_count);
+    const ChipWaits waits = std::exchange(chip_waits, ChipWaits{});
+    const cudaError_t e = launch_iter_chip(&job, 1, mixed(), s, (int)chunk, waits, stream, track && !f32, f32);
     if (e == cudaErrorCooperativeLaunchTooLarge) {
       cudaGetLastError();
       chip = ChipShape{};
-      *done = false;
-      return EP2D_OK;
+      break;
     }
     EP2D_CK(e);
+    chip_count = job.full;
     cur ^= (int)(chunk & 1);
     launches++;
     resident_launches++;
-    n -= chunk;
+    launched = true;
+    *n -= chunk;
+    if (more) {  // the next chunk starts from this one's result
+      const int rc = check_resident();
+      if (rc) return rc;
+      last_ = {*n, record, cur};
+    }
   }
   // the padding beside the displacements is read as zeros
-  if (f32) EP2D_CK(cudaMemsetAsync(f.ux[0], 0, chip_rim_bytes(prm.nx, prm.ny, chip.warps, chip.rows, true), stream));
-  vmax_zero_ = true;
+  if (f32 && launched) EP2D_CK(cudaMemsetAsync(f.ux[0], 0, chip_rim_bytes(prm.nx, prm.ny, s.warps, s.rows, true), stream));
+  vmax_zero_ = launched && *n == 0 && chip.warps;
   return EP2D_OK;
 }
 
@@ -728,9 +743,8 @@ bool Rve::chip_f32_fits() const {
 int Rve::run_plain(int64_t n) {
   if (chip.warps && n >= CHIP_MIN_RUN &&
       (f32 ? chip_f32_fits() : !track || chip_smem(chip.groups, chip.warps, chip.rows, true) <= CHIP_SMEM)) {
-    bool done = false;
-    const int rc = run_chip(n, &done);
-    if (rc || done) return rc;
+    const int rc = run_chip(&n);
+    if (rc || n == 0) return rc;
   }
   if (shape.form == FORM_RESIDENT && !f32 && !track) {
     // one cooperative launch for all n iterations (n == 1: an ordinary tile launch)
@@ -772,14 +786,17 @@ int Rve::reset_vmax() {
   return EP2D_OK;
 }
 
-int Rve::iterate(int64_t n, bool record_last) {
-  if (n <= 0) return EP2D_OK;
-  DeviceScope ds(device);
-  TurnScope ts{*this};
-  EP2D_CK(cudaEventRecord(ev_[0], stream));
-  int rc = run_plain(record_last ? n - 1 : n);
+int Rve::run_off_chip(int64_t n) {
+  chip = ChipShape{};
+  if (prm.kernel == EP2D_KERNEL_AUTO && shape.form == FORM_RESIDENT) shape.form = FORM_TILE;
+  return run_plain(n);
+}
+
+int Rve::launch_interval(int64_t n, bool record) {
+  last_ = {n, record, cur};
+  int rc = run_plain(n);
   if (rc) return rc;
-  if (record_last) {
+  if (record) {
     rc = reset_vmax();
     if (rc) return rc;
     rc = launch_one(true);
@@ -787,8 +804,18 @@ int Rve::iterate(int64_t n, bool record_last) {
     launches++;
   }
   vmax_zero_ = false;
+  return EP2D_OK;
+}
+
+int Rve::iterate(int64_t n, bool record_last) {
+  if (n <= 0) return EP2D_OK;
+  DeviceScope ds(device);
+  TurnScope ts{*this};
+  EP2D_CK(cudaEventRecord(ev_[0], stream));
+  int rc = launch_interval(record_last ? n - 1 : n, record_last);
+  if (rc) return rc;
   EP2D_CK(cudaEventRecord(ev_[1], stream));
-  rc = check_resident();  // waits for the stream, if it has a flag to read
+  rc = check_resident();  // waits for the stream, if it has words to read
   if (rc) return rc;
   EP2D_CK(cudaEventSynchronize(ev_[1]));
   end_turn();
@@ -806,27 +833,49 @@ double Rve::error_from_vmax(double vmx, double vmy) const {
   return (vmx / (d.dX * (prm.nx - 1)) + vmy / (d.dY * (prm.ny - 1))) * d.dT / std::max(a, b);
 }
 
-static int failed_wait() {
-  return fail(EP2D_ERR_CUDA, "resident or on-chip form: a wait for another CTA ran out; the RVE's state is invalid");
+// words: the resident form's error flag and the on-chip form's state word.  An on-chip launch that
+// gave up before all its CTAs had started, and the recording launch behind it, have left the state as
+// it was: the interval runs again, now and from here on, in the forms whose CTAs do not wait for one
+// another (*again).
+int Rve::look_at_waits(const unsigned words[2], bool* again) {
+  *again = false;
+  if (words[0] || (words[1] & CHIP_STALLED))
+    return fail(EP2D_ERR_CUDA, "resident or on-chip form: a wait for another CTA ran out; the RVE's state is invalid");
+  if (!(words[1] & CHIP_GAVE_UP)) return EP2D_OK;
+  *again = true;
+  EP2D_CK(cudaMemsetAsync(f.gbar + 3, 0, sizeof(unsigned), stream));
+  chip_count = 0;
+  chip = ChipShape{};
+  if (prm.kernel == EP2D_KERNEL_AUTO && shape.form == FORM_RESIDENT) shape.form = FORM_TILE;
+  cur = last_.cur;
+  return launch_interval(last_.n, last_.record);
 }
 
-// The error flag of the forms whose CTAs wait on one another (sticky), read back; EP2D_OK if
-// the RVE never ran one.
+// The words of the forms whose CTAs wait on one another, read back; nothing to do if the RVE never ran
+// one.
 int Rve::check_resident() {
   if (!resident_launches) return EP2D_OK;
   unsigned* hf = reinterpret_cast<unsigned*>(h_pin + 2 * NAVG + holes.size() + 2);
-  EP2D_CK(cudaMemcpyAsync(hf, f.gbar + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
-  EP2D_CK(cudaStreamSynchronize(stream));
-  return *hf ? failed_wait() : EP2D_OK;
+  for (bool again = true; again;) {
+    EP2D_CK(cudaMemcpyAsync(hf, f.gbar + 2, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
+    EP2D_CK(cudaStreamSynchronize(stream));
+    const int rc = look_at_waits(hf, &again);
+    if (rc) return rc;
+  }
+  return EP2D_OK;
 }
 
 int Rve::read_error(double* error) {
-  // the max|V| pair and, right behind it, the barrier words with the error flag (check_resident)
+  // the max|V| pair and, right behind it, the barrier's count and the words of check_resident
   unsigned long long* hv = reinterpret_cast<unsigned long long*>(h_pin + 2 * NAVG + holes.size());
-  EP2D_CK(cudaMemcpyAsync(hv, f.vmax, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
-  EP2D_CK(cudaStreamSynchronize(stream));
-  end_turn();
-  if (resident_launches && reinterpret_cast<unsigned*>(hv + 3)[0]) return failed_wait();
+  for (bool again = true; again;) {
+    EP2D_CK(cudaMemcpyAsync(hv, f.vmax, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
+    EP2D_CK(cudaStreamSynchronize(stream));
+    end_turn();
+    again = false;
+    const int rc = resident_launches ? look_at_waits(reinterpret_cast<unsigned*>(hv + 3), &again) : EP2D_OK;
+    if (rc) return rc;
+  }
   double vmx, vmy;
   std::memcpy(&vmx, &hv[0], sizeof(double));
   std::memcpy(&vmy, &hv[1], sizeof(double));
@@ -948,7 +997,7 @@ int Rve::solve_step(int step, double lsv, const double lt[3], int n_time_steps) 
     double error = 0.0;
     int64_t iter = 0, iters = prm.niter;
     int converged = 0;
-    bool flag_read = false;  // the last interval ended with a checkpoint, which read the error flag
+    bool flag_read = false;  // the last interval ended with a checkpoint, which looked at the waits
     EP2D_CK(cudaEventRecord(ev_[0], stream));
     while (iter < prm.niter) {
       const int64_t block_end = std::min<int64_t>(prm.niter, (iter / ce + 1) * ce);
@@ -958,13 +1007,8 @@ int Rve::solve_step(int step, double lsv, const double lt[3], int n_time_steps) 
         if (rc) return rc;
       }
       const bool in_f32 = f32;
-      rc = run_plain(block_end - iter - 1);
+      rc = launch_interval(block_end - iter - 1, true);
       if (rc) return rc;
-      rc = reset_vmax();
-      if (rc) return rc;
-      rc = launch_one(true);
-      if (rc) return rc;
-      launches++;
       if (in_f32) f32_iterations += block_end - iter;
       iter = block_end;
       flag_read = false;
@@ -998,13 +1042,13 @@ int Rve::solve_step(int step, double lsv, const double lt[3], int n_time_steps) 
       if (rc) return rc;
     }
     EP2D_CK(cudaEventRecord(ev_[1], stream));
+    if (!flag_read) rc = check_resident();
+    if (rc) return rc;
     EP2D_CK(cudaEventSynchronize(ev_[1]));
     float ms = 0.0f;
     EP2D_CK(cudaEventElapsedTime(&ms, ev_[0], ev_[1]));
     kernel_ms += ms;
     cell_updates += iters * (int64_t)prm.nx * prm.ny;
-    if (!flag_read) rc = check_resident();
-    if (rc) return rc;
     end_turn();
     r.iterations = iters;
     r.converged = converged;

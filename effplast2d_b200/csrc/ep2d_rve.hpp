@@ -107,14 +107,15 @@ class Rve {
   int begin_time_step(int step, int it, double load_step_value, const double load_type[3], int n_time_steps);
   int iterate(int64_t n, bool record_last);  // n iterations; the last one records stresses
   int launch_one(bool record);                // one iteration kernel (no stats)
+  int run_off_chip(int64_t n);                // n plain iterations in single launches, here and from now on
   int reset_vmax();
-  int check_resident();  // the error flag of the forms with bounded waits (sticky)
+  int check_resident();  // the words of the forms with bounded waits; runs an interval again that gave up
   int read_error(double* error);              // after a recording launch: D2H + error formula
   int finish_time_step(int step, int it);     // averaging etc. into the record
   double error_from_vmax(double vmx, double vmy) const;
   // this RVE as a job of an on-chip launch of n iterations; the caller flips `cur` by n & 1
   // when it has been made
-  ChipJob chip_job(unsigned* flag) const;
+  ChipJob chip_job(unsigned* state, unsigned count0) const;
 
   int get_field(int field, double* host) const;
   int set_field(int field, const double* host);
@@ -139,6 +140,7 @@ class Rve {
   // (the FP32 phase: chip_f32_fits)
   char* d_rim = nullptr;
   ChipWaits chip_waits;  // of the next on-chip launch
+  unsigned chip_count = 0;  // CTAs counted in the state word f.gbar[3]
   // velocities stored in FP32 (the mixed path, and both phases of the FP32 bulk)
   bool mixed() const { return prm.precision == EP2D_MIXED || prm.precision == EP2D_F32_BULK; }
   // FP32 bulk: true while the state is in its FP32 form (u' in f.ux32/uy32)
@@ -193,7 +195,16 @@ class Rve {
 
  private:
   int run_plain(int64_t n);
-  int run_chip(int64_t n, bool* done);
+  int run_chip(int64_t* n);
+  // n plain iterations, and a recording one behind them
+  int launch_interval(int64_t n, bool record);
+  struct Interval {
+    int64_t n;
+    bool record;
+    int cur;
+  };
+  Interval last_{};  // what the on-chip launch in flight and the launches behind it do, and from which buffer
+  int look_at_waits(const unsigned words[2], bool* again);
   bool chip_f32_fits() const;
   // this handle's turn for launches whose CTAs wait on one another (chip_turn): given back once the
   // stream has been waited for -- by end_turn at the latest when iterate or solve_step returns

@@ -44,7 +44,8 @@ struct Fields {
   // FP32 bulk only: the displacement perturbations u' = U - Ua (ping-pong), float
   float* ux32[2];
   float* uy32[2];
-  // resident form: the grid barrier {64-bit arrival count, error flag, unused}, 8-byte aligned
+  // resident form: the grid barrier {64-bit arrival count, error flag}, 8-byte aligned; behind it the
+  // on-chip form's state word
   unsigned* gbar;
 };
 
@@ -120,29 +121,42 @@ constexpr int CHIP_SMEM = 226 * 1024;
 // every CTA takes at least this much, of which no two fit an SM: a second CTA there would wait for the
 // first one's tensor memory, and the first for the second's rim
 constexpr int CHIP_SMEM_MIN = 116 * 1024;
-// How long a launch's CTAs wait for one another; `missing` of them, the last ones, are left out
-// (ep2d_check_chip_wait).
+// The state word of an RVE's on-chip launches: the number of CTAs that have started (it goes on from
+// launch to launch), and what ended a launch early.  Both are decided by atomics on this one word:
+// CHIP_GAVE_UP is only ever set while a CTA has not started, and a CTA that finds it set leaves at once.
+constexpr unsigned CHIP_GAVE_UP = 1u << 31;  // not all CTAs started: nobody has written the state, it is as before
+constexpr unsigned CHIP_STALLED = 1u << 30;  // a running CTA's records did not come: the state is invalid
+constexpr unsigned CHIP_FAILED = CHIP_GAVE_UP | CHIP_STALLED;
+constexpr unsigned CHIP_COUNT = CHIP_STALLED - 1;
+// How long a launch's CTAs wait for one another.  Work that holds an SM may hold it for good (a kernel of
+// the program's that waits for something), and the other forms run beside it: hence the shorter limit on
+// the start.  `missing`: the last CTAs that are left out (ep2d_check_chip_wait, ep2d_check_chip_start).
 struct ChipWaits {
-  unsigned long long records_ns = 10000000000ull;  // for a neighbour's rim records
+  unsigned long long start_ns = 2000000000ull;     // for a CTA that has not started: CHIP_GAVE_UP
+  unsigned long long records_ns = 10000000000ull;  // for the records of one that has: CHIP_STALLED
   int missing = 0;
+  bool missing_started = false;  // the missing CTAs count as started
 };
 constexpr int CHIP_MIN_RUN = 8;  // shorter runs of plain iterations are launched one by one
 ChipShape chip_shape(int nx, int ny);
 // One RVE of an on-chip launch: its fields, rim records (chip_rim_bytes; zeroed by the launch),
-// error flag, buffer holding U, tiles and first CTA.
+// state word and the count it holds before the launch, buffer holding U, tiles, first CTA, and the
+// count once all its CTAs have started.
 struct ChipJob {
   Geo g;
   Fields f;
   char* rim;
-  unsigned* flag;
+  unsigned* state;
+  unsigned count0;
   int src, plastic;
   int ncx, ncy, cta0;
+  unsigned full;
 };
 constexpr int CHIP_JOBS = 64;  // RVEs of one launch
 template <int JOBS>
 struct ChipArgs {
   int njobs, warps, rows, n_iter;
-  unsigned long long timeout_ns;
+  unsigned long long start_ns, records_ns;
   ChipJob job[JOBS];
 };
 // bytes of a grid's rim records at a given warps x rows, and the most any shape may need
@@ -153,8 +167,8 @@ size_t chip_rim_capacity(int nx, int ny);
 int chip_ctas(int nx, int ny, int groups, int warps, int rows);
 size_t chip_smem(int groups, int warps, int rows, bool track = false);
 // n_iter >= 2 plain iterations of the jobs' RVEs in one cooperative launch: CTAs of s.groups tiles of
-// s.warps x s.rows (s.ncx, s.ncy unused); fills in the jobs' tiles and CTAs.  A wait for records that
-// gives up sets the job's flag
+// s.warps x s.rows (s.ncx, s.ncy unused); fills in the jobs' tiles and CTAs.  A wait that gives up is
+// recorded in the job's state word
 // (track: also mark what yields, as launch_iter does; f32: the FP32 bulk's iterations, on
 // f.ux32/uy32; one job each)
 cudaError_t launch_iter_chip(ChipJob* jobs, int njobs, bool mixed, const ChipShape& s, int n_iter,

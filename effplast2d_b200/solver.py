@@ -26,6 +26,7 @@ EXPORTS = (
     "ep2d_server_stats", "ep2d_server_destroy", "ep2d_average_fields_noalloc", "ep2d_get_kernel_shape",
     "ep2d_compute_eff_damping", "ep2d_polar_fields", "ep2d_get_f32_iterations",
     "ep2d_iterate_f32", "ep2d_track_plastic_zone", "ep2d_check_grid_barrier", "ep2d_check_chip_wait",
+    "ep2d_check_chip_start", "ep2d_check_batch_start",
 )
 
 
@@ -82,6 +83,8 @@ def lib():
         L.ep2d_polar_fields.argtypes = [vp, d] + [P(d)] * 4 + [P(ctypes.c_uint8)]
         L.ep2d_check_grid_barrier.argtypes = [i32, i32, i32, i32, i64, P(i32), P(i32)]
         L.ep2d_check_chip_wait.argtypes = [vp, i32, i64]
+        L.ep2d_check_chip_start.argtypes = [vp, i32, i64]
+        L.ep2d_check_batch_start.argtypes = [P(_abi.BatchConfig), P(_abi.RveSpec), i32, i32, i64, P(_abi.Result), P(_abi.BatchStats)]
         _lib = L
     return _lib
 
@@ -182,6 +185,11 @@ class Solver:
         """the next on-chip launch leaves out its last `missing` CTAs and its waits give up
         after timeout_ns (ep2d_check_chip_wait)"""
         _check(lib().ep2d_check_chip_wait(self._h, int(missing), int(timeout_ns)))
+
+    def check_chip_start(self, missing, timeout_ns=2_000_000):
+        """the next on-chip launch's last `missing` CTAs never start; the others give up
+        after timeout_ns and the iterations run in single launches (ep2d_check_chip_start)"""
+        _check(lib().ep2d_check_chip_start(self._h, int(missing), int(timeout_ns)))
 
     def track_plastic_zone(self, on=True):
         """get_sigma_2D.m's plastic zone: mark every node / corner that yields at any

@@ -235,7 +235,7 @@ int ep2d_destroy(ep2d_handle* h);
 /* Return a handle to the state of a freshly constructed object (EffPlast2D.cu:1585-1604:
  * every field zero, no records) without reallocating.  The reference object keeps its
  * velocities across ComputeEffModuli calls; a new object starts from rest, as this does.
- * A handle whose kernel gave up a wait (EP2D_ERR_CUDA) is usable again after it. */
+ * A handle whose kernel gave up a wait for a running CTA (EP2D_ERR_CUDA) is usable again after it. */
 int ep2d_reset(ep2d_handle* h);
 
 /* Exactly n pseudo-time iterations of the reference's kernel sequence
@@ -425,12 +425,22 @@ int ep2d_get_kernel_shape(ep2d_handle* h, int32_t* kernel, int32_t* rows);
 int ep2d_check_grid_barrier(int32_t device, int32_t blocks, int32_t missing, int32_t rounds, int64_t timeout_ns,
                             int32_t* passed, int32_t* flag);
 /* For checking the failure path of the on-chip form without a fault: the handle's next
- * on-chip launch (one only) leaves out its last `missing` CTAs (one always runs), and its
- * waits for a neighbour's values give up after timeout_ns (at most 10 s).  The neighbours of
- * the missing CTAs then set the error flag, the others see it, the launch ends, and the
- * handle's next checkpoint (or the end of ep2d_iterate / the time step) returns
- * EP2D_ERR_CUDA.  No counterpart in the reference. */
+ * on-chip launch (one only) leaves out its last `missing` CTAs (one always runs) but counts
+ * them as started, and its waits for a neighbour's values give up after timeout_ns (at most
+ * 10 s), as if a running CTA's values never came.  The neighbours of the missing CTAs then
+ * record it, the others see it, the launch ends, and the handle's next checkpoint (or the
+ * end of ep2d_iterate / the time step) returns EP2D_ERR_CUDA.  No counterpart in the
+ * reference. */
 int ep2d_check_chip_wait(ep2d_handle* h, int32_t missing, int64_t timeout_ns);
+/* The same for CTAs that cannot start, as when other work holds their SMs: they are left
+ * out, not counted, and the others give up after timeout_ns (without this call 2 s).  They leave the state
+ * as it was, and the iterations run in single launches, then and from there on: the call
+ * succeeds with the same results.  No counterpart in the reference. */
+int ep2d_check_chip_start(ep2d_handle* h, int32_t missing, int64_t timeout_ns);
+/* ep2d_batch_solve whose first on-chip launch leaves out its last `missing` CTAs (the last
+ * RVE's, of which one always runs) in that way. */
+int ep2d_check_batch_start(const ep2d_batch_config* cfg, const ep2d_rve_spec* specs, int32_t n, int32_t missing,
+                           int64_t timeout_ns, ep2d_result* results, ep2d_batch_stats* stats);
 
 #ifdef __cplusplus
 }

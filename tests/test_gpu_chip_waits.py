@@ -7,8 +7,9 @@ import numpy as np
 import pytest
 
 import effplast2d_b200 as ep
+from effplast2d_b200 import batch as B
 from test_gpu_chip import _run
-from test_gpu_kernels import FIELDS, _pa, _random_state
+from test_gpu_kernels import FIELDS, PLASTIC_FIELDS, _pa, _random_state
 
 pytestmark = pytest.mark.gpu
 
@@ -69,3 +70,78 @@ def test_reset_after_a_failed_wait_gives_a_fresh_handle(precision):
         assert np.array_equal(s.get(f), t.get(f)), f
     s.close()
     t.close()
+
+
+# 2047 x 64 has 74 tiles beside one another: those far from the missing ones have gone through the 9
+# iterations of the first launch when it gives up
+@pytest.mark.parametrize("nx,ny", [(64, 64), (301, 203), (2047, 64), (1024, 1024)])
+@pytest.mark.parametrize("nl,precision", [(1, ep.FP64), (3, ep.FP64), (2, ep.MIXED)], ids=["elastic", "plastic", "mixed"])
+def test_launch_whose_ctas_cannot_all_start(nx, ny, nl, precision):
+    pa = _pa(nx, ny, n_pores=2, porosity=0.03, yield_stress=1e-5)
+    st = _random_state(nx, ny, 81)
+    out = []
+    for missing in (0, 1, 3):
+        s = ep.Solver(nx, ny, pa, nl=nl, precision=precision)
+        _set(s, st)
+        if missing:
+            s.check_chip_start(missing)
+        for n in (10, 33, 1):
+            s.iterate(n)
+        out.append({f: s.get(f) for f in FIELDS + PLASTIC_FIELDS})
+        if missing:  # the plain iterations after the first attempt were single launches
+            assert s.stats()["launches"] > 20
+        s.close()
+    for o in out[1:]:
+        for f in o:
+            assert np.array_equal(o[f], out[0][f]), f
+
+
+@pytest.mark.parametrize("precision", [ep.FP64, ep.MIXED, ep.F32_BULK], ids=["fp64", "mixed", "f32"])
+@pytest.mark.parametrize("niter", [120, 100], ids=["checkpoint-last", "no-checkpoint-last"])
+def test_solve_goes_on_when_ctas_cannot_start(precision, niter):
+    # with the plastic zone tracked; the interval that gives up is the first, with the recording
+    # launch behind it, or (second step of a handle) the FP32 phase's
+    nx, ny = 130, 96
+    out = []
+    for missing in (0, 2):
+        s, _ = _solver(nx, ny, niter=niter, check_every=40, precision=precision)
+        s.track_plastic_zone(True)
+        if missing:
+            s.check_chip_start(missing)
+        r = s.solve_step(0, -6e-5, [1.0, 0.8, 0.3], 2)
+        p = s.polar_fields(-6e-5)
+        out.append(([(q["iterations"], q["sigma"], q["error"]) for q in r], s.check_errors(0, 0), p,
+                    {f: s.get(f) for f in FIELDS}))
+        s.close()
+    assert out[0][0] == out[1][0] and out[0][1] == out[1][1]
+    for k in (2, 3):
+        for f in out[0][k]:
+            assert np.array_equal(out[0][k][f], out[1][k][f]), f
+
+
+@pytest.mark.parametrize("precision", [ep.FP64, ep.MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("missing", [1, 100])
+def test_batch_goes_on_when_ctas_cannot_start(precision, missing):
+    # of the RVEs of one launch some have their CTAs and some not
+    specs = []
+    for k, n in enumerate([512, 300, 310]):
+        pa = ep.make_pa(20.0, 20.0, n, n, yield_stress=1e-5, porosity=0.01, n_pores=1)
+        specs.append(B.spec(n, pa, 1 + k % 3, 1, -6e-5, (1.0, 0.8, 0.3)))
+    kw = dict(niter=160, check_every=80, precision=precision)
+    a, sa = B.batch_solve(specs, **kw)
+    b, sb = B.batch_solve(specs, check_start=(missing, 2_000_000), **kw)
+    assert sb["launches"] > sa["launches"] + 100
+    for x, y in zip(a, b):
+        assert x["total_iterations"] == y["total_iterations"]
+        for m in ("kphi", "kd", "g"):
+            u, v = x["num"][m], y["num"][m]
+            assert u == v or (np.isnan(u) and np.isnan(v)), (m, u, v)
+
+
+def test_check_start_arguments():
+    s, _ = _solver(16, 16)
+    for kw in (dict(missing=-1), dict(missing=1, timeout_ns=-1), dict(missing=1, timeout_ns=20_000_000_000)):
+        with pytest.raises(ep.EP2DError) as e:
+            s.check_chip_start(**kw)
+        assert e.value.status == ep.ERR_ARG
+    s.close()
