@@ -20,16 +20,19 @@ def footprint(s, precision=_abi.FP64):
 
 
 def batch_solve(specs, niter=100000, eiter=1e-9, check_every=10000, precision=_abi.FP64, device=0, rows=0,
-                graph_len=0, kernel=_abi.KERNEL_AUTO, check_start=None):
+                graph_len=0, kernel=_abi.KERNEL_AUTO, check_start=None, check_room=None):
     """Solve every spec together; returns (list of result dicts, stats dict).  rows = 0
     lets the library time the kernel forms and rows on the first launches.
-    check_start = (missing, timeout_ns): ep2d_check_batch_start."""
+    check_start = (missing, timeout_ns): ep2d_check_batch_start; check_room = launches:
+    ep2d_check_batch_room."""
     cfg = _abi.make_batch_config(niter, eiter, check_every, precision, device, rows, graph_len, kernel)
     n = len(specs)
     arr = (_abi.RveSpec * n)(*specs)
     res = (_abi.Result * n)()
     st = _abi.BatchStats()
-    if check_start is None:
+    if check_room is not None:
+        _check(lib().ep2d_check_batch_room(ctypes.byref(cfg), arr, n, int(check_room), res, ctypes.byref(st)))
+    elif check_start is None:
         _check(lib().ep2d_batch_solve(ctypes.byref(cfg), arr, n, res, ctypes.byref(st)))
     else:
         _check(lib().ep2d_check_batch_start(ctypes.byref(cfg), arr, n, int(check_start[0]), int(check_start[1]), res,

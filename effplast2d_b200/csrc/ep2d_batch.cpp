@@ -427,19 +427,27 @@ bool BatchEngine::plan_waves(const std::vector<char>& batched) {
 int BatchEngine::run_waves(int64_t n, bool* done) {
   std::lock_guard<std::mutex> turn(chip_turn(device));
   std::vector<ChipJob> jobs;
+  std::vector<int> left;  // slots the chunk's launches have not advanced
   *done = false;
   while (n > 0) {  // chunks of an even length keep the parity
     const int64_t chunk = n > ((int64_t)1 << 30) ? (int64_t)1 << 29 : n;
+    left.clear();
     EP2D_CK(cudaMemsetAsync(d_state_, 0, slots_.size() * sizeof(unsigned), stream));
     for (const Wave& w : waves_) {
       jobs.clear();
       for (int q : w.slots) jobs.push_back(slots_[q].rve->chip_job(d_state_ + q, 0));
-      const cudaError_t e = launch_iter_chip(jobs.data(), (int)jobs.size(), cfg.precision == EP2D_MIXED, w.shape,
-                                             (int)chunk, std::exchange(chip_waits, ChipWaits{}), stream);
-      if (e == cudaErrorCooperativeLaunchTooLarge && !*done) {  // no room for the CTAs here
+      cudaError_t e = cudaErrorCooperativeLaunchTooLarge;
+      if (waves_ok_ && chip_room != 0) {
+        if (chip_room > 0) chip_room--;
+        e = launch_iter_chip(jobs.data(), (int)jobs.size(), cfg.precision == EP2D_MIXED, w.shape, (int)chunk,
+                             std::exchange(chip_waits, ChipWaits{}), stream);
+      }
+      if (e == cudaErrorCooperativeLaunchTooLarge) {  // no room for the CTAs here
         cudaGetLastError();
         waves_ok_ = use_waves_ = false;
-        return EP2D_OK;
+        if (!*done) return EP2D_OK;
+        left.insert(left.end(), w.slots.begin(), w.slots.end());
+        continue;
       }
       EP2D_CK(e);
       *done = true;
@@ -455,10 +463,13 @@ int BatchEngine::run_waves(int64_t n, bool* done) {
         if (h_state_[q] & CHIP_GAVE_UP) {
           waves_ok_ = use_waves_ = false;
           slots_[q].rve->cur ^= (int)(chunk & 1);
-          const int rc = run_off_chip(q, chunk);
-          if (rc) return rc;
+          left.push_back(q);
         }
       }
+    for (int q : left) {
+      const int rc = run_off_chip(q, chunk);
+      if (rc) return rc;
+    }
     n -= chunk;
   }
   return EP2D_OK;
@@ -872,7 +883,7 @@ struct ep2d_server {
 };
 
 static int batch_solve(const ep2d_batch_config* cfg, const ep2d_rve_spec* specs, int32_t n, ep2d_result* results,
-                       ep2d_batch_stats* stats, const ep2d::ChipWaits& waits) {
+                       ep2d_batch_stats* stats, const ep2d::ChipWaits& waits, int chip_room) {
   if (!cfg || (!specs && n > 0) || n < 0) return fail(EP2D_ERR_ARG, "null argument");
   try {
     const double t0 = ep2d::now_s();
@@ -880,6 +891,7 @@ static int batch_solve(const ep2d_batch_config* cfg, const ep2d_rve_spec* specs,
     int rc = eng.init(*cfg);
     if (rc) return rc;
     eng.chip_waits = waits;
+    eng.chip_room = chip_room;
     size_t need = 0;
     for (int k = 0; k < n; k++) {
       rc = ep2d::validate_params(ep2d::params_of(*cfg, specs[k]));
@@ -937,7 +949,7 @@ int64_t ep2d_rve_footprint(const ep2d_rve_spec* spec, int32_t precision) {
 
 int ep2d_batch_solve(const ep2d_batch_config* cfg, const ep2d_rve_spec* specs, int32_t n, ep2d_result* results,
                      ep2d_batch_stats* stats) {
-  return batch_solve(cfg, specs, n, results, stats, ep2d::ChipWaits{});
+  return batch_solve(cfg, specs, n, results, stats, ep2d::ChipWaits{}, -1);
 }
 
 int ep2d_check_batch_start(const ep2d_batch_config* cfg, const ep2d_rve_spec* specs, int32_t n, int32_t missing,
@@ -947,7 +959,13 @@ int ep2d_check_batch_start(const ep2d_batch_config* cfg, const ep2d_rve_spec* sp
   ep2d::ChipWaits w;
   w.missing = missing;
   w.start_ns = (unsigned long long)timeout_ns;
-  return batch_solve(cfg, specs, n, results, stats, w);
+  return batch_solve(cfg, specs, n, results, stats, w, -1);
+}
+
+int ep2d_check_batch_room(const ep2d_batch_config* cfg, const ep2d_rve_spec* specs, int32_t n, int32_t launches,
+                          ep2d_result* results, ep2d_batch_stats* stats) {
+  if (launches < 0) return fail(EP2D_ERR_ARG, "need launches >= 0");
+  return batch_solve(cfg, specs, n, results, stats, ep2d::ChipWaits{}, launches);
 }
 
 int ep2d_server_create(const ep2d_batch_config* cfg, int64_t mem_budget_bytes, int32_t max_active, ep2d_server** out) {

@@ -69,6 +69,7 @@ class BatchEngine {
   double tune_us[7] = {0, 0, 0, 0, 0, 0, 0};  // tile rows 8/16/32, stream rows 8/16/32/64
   void fill_stats(ep2d_batch_stats* st) const;
   ChipWaits chip_waits;  // of the next on-chip launch (ep2d_check_batch_start)
+  int chip_room = -1;    // on-chip launches the device has room for (ep2d_check_batch_room); -1: no such limit
 
  private:
   struct Slot {

@@ -26,7 +26,7 @@ EXPORTS = (
     "ep2d_server_stats", "ep2d_server_destroy", "ep2d_average_fields_noalloc", "ep2d_get_kernel_shape",
     "ep2d_compute_eff_damping", "ep2d_polar_fields", "ep2d_get_f32_iterations",
     "ep2d_iterate_f32", "ep2d_track_plastic_zone", "ep2d_check_grid_barrier", "ep2d_check_chip_wait",
-    "ep2d_check_chip_start", "ep2d_check_batch_start",
+    "ep2d_check_chip_start", "ep2d_check_batch_start", "ep2d_check_batch_room",
 )
 
 
@@ -85,6 +85,7 @@ def lib():
         L.ep2d_check_chip_wait.argtypes = [vp, i32, i64]
         L.ep2d_check_chip_start.argtypes = [vp, i32, i64]
         L.ep2d_check_batch_start.argtypes = [P(_abi.BatchConfig), P(_abi.RveSpec), i32, i32, i64, P(_abi.Result), P(_abi.BatchStats)]
+        L.ep2d_check_batch_room.argtypes = [P(_abi.BatchConfig), P(_abi.RveSpec), i32, i32, P(_abi.Result), P(_abi.BatchStats)]
         _lib = L
     return _lib
 

@@ -441,6 +441,10 @@ int ep2d_check_chip_start(ep2d_handle* h, int32_t missing, int64_t timeout_ns);
  * RVE's, of which one always runs) in that way. */
 int ep2d_check_batch_start(const ep2d_batch_config* cfg, const ep2d_rve_spec* specs, int32_t n, int32_t missing,
                            int64_t timeout_ns, ep2d_result* results, ep2d_batch_stats* stats);
+/* ep2d_batch_solve on a device that refuses on-chip launches after `launches` of them, as one
+ * without room for their CTAs does: the remaining iterations take the other forms. */
+int ep2d_check_batch_room(const ep2d_batch_config* cfg, const ep2d_rve_spec* specs, int32_t n, int32_t launches,
+                          ep2d_result* results, ep2d_batch_stats* stats);
 
 #ifdef __cplusplus
 }

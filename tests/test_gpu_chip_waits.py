@@ -145,3 +145,21 @@ def test_check_start_arguments():
             s.check_chip_start(**kw)
         assert e.value.status == ep.ERR_ARG
     s.close()
+
+
+@pytest.mark.parametrize("room", [0, 1, 2])
+def test_batch_goes_on_when_the_device_refuses_a_wave(room):
+    # the two waves of the first interval and the one of the second: each refused in turn
+    specs = []
+    for k, n in enumerate([700, 640, 512, 300, 33]):
+        pa = ep.make_pa(20.0, 20.0, n, n, yield_stress=1e-5, porosity=0.01, n_pores=1)
+        specs.append(B.spec(n, pa, 1 + k % 2, 1, -6e-5, (1.0, 0.8, 0.3)))
+    kw = dict(niter=161, check_every=161)
+    a, sa = B.batch_solve(specs, **kw)
+    b, sb = B.batch_solve(specs, check_room=room, **kw)
+    assert sa["launches"] < 20 and sb["launches"] > sa["launches"] + 100
+    for x, y in zip(a, b):
+        assert x["total_iterations"] == y["total_iterations"]
+        for m in ("kphi", "kd", "g"):
+            u, v = x["num"][m], y["num"][m]
+            assert u == v or (np.isnan(u) and np.isnan(v)), (m, u, v)
