@@ -351,6 +351,29 @@ int BatchEngine::autotune(int64_t* k, int64_t n_avail) {
   return rebuild_tiles();
 }
 
+// The fewest rows per warp, and then the fewest warps, with which a wave's RVEs fit on `sms` SMs.
+bool BatchEngine::wave_shape(Wave* w, int tall, int sms) const {
+  int cost = 1 << 30;
+  for (int rows = 2; rows <= tall && cost == 1 << 30; rows += 2)
+    for (int g = 1; g <= 4; g++)
+      for (int nw = 4; g * nw <= CHIP_WARPS; nw++) {
+        ChipShape s;
+        s.groups = g;
+        s.warps = nw;
+        s.rows = rows;
+        const int c = g * nw + (g == 1 ? 1 : 0);
+        if (wave_ctas(*w, s) > sms || chip_smem(g, nw, rows) > CHIP_SMEM || c > cost) continue;
+        cost = c;
+        w->shape = s;
+      }
+  return cost != 1 << 30;
+}
+int BatchEngine::wave_ctas(const Wave& w, const ChipShape& s) const {
+  int n = 0;
+  for (int q : w.slots) n += chip_ctas(slots_[q].rve->g.nx, slots_[q].rve->g.ny, s.groups, s.warps, s.rows);
+  return n;
+}
+
 // Split the batched RVEs into waves, each one on-chip launch of all the interval's plain
 // iterations of its RVEs side by side.  An iteration of a wave takes about 1.95 + 0.485 R us
 // for R rows per warp (measured, FP64 with the return map: R = 2 2.9, 8 5.8, 16 9.8 us), so few
@@ -396,20 +419,7 @@ bool BatchEngine::plan_waves(const std::vector<char>& batched) {
     }
     double us = 0.0;
     for (Wave& w : ws) {
-      int cost = 1 << 30;
-      for (int rows = 2; rows <= tall && cost == 1 << 30; rows += 2)
-        for (int g = 1; g <= 4; g++)
-          for (int nw = 4; g * nw <= CHIP_WARPS; nw++) {
-            int sum = 0;
-            for (int q : w.slots) sum += ctas(q, g, nw, rows);
-            const int c = g * nw + (g == 1 ? 1 : 0);
-            if (sum > CHIP_SMS || chip_smem(g, nw, rows) > CHIP_SMEM || c > cost) continue;
-            cost = c;
-            w.shape.groups = g;
-            w.shape.warps = nw;
-            w.shape.rows = rows;
-          }
-      if (cost == 1 << 30) {
+      if (!wave_shape(&w, tall, CHIP_SMS)) {
         us = 1e30;
         break;
       }
@@ -425,7 +435,28 @@ bool BatchEngine::plan_waves(const std::vector<char>& batched) {
 }
 
 int BatchEngine::run_waves(int64_t n, bool* done) {
-  std::lock_guard<std::mutex> turn(chip_turn(device));
+  // Alone on the device the waves go one behind another without a wait.  Beside other calls each takes
+  // its RVEs' part of the SMs, if they fit there, and gives them back when it has completed.
+  int n_rves = 0;
+  for (const Wave& w : waves_) n_rves += (int)w.slots.size();
+  SmShare& share = SmShare::of(device);
+  const SmShare::Call call(share, n_rves);
+  const bool alone = share.rves() <= n_rves;
+  struct Held {
+    SmShare& s;
+    cudaStream_t stream;
+    int sms = 0;
+    void give() {
+      s.give(sms);
+      sms = 0;
+    }
+    ~Held() {
+      if (sms) cudaStreamSynchronize(stream);
+      give();
+    }
+  } held{share, stream};
+  int most = 0;
+  for (const Wave& w : waves_) most = std::max(most, wave_ctas(w, w.shape));
   std::vector<ChipJob> jobs;
   std::vector<int> left;  // slots the chunk's launches have not advanced
   *done = false;
@@ -437,9 +468,17 @@ int BatchEngine::run_waves(int64_t n, bool* done) {
       jobs.clear();
       for (int q : w.slots) jobs.push_back(slots_[q].rve->chip_job(d_state_ + q, 0));
       cudaError_t e = cudaErrorCooperativeLaunchTooLarge;
+      ChipShape fit = w.shape;
       if (waves_ok_ && chip_room != 0) {
         if (chip_room > 0) chip_room--;
-        e = launch_iter_chip(jobs.data(), (int)jobs.size(), cfg.precision == EP2D_MIXED, w.shape, (int)chunk,
+        if (!held.sms)
+          held.sms = share.take([&](int rves, int) {
+            if (alone) return most;
+            Wave part = w;
+            if (wave_shape(&part, 18, (int)((int64_t)CHIP_SMS * n_rves / std::max(rves, n_rves)))) fit = part.shape;
+            return wave_ctas(w, fit);
+          });
+        e = launch_iter_chip(jobs.data(), (int)jobs.size(), cfg.precision == EP2D_MIXED, fit, (int)chunk,
                              std::exchange(chip_waits, ChipWaits{}), stream);
       }
       if (e == cudaErrorCooperativeLaunchTooLarge) {  // no room for the CTAs here
@@ -453,6 +492,10 @@ int BatchEngine::run_waves(int64_t n, bool* done) {
       *done = true;
       launches++;
       for (int q : w.slots) slots_[q].rve->cur ^= (int)(chunk & 1);
+      if (!alone) {
+        EP2D_CK(cudaStreamSynchronize(stream));
+        held.give();
+      }
     }
     EP2D_CK(cudaMemcpyAsync(h_state_, d_state_, slots_.size() * sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
     EP2D_CK(cudaStreamSynchronize(stream));
@@ -466,6 +509,7 @@ int BatchEngine::run_waves(int64_t n, bool* done) {
           left.push_back(q);
         }
       }
+    if (!left.empty()) held.give();
     for (int q : left) {
       const int rc = run_off_chip(q, chunk);
       if (rc) return rc;

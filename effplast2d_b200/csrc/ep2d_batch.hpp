@@ -92,6 +92,8 @@ class BatchEngine {
     std::vector<int> slots;
     ChipShape shape;
   };
+  bool wave_shape(Wave* w, int tall, int sms) const;
+  int wave_ctas(const Wave& w, const ChipShape& s) const;
   bool plan_waves(const std::vector<char>& batched);  // false: the batched launches are faster
   int run_waves(int64_t n, bool* done);               // n plain iterations of every RVE of the waves
   int run_off_chip(int slot, int64_t n);              // ... of one RVE that an on-chip launch has left as it was

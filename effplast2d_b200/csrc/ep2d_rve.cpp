@@ -351,9 +351,38 @@ std::mutex g_prep_mu;
 std::set<int> g_prepared;
 }  // namespace
 
-std::mutex& chip_turn(int dev) {
-  static std::mutex mu[64];
-  return mu[dev & 63];
+SmShare& SmShare::of(int dev) {
+  static SmShare s[64];
+  return s[dev & 63];
+}
+SmShare::Call::Call(SmShare& share, int n) : s(share), rves(n) {
+  std::lock_guard<std::mutex> lk(s.mu_);
+  s.rves_ += rves;
+}
+SmShare::Call::~Call() {
+  std::lock_guard<std::mutex> lk(s.mu_);
+  s.rves_ -= rves;
+}
+int SmShare::take(const std::function<int(int, int)>& need) {
+  std::unique_lock<std::mutex> lk(mu_);
+  const uint64_t me = next_++;
+  cv_.wait(lk, [&] { return serving_ == me; });
+  const int n = std::min(need(rves_, free_), CHIP_SMS);
+  cv_.wait(lk, [&] { return free_ >= n; });
+  free_ -= n;
+  serving_++;
+  cv_.notify_all();
+  return n;
+}
+void SmShare::give(int sms) {
+  if (!sms) return;
+  std::lock_guard<std::mutex> lk(mu_);
+  free_ += sms;
+  cv_.notify_all();
+}
+int SmShare::rves() {
+  std::lock_guard<std::mutex> lk(mu_);
+  return rves_;
 }
 
 int prepare_device(int dev) {
@@ -681,8 +710,7 @@ ChipJob Rve::chip_job(unsigned* state, unsigned count0) const {
 // *n plain iterations in one launch of the on-chip form; *n: those left, where the device has no
 // room for its CTAs (the other forms take over for good).
 int Rve::run_chip(int64_t* n) {
-  take_turn();
-  const ChipShape s = chip;
+  const ChipShape s = take_sms();
   bool launched = false;
   while (*n > 0 && chip.warps) {
     // chunks of an even length keep the parity; a chunk of one iteration cannot arise
@@ -720,36 +748,58 @@ int Rve::run_chip(int64_t* n) {
   return EP2D_OK;
 }
 
-void Rve::take_turn() {
-  if (!turn_.owns_lock()) turn_ = std::unique_lock<std::mutex>(chip_turn(device));
+ChipShape Rve::take_sms() {
+  give_sms();
+  ChipShape s = chip;
+  sms_ = SmShare::of(device).take([&](int rves, int free) {
+    if (rves > 1) {
+      ChipShape t = chip_shape_beside(prm.nx, prm.ny, rves, CHIP_SMS);
+      // rather than wait, the SMs that are left (a 64^2 handle beside a batch on 138 of them: 8.6 -> 6.3 us
+      // an iteration, a 128^2 one 7.9 -> 4.6)
+      if (chip_ctas(prm.nx, prm.ny, t.groups, t.warps, t.rows) > free) {
+        const ChipShape left = chip_shape_beside(prm.nx, prm.ny, rves, free);
+        if (left.warps) t = left;
+      }
+      if (chip_usable(t)) s = t;
+    }
+    return chip_ctas(prm.nx, prm.ny, s.groups, s.warps, s.rows);
+  });
+  return s;
 }
-// the stream is idle: another handle may have the turn
-void Rve::end_turn() {
-  if (turn_.owns_lock()) turn_.unlock();
+void Rve::take_all_sms() {
+  give_sms();
+  sms_ = SmShare::of(device).take([](int, int) { return CHIP_SMS; });
 }
-Rve::TurnScope::~TurnScope() {
-  if (!r.turn_.owns_lock()) return;
+// the stream is idle: other handles may have them
+void Rve::give_sms() {
+  SmShare::of(device).give(sms_);
+  sms_ = 0;
+}
+Rve::SmScope::SmScope(Rve& rve)
+    : r(rve), call(SmShare::of(rve.device), rve.chip.warps || rve.shape.form == FORM_RESIDENT ? 1 : 0) {}
+Rve::SmScope::~SmScope() {
+  if (!r.sms_) return;
   cudaStreamSynchronize(r.stream);  // an error shows again at the next call
-  r.turn_.unlock();
+  r.give_sms();
 }
 
 // The FP32 phase keeps its rim records in the FP64 displacements (four contiguous arrays), which are
-// written anew when it ends; grids of a few tiles with hardly a column or row in the last one need more
-bool Rve::chip_f32_fits() const {
-  return chip_rim_bytes(prm.nx, prm.ny, chip.warps, chip.rows, true) <=
-         4 * align256(field_elems(prm) * sizeof(double));
+// written anew when it ends; grids of a few tiles with hardly a column or row in the last one need more.
+// Tracking takes a byte more of shared memory per cell.
+bool Rve::chip_usable(const ChipShape& s) const {
+  if (f32) return chip_rim_bytes(prm.nx, prm.ny, s.warps, s.rows, true) <= 4 * align256(field_elems(prm) * sizeof(double));
+  return !track || chip_smem(s.groups, s.warps, s.rows, true) <= CHIP_SMEM;
 }
 
 int Rve::run_plain(int64_t n) {
-  if (chip.warps && n >= CHIP_MIN_RUN &&
-      (f32 ? chip_f32_fits() : !track || chip_smem(chip.groups, chip.warps, chip.rows, true) <= CHIP_SMEM)) {
+  if (chip.warps && n >= CHIP_MIN_RUN && chip_usable(chip)) {
     const int rc = run_chip(&n);
     if (rc || n == 0) return rc;
   }
   if (shape.form == FORM_RESIDENT && !f32 && !track) {
     // one cooperative launch for all n iterations (n == 1: an ordinary tile launch)
     if (n > 1) {
-      take_turn();
+      take_all_sms();
       EP2D_CK(launch_iter_resident(g, f, cur, prm.nl > 1, mixed(), shape.rows, n, RESIDENT_TIMEOUT_NS, stream));
       cur ^= (int)(n & 1);
       launches++;
@@ -810,7 +860,7 @@ int Rve::launch_interval(int64_t n, bool record) {
 int Rve::iterate(int64_t n, bool record_last) {
   if (n <= 0) return EP2D_OK;
   DeviceScope ds(device);
-  TurnScope ts{*this};
+  SmScope ss(*this);
   EP2D_CK(cudaEventRecord(ev_[0], stream));
   int rc = launch_interval(record_last ? n - 1 : n, record_last);
   if (rc) return rc;
@@ -818,7 +868,7 @@ int Rve::iterate(int64_t n, bool record_last) {
   rc = check_resident();  // waits for the stream, if it has words to read
   if (rc) return rc;
   EP2D_CK(cudaEventSynchronize(ev_[1]));
-  end_turn();
+  give_sms();
   float ms = 0.0f;
   EP2D_CK(cudaEventElapsedTime(&ms, ev_[0], ev_[1]));
   kernel_ms += ms;
@@ -871,7 +921,7 @@ int Rve::read_error(double* error) {
   for (bool again = true; again;) {
     EP2D_CK(cudaMemcpyAsync(hv, f.vmax, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
     EP2D_CK(cudaStreamSynchronize(stream));
-    end_turn();
+    give_sms();
     again = false;
     const int rc = resident_launches ? look_at_waits(reinterpret_cast<unsigned*>(hv + 3), &again) : EP2D_OK;
     if (rc) return rc;
@@ -979,7 +1029,7 @@ void Rve::finish_chain(int n_time_steps, ep2d_result* out) {
 int Rve::solve_step(int step, double lsv, const double lt[3], int n_time_steps) {
   if (!lt) return fail(EP2D_ERR_ARG, "load_type is null");
   DeviceScope ds(device);
-  TurnScope ts{*this};
+  SmScope ss(*this);
   int rc0 = begin_step(step, n_time_steps);
   if (rc0) return rc0;
   const int64_t ce = prm.check_every;
@@ -1049,7 +1099,7 @@ int Rve::solve_step(int step, double lsv, const double lt[3], int n_time_steps) 
     EP2D_CK(cudaEventElapsedTime(&ms, ev_[0], ev_[1]));
     kernel_ms += ms;
     cell_updates += iters * (int64_t)prm.nx * prm.ny;
-    end_turn();
+    give_sms();
     r.iterations = iters;
     r.converged = converged;
     r.error = error;

@@ -2,7 +2,9 @@
 // its records.  Shared by the single-RVE C ABI, the batched solver and the server.
 #pragma once
 
+#include <condition_variable>
 #include <cstdint>
+#include <functional>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -63,10 +65,33 @@ IterShape shape_of(const ep2d_params& p, int sm_count = 0);
 // Device row pitch (elements) for an nx-wide grid.
 int row_pitch(int nx);
 
-// On-chip and resident-form launches of different handles take turns on a device: their CTAs wait on
-// one another, so two such grids that each found room for only part of their CTAs would wait for
-// each other until their waits ran out.  Held from the launch to its completion.
-std::mutex& chip_turn(int dev);
+// How the on-chip and resident-form launches of different handles share a device's SMs.  The CTAs of
+// such a launch wait on one another, so two grids that each found room for only part of their CTAs
+// would wait for each other until their waits ran out.  A launch therefore takes its SMs (one per CTA:
+// no two fit one) beforehand, in the order in which the handles ask, and gives them back when it has
+// completed.  Where several RVEs are on the device a launch takes a shape that lets them run side by side
+// (chip_shape_beside; a batch gives up SMs for the handles beside it).
+class SmShare {
+ public:
+  static SmShare& of(int dev);
+  // a call that makes such launches of `rves` RVEs, from its beginning to its end
+  struct Call {
+    SmShare& s;
+    const int rves;
+    Call(SmShare& share, int rves);
+    ~Call();
+  };
+  // wait for need(RVEs of all calls in progress, SMs free now) SMs
+  int take(const std::function<int(int, int)>& need);
+  void give(int sms);
+  int rves();  // of all calls in progress
+
+ private:
+  std::mutex mu_;
+  std::condition_variable cv_;
+  uint64_t next_ = 0, serving_ = 0;
+  int free_ = CHIP_SMS, rves_ = 0;
+};
 
 // Per-device kernel attributes, once per device (the device must be current).
 int prepare_device(int dev);
@@ -205,15 +230,18 @@ class Rve {
   };
   Interval last_{};  // what the on-chip launch in flight and the launches behind it do, and from which buffer
   int look_at_waits(const unsigned words[2], bool* again);
-  bool chip_f32_fits() const;
-  // this handle's turn for launches whose CTAs wait on one another (chip_turn): given back once the
-  // stream has been waited for -- by end_turn at the latest when iterate or solve_step returns
-  std::unique_lock<std::mutex> turn_;
-  void take_turn();
-  void end_turn();
-  struct TurnScope {
+  bool chip_usable(const ChipShape& s) const;
+  // the SMs of this handle's launches whose CTAs wait on one another (SmShare): given back once the
+  // stream has been waited for -- by give_sms, at the latest when iterate or solve_step returns
+  int sms_ = 0;
+  ChipShape take_sms();  // for an on-chip launch, and the shape it takes
+  void take_all_sms();   // for a resident-form launch
+  void give_sms();
+  struct SmScope {
     Rve& r;
-    ~TurnScope();
+    SmShare::Call call;
+    explicit SmScope(Rve& rve);
+    ~SmScope();
   };
   bool vmax_zero_ = false;  // an on-chip launch has just zeroed the max|V| pair
   int capture(int parity);

@@ -139,6 +139,7 @@ struct ChipWaits {
 };
 constexpr int CHIP_MIN_RUN = 8;  // shorter runs of plain iterations are launched one by one
 ChipShape chip_shape(int nx, int ny);
+ChipShape chip_shape_beside(int nx, int ny, int rves, int sms);  // with `rves` such grids on `sms` SMs
 // One RVE of an on-chip launch: its fields, rim records (chip_rim_bytes; zeroed by the launch),
 // state word and the count it holds before the launch, buffer holding U, tiles, first CTA, and the
 // count once all its CTAs have started.

@@ -66,7 +66,8 @@ enum {
                              elastic ones; batches: timed).  A single RVE whose grid fits
                              on chip (up to about 1080^2) runs the plain iterations between
                              two recording launches in one cooperative launch with its
-                             state held on the SMs; handles take turns for such launches */
+                             state held on the SMs; calls on several handles share the SMs
+                             of a device for such launches */
   EP2D_KERNEL_TILE = 1,   /* one CTA per 32-column x `rows`-row tile, stencil halos in
                              shared memory; rows 8, 16 or 32 */
   EP2D_KERNEL_STREAM = 2, /* one warp per 28-column strip segment of `rows` rows, marching

@@ -3,6 +3,9 @@
 Nothing here faults: CTAs are left out of a launch, the others' waits run out after a few
 milliseconds, the launch ends, and the context stays usable.
 """
+import threading
+import time
+
 import numpy as np
 import pytest
 
@@ -163,3 +166,79 @@ def test_batch_goes_on_when_the_device_refuses_a_wave(room):
         for m in ("kphi", "kd", "g"):
             u, v = x["num"][m], y["num"][m]
             assert u == v or (np.isnan(u) and np.isnan(v)), (m, u, v)
+
+
+def _in_threads(work, args):
+    bar = threading.Barrier(len(args) + 1)
+
+    def run(a):
+        bar.wait()
+        work(*a)
+
+    ths = [threading.Thread(target=run, args=(a,)) for a in args]
+    for t in ths:
+        t.start()
+    bar.wait()
+    t0 = time.perf_counter()
+    for t in ths:
+        t.join()
+    return time.perf_counter() - t0
+
+
+def test_small_handles_run_side_by_side():
+    # eight 128^2 handles in eight threads: one after another they would take eight times one
+    # handle's time (a quarter of that was measured with shares of the SMs)
+    n = 128
+    hs = [_solver(n, n, nl=3, niter=8000, eiter=0.0, check_every=2000)[0] for _ in range(8)]
+
+    def solve(h):
+        h.solve_step(0, -6e-5, [1.0, 0.8, 0.3])
+
+    for h in hs:
+        solve(h)
+    one = min(_in_threads(solve, [(hs[0],)]) for _ in range(3))
+    all_ = min(_in_threads(solve, [(h,) for h in hs]) for _ in range(3))
+    assert all_ < 0.7 * 8 * one, (all_, one)
+    for h in hs:
+        h.close()
+
+
+def test_handles_of_all_kinds_side_by_side():
+    # shapes for any share of the SMs, beside a batch: each result as alone
+    kinds = [(48, 64, dict(nl=1)), (64, 64, dict(nl=3)), (128, 130, dict(nl=3)), (200, 90, dict(nl=2, precision=ep.MIXED)),
+             (301, 203, dict(nl=2, track=True)), (256, 256, dict(nl=2, precision=ep.F32_BULK)), (512, 500, dict(nl=3)),
+             (640, 640, dict(nl=1)), (1024, 1024, dict(nl=2)), (128, 128, dict(nl=1, kernel=ep.KERNEL_RESIDENT, rows=8))]
+    specs = [B.spec(n, ep.make_pa(20.0, 20.0, n, n, yield_stress=1e-5, porosity=0.01, n_pores=1), 2, 1, -6e-5, (1.0, 0.8, 0.3))
+             for n in (700, 640, 512, 300, 64)]
+
+    def handle(nx, ny, kw):
+        kw = dict(kw)
+        track = kw.pop("track", False)
+        s, _ = _solver(nx, ny, niter=1600, eiter=0.0, check_every=200, **kw)
+        if track:
+            s.track_plastic_zone(True)
+        r = s.solve_step(0, -6e-5, [1.0, 0.8, 0.3])[0]
+        out = {f: s.get(f) for f in FIELDS}
+        if track:
+            out.update(s.polar_fields(-6e-5))
+        s.close()
+        return r["sigma"], out
+
+    def batch():
+        return [[r["num"][m] for m in ("kphi", "kd", "g")] for r in B.batch_solve(specs, niter=800, check_every=400, eiter=0.0)[0]]
+
+    want, want_b = [handle(*k) for k in kinds], batch()
+    got, got_b = [None] * len(kinds), [None]
+
+    def work(k):
+        if k < len(kinds):
+            got[k] = handle(*kinds[k])
+        else:
+            got_b[0] = batch()
+
+    _in_threads(work, [(k,) for k in range(len(kinds) + 1)])
+    assert np.array_equal(np.array(got_b[0]), np.array(want_b), equal_nan=True)
+    for k, (sigma, fields) in enumerate(want):
+        assert got[k][0] == sigma, kinds[k]
+        for f in fields:
+            assert np.array_equal(got[k][1][f], fields[f]), (kinds[k], f)
