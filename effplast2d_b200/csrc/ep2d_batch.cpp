@@ -501,7 +501,7 @@ int BatchEngine::run_waves(int64_t n, bool* done) {
     EP2D_CK(cudaStreamSynchronize(stream));
     for (const Wave& w : waves_)
       for (int q : w.slots) {
-        if (h_state_[q] & CHIP_STALLED)
+        if ((h_state_[q] & CHIP_FAILED) == CHIP_STALLED)
           return fail(EP2D_ERR_CUDA, "on-chip form: a wait for another CTA ran out; the batch's state is invalid");
         if (h_state_[q] & CHIP_GAVE_UP) {
           waves_ok_ = use_waves_ = false;

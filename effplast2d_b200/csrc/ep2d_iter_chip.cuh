@@ -76,17 +76,6 @@ __device__ __forceinline__ bool group_barrier_or(int id, int threads, int flag) 
   return r != 0;
 }
 
-// Waited longer than start_ns (long_wait: than records_ns) for another CTA of the job.
-__device__ __forceinline__ void chip_give_up(const ChipJob& job, bool long_wait) {
-  unsigned w = *reinterpret_cast<volatile unsigned*>(job.state);
-  while (!(w & CHIP_FAILED)) {
-    const bool all = (w & CHIP_COUNT) == job.full;
-    if (all && !long_wait) return;
-    const unsigned old = atomicCAS(job.state, w, w | (all ? CHIP_STALLED : CHIP_GAVE_UP));
-    if (old == w) return;
-    w = old;
-  }
-}
 // The time a wait has taken in ns, looked at now and then: time between two looks counts as at most
 // 10 ms, so that time in which the GPU runs another context does not.
 struct ChipClock {
@@ -98,14 +87,34 @@ struct ChipClock {
     return (unsigned long long)waited << 10;
   }
 };
-// Waits until all CTAs of the job have started; false if the launch has given up.  Called by whole warps.
+// A look at the job's state word by a warp that has waited this long: gives up where its limit has passed
+// (the mark shows at the next look); true if the launch has failed.
+__device__ __forceinline__ bool chip_look(const ChipJob& job, unsigned long long waited, unsigned long long start_ns,
+                                          unsigned long long records_ns) {
+  const unsigned w = *reinterpret_cast<volatile unsigned*>(job.state);
+  const bool all = (w & CHIP_COUNT) == job.full;
+  if (waited > (all ? records_ns : start_ns))
+    atomicCAS(job.state, w, w | (all ? CHIP_STALLED : CHIP_GAVE_UP));
+  return __any_sync(0xffffffffu, (w & CHIP_FAILED) != 0);
+}
+// Gives up waiting for a CTA that has not started, unless it just has.
+__device__ __forceinline__ void chip_give_up(const ChipJob& job) {
+  unsigned w = *reinterpret_cast<volatile unsigned*>(job.state);
+  while (!(w & CHIP_FAILED)) {
+    if ((w & CHIP_COUNT) == job.full) return;
+    const unsigned old = atomicCAS(job.state, w, w | CHIP_GAVE_UP);
+    if (old == w) return;
+    w = old;
+  }
+}
+// Waits until all CTAs of the job have started; false if the launch has failed.
 __device__ __forceinline__ bool chip_all_started(const ChipJob& job, unsigned long long start_ns) {
   ChipClock clock;
   for (unsigned tries = 1;; tries++) {
     const unsigned w = *reinterpret_cast<volatile unsigned*>(job.state);
     if (__any_sync(0xffffffffu, (w & CHIP_FAILED) != 0)) return false;
     if (__all_sync(0xffffffffu, (w & CHIP_COUNT) == job.full)) return true;
-    if ((tries & 1023u) == 0 && clock.look() > start_ns) chip_give_up(job, false);
+    if ((tries & 1023u) == 0 && clock.look() > start_ns) chip_give_up(job);
   }
 }
 
@@ -331,8 +340,7 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_consta
   const int npairs = rows / 2, ppw = chip_pairs_per_warp(rows);
   const int ncol = chip_col_polls(rows), npoll = chip_polls(nw, rows);
   // counted before anything is published: a tile whose neighbours' records have come knows they started
-  unsigned state = 0;
-  if (threadIdx.x == 0) state = atomicAdd(job.state, 1u);
+  if (__syncthreads_or(threadIdx.x == 0 && (atomicAdd(job.state, 1u) & CHIP_FAILED))) return;
 
   MatT<T>* mats = reinterpret_cast<MatT<T>*>(smem_raw);
   char* urows = reinterpret_cast<char*>(smem_raw) + N_MATS * sizeof(MatT<T>) + group * chip_group_bytes(nw, rows, US);
@@ -351,8 +359,10 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_consta
   // the recording launch that follows folds max|V| into the pair
   if ((int)blockIdx.x == job.cta0 && threadIdx.x < 2) f.vmax[threadIdx.x] = 0;
   for (int t = threadIdx.x; t < N_MATS; t += blockDim.x) mats[t] = mat_entry<T>(g, t);
-  const bool late = __syncthreads_or((state & CHIP_FAILED) != 0);  // the others have given up
-  if (!idle && !late) {
+  __syncthreads();
+  // A tile that has gone through n iterations has records that go back to every tile up to n - 1 away, so
+  // all have started when it writes the state back; with fewer iterations it has to look.
+  if (!idle && (n_iter >= max(ncx, ncy) || chip_all_started(job, a.start_ns))) {
     const int i = x0 - 2 + lane;
     const int jA = y0 + w * rows;
 #pragma unroll 4
@@ -524,9 +534,7 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_consta
           }
           if (!__any_sync(0xffffffffu, any)) break;
           if ((++tries & 1023u) == 0) {  // bounded: look at the clock and the state word now and then
-            const unsigned long long waited = clock.look();
-            if (waited > min(a.start_ns, a.records_ns)) chip_give_up(job, waited > a.records_ns);
-            if (__any_sync(0xffffffffu, (*reinterpret_cast<volatile unsigned*>(job.state) & CHIP_FAILED) != 0)) {
+            if (chip_look(job, clock.look(), a.start_ns, a.records_ns)) {
               failed = 1;
               break;
             }
@@ -539,15 +547,16 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_consta
           *reinterpret_cast<U2*>(urows + off) = rec[k].value();
         }
       }
-      if (group_barrier_or(1 + group, 32 * nw, failed)) break;
+      if (group_barrier_or(1 + group, 32 * nw, failed)) {
+        // (which way out decides how the march comes out at 128 registers: 1024^2 9.98 us with break, 10.05 with
+        // goto, a mixed batch 254 / 259 ms; tracking 1024^2 10.8 / 10.45)
+        if (TRACK) goto leave;
+        break;
+      }
     }
 
-    // Back to global memory: U of the last copy written, V -- unless the launch has failed.  A tile that
-    // has gone through n iterations has records that go back to every tile up to n - 1 away, so all have
-    // started; after fewer it has to look.
-    bool write = it + 1 >= n_iter;
-    if (write && n_iter < max(ncx, ncy)) write = chip_all_started(job, a.start_ns);
-    if (write && jA < ny) {
+    // back to global memory, unless the launch has failed: U of the last copy written, V
+    if ((TRACK || it + 1 >= n_iter) && jA < ny) {
       __syncwarp();
       T* uxo = u_field<T>(f, false, src ^ (n_iter & 1));
       T* uyo = u_field<T>(f, true, src ^ (n_iter & 1));
@@ -570,6 +579,7 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_iter_chip(const __grid_consta
       }
     }
   }
+leave:
   __syncthreads();
   if (wc == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(s_tmem));
 }

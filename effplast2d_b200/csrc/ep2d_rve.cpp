@@ -889,7 +889,7 @@ double Rve::error_from_vmax(double vmx, double vmy) const {
 // another (*again).
 int Rve::look_at_waits(const unsigned words[2], bool* again) {
   *again = false;
-  if (words[0] || (words[1] & CHIP_STALLED))
+  if (words[0] || (words[1] & CHIP_FAILED) == CHIP_STALLED)
     return fail(EP2D_ERR_CUDA, "resident or on-chip form: a wait for another CTA ran out; the RVE's state is invalid");
   if (!(words[1] & CHIP_GAVE_UP)) return EP2D_OK;
   *again = true;

@@ -126,6 +126,7 @@ constexpr int CHIP_SMEM_MIN = 116 * 1024;
 // CHIP_GAVE_UP is only ever set while a CTA has not started, and a CTA that finds it set leaves at once.
 constexpr unsigned CHIP_GAVE_UP = 1u << 31;  // not all CTAs started: nobody has written the state, it is as before
 constexpr unsigned CHIP_STALLED = 1u << 30;  // a running CTA's records did not come: the state is invalid
+                                             // (set behind CHIP_GAVE_UP, once all are there, it means nothing)
 constexpr unsigned CHIP_FAILED = CHIP_GAVE_UP | CHIP_STALLED;
 constexpr unsigned CHIP_COUNT = CHIP_STALLED - 1;
 // How long a launch's CTAs wait for one another.  Work that holds an SM may hold it for good (a kernel of
