@@ -7,6 +7,7 @@ The CUDA runtime is linked statically: the library needs only the NVIDIA driver.
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -19,7 +20,8 @@ CXX = os.environ.get("CXX", "g++")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CUDA_INC = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
 
-CU_SOURCES = ["ep2d_kernels.cu", "ep2d_noalloc.cu"]
+CU_SOURCES = ["ep2d_kernels.cu", "ep2d_chip.cu", "ep2d_noalloc.cu"]
+CHIP_PARTS = 5  # modules of ep2d_chip_kernels.cu
 CPP_SOURCES = ["ep2d_rve.cpp", "ep2d_api.cpp", "ep2d_batch.cpp"]
 HEADERS = ["ep2d_device.cuh", "ep2d_stencil.cuh", "ep2d_iter_f64.cuh", "ep2d_iter_stream.cuh", "ep2d_iter_chip.cuh", "ep2d_march.cuh", "ep2d_types.hpp", "ep2d_rve.hpp", "ep2d_batch.hpp"]
 
@@ -42,16 +44,23 @@ def _run(cmd):
 def build_lib(verbose=False, force=False):
     os.makedirs(BUILD, exist_ok=True)
     hdrs = [os.path.join(CSRC, h) for h in HEADERS] + [os.path.join(INCLUDE, "ep2d.h")]
-    objs = []
-    for src in CU_SOURCES:
-        s = os.path.join(CSRC, src)
-        o = os.path.join(BUILD, src + ".o")
-        if force or _newer(o, [s] + hdrs):
-            out = _run([NVCC, "-std=c++17", "-O3", "-lineinfo", *ARCH, "-Xptxas", "-v", "-Xcompiler", "-fPIC",
+    units = [(src, src + ".o", []) for src in CU_SOURCES]
+    units += [("ep2d_chip_kernels.cu", "ep2d_chip_kernels.%d.o" % k, ["-DEP2D_CHIP_PART=%d" % k]) for k in range(CHIP_PARTS)]
+
+    def compile_cu(unit):
+        s = os.path.join(CSRC, unit[0])
+        o = os.path.join(BUILD, unit[1])
+        if not (force or _newer(o, [s] + hdrs)):
+            return o, ""
+        return o, _run([NVCC, "-std=c++17", "-O3", "-lineinfo", *ARCH, *unit[2], "-Xptxas", "-v", "-Xcompiler", "-fPIC",
                         "-I" + INCLUDE, "-I" + CSRC, "-c", s, "-o", o])
+
+    objs = []
+    with ThreadPoolExecutor(min(len(units), os.cpu_count() or 1)) as pool:
+        for o, out in pool.map(compile_cu, units):
             if verbose:
                 sys.stdout.write(out)
-        objs.append(o)
+            objs.append(o)
     for src in CPP_SOURCES:
         s = os.path.join(CSRC, src)
         o = os.path.join(BUILD, src + ".o")
@@ -77,7 +86,7 @@ def build_cli_unity(macros, out, force=False):
     library sources compiled into the binary (no libep2d.so needed at run time)."""
     srcs = [os.path.join(DROPIN, s) for s in ("EffPlast2D.cu", "main.cu")]
     deps = srcs + [os.path.join(DROPIN, "EffPlast2D.h")] + [os.path.join(CSRC, h) for h in HEADERS] + \
-        [os.path.join(CSRC, s) for s in ("ep2d_kernels.cu", "ep2d_rve.cpp", "ep2d_api.cpp")]
+        [os.path.join(CSRC, s) for s in ("ep2d_kernels.cu", "ep2d_chip.cu", "ep2d_chip_kernels.cu", "ep2d_rve.cpp", "ep2d_api.cpp")]
     if force or _newer(out, deps):
         flags = ["-D%s=%s" % (k, v) for k, v in macros.items()]
         _run([NVCC, "-O3", "-std=c++17", *ARCH, "-DEP2D_UNITY", *flags, "-I" + INCLUDE, "-I" + CSRC, "-o", out,

@@ -18,6 +18,8 @@
 
 #if defined(EP2D_UNITY)
 #include "ep2d_kernels.cu"
+#include "ep2d_chip.cu"
+#include "ep2d_chip_kernels.cu"
 #include "ep2d_rve.cpp"
 #include "ep2d_api.cpp"
 #endif

@@ -35,7 +35,6 @@
 // 6.2 / 2.50, 512^2 8.9 / 3.75, 768^2 14.3 / 6.83, 1024^2 16.3 / 9.96.
 #pragma once
 
-#include "ep2d_iter_f64.cuh"
 #include "ep2d_march.cuh"
 #include "ep2d_types.hpp"
 
@@ -583,5 +582,12 @@ leave:
   __syncthreads();
   if (wc == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(s_tmem));
 }
+
+// the kernels (ep2d_chip_kernels.cu) for a shape's warps per CTA and rows per warp
+const void* chip_kernel_fp64(bool plastic, int warps, int rows);
+const void* chip_kernel_mixed(bool plastic, int warps, int rows);
+const void* chip_kernel_track(bool mixed, int warps, int rows);  // plastic
+const void* chip_kernel_f32(bool plastic);
+const void* chip_kernel_jobs(bool mixed);  // several RVEs
 
 }  // namespace ep2d

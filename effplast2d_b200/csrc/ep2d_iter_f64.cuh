@@ -315,12 +315,6 @@ __global__ void __launch_bounds__(256) k_iter_batch(const BatchEntry* __restrict
 // the flag set instead of hanging.  The flag stays set until the RVE is reset (later launches return at
 // once); the host reads it at every checkpoint and reports the RVE as failed.
 
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
 __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
   unsigned long long v;
   asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");

@@ -20,6 +20,13 @@
 
 namespace ep2d {
 
+// the clock of the bounded waits
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
 // ComputeStress at a node (EffPlast2D.cu:43-60): P = -K div U, tau = 2G (eps - div/3).
 // dux = Ux(i+1, j) - Ux(i, j), duy = Uy(i, j+1) - Uy(i, j).
 __device__ __forceinline__ void node_trial(double dux, double duy, double K, double G2, double rdX, double rdY,
