@@ -575,7 +575,7 @@ bool BatchEngine::fills_gpu(const Rve& r) const {
   return (int64_t)ux * uy >= 12 * (int64_t)sm_count_;
 }
 
-// One checkpoint interval of slot q through the single-RVE path: ce - 1 plain launches
+// One checkpoint interval of slot q through the single-RVE path: ce - 1 plain iterations
 // and the recording one, its max|V| into the slot's pair of d_vmax_.  Every form rounds
 // alike, so the result is the one the batched launches would give.
 int BatchEngine::run_solo_launches(int q) {
@@ -585,10 +585,11 @@ int BatchEngine::run_solo_launches(int q) {
   r.f.vmax = d_vmax_ + 2 * q;
   r.shape = shape_of(r.prm, sm_count_);  // always the same shape: its cached graphs stay valid
   const double ms0 = r.kernel_ms;
+  const int64_t l0 = r.launches;
   const int rc = r.iterate(ce, true);  // cur follows the launches
+  launches += r.launches - l0;
   if (rc) return rc;
   kernel_ms += r.kernel_ms - ms0;
-  launches += ce;
   cell_updates += ce * (int64_t)r.g.nx * r.g.ny;
   solo_intervals++;
   return EP2D_OK;

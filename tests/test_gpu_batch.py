@@ -208,3 +208,17 @@ def test_batch_with_gpu_filling_rve_matches_single_bit_for_bit():
         ref = s.compute_eff_moduli(load, list(lt), nts)
         s.close()
         check_result(r, ref, 0.0, nl)
+
+
+@pytest.mark.parametrize("sides", [[1024], [128], [1024, 1100, 64, 96]], ids=["large", "lone", "mixed"])
+def test_batch_counts_launches_once(sides):
+    # an interval of an RVE that runs through the single-RVE path is two launches on chip (one of many
+    # iterations, and the recording one) and one per iteration off chip; so are the shared ones'
+    ce = 40
+    specs = [B.spec(n, ep.make_pa(20.0, 20.0, n, n, yield_stress=1e-5, porosity=0.01, n_pores=1), 2, 1, -6e-5, (1.0, 0.8, 0.3))
+             for n in sides]
+    _, st = B.batch_solve(specs, niter=ce, check_every=ce, eiter=0.0)
+    per_interval = {1024: 2, 1100: ce, 128: 2}
+    shared = 2 if 64 in sides else 0
+    assert st["launches"] == 2 * (sum(per_interval.get(n, 0) for n in sides) + shared)
+    assert st["cell_updates"] == 2 * ce * sum(n * n for n in sides)
