@@ -405,21 +405,22 @@ bool BatchEngine::plan_waves(const std::vector<char>& batched) {
   for (int tall = 18; tall >= 16; tall -= 2) {
     std::vector<Wave> ws;
     std::vector<int> used;
+    bool fits = true;
     for (int q : order) {
       const int need = ctas(q, 4, 4, tall);
+      fits &= need <= CHIP_SMS;  // else there is no plan with tiles of this height
       size_t k = 0;
       while (k < ws.size() && (used[k] + need > CHIP_SMS || (int)ws[k].slots.size() == CHIP_JOBS)) k++;
       if (k == ws.size()) {
-        if (need > CHIP_SMS) return false;
         ws.emplace_back();
         used.push_back(0);
       }
       ws[k].slots.push_back(q);
       used[k] += need;
     }
-    double us = 0.0;
+    double us = fits ? 0.0 : 1e30;
     for (Wave& w : ws) {
-      if (!wave_shape(&w, tall, CHIP_SMS)) {
+      if (!fits || !wave_shape(&w, tall, CHIP_SMS)) {
         us = 1e30;
         break;
       }

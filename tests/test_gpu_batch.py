@@ -222,3 +222,18 @@ def test_batch_counts_launches_once(sides):
     shared = 2 if 64 in sides else 0
     assert st["launches"] == 2 * (sum(per_interval.get(n, 0) for n in sides) + shared)
     assert st["cell_updates"] == 2 * ce * sum(n * n for n in sides)
+
+
+def test_batch_waves_of_the_tallest_tiles_only():
+    # 300 strips of 72 rows fit the SMs with tiles of 72 rows (18 per warp), not with tiles of 64
+    nx, ny, ce = 8400, 72, 100
+    pa = ep.make_pa(20.0, 20.0, nx, ny, yield_stress=1e-5, porosity=0.01, n_pores=1)
+    specs = [B.spec(nx, pa, 2, 1, -6e-5, (1.0, 0.8, 0.3 * k), ny=ny) for k in (1, 2)]
+    kw = dict(niter=ce, check_every=ce, eiter=0.0)
+    a, _ = B.batch_solve(specs, kernel=ep.KERNEL_STREAM, rows=16, **kw)
+    b, sb = B.batch_solve(specs, **kw)
+    assert sb["solo_intervals"] == 0 and sb["launches"] == 2 * 3  # two waves and a recording launch
+    for x, y in zip(a, b):
+        for m in ("kphi", "kd", "g"):
+            u, v = x["num"][m], y["num"][m]
+            assert u == v or (math.isnan(u) and math.isnan(v)), (m, u, v)
