@@ -83,13 +83,43 @@ def measured_peaks():
     return 6650.0, "fallback"
 
 
-def ncu_traffic(workload):
-    """DRAM bytes per launch of the iteration kernel from the committed ncu summary."""
-    p = os.path.join(ROOT, "profiles", "iter_stream_%s.json" % workload)
-    if os.path.exists(p):
-        d = json.load(open(p))
-        return d.get("dram_bytes_per_launch")
-    return None
+def kernel_name(form, on_chip):
+    """the kernel that runs a plain iteration"""
+    if on_chip:
+        return "k_iter_chip"
+    return {"stream": "k_iter_pairs", "tile": "k_iter", "resident": "k_iter_resident"}[form]
+
+
+def ncu_traffic(kernel, workload, precision="fp64"):
+    """DRAM bytes per launch of an iteration kernel on a workload from the committed ncu summary
+    of that kernel, None without one."""
+    p = os.path.join(ROOT, "profiles", "%s_%s.json" % (kernel[2:], workload))
+    if precision != "fp64" or not os.path.exists(p):
+        return None
+    d = json.load(open(p))
+    return d["dram_bytes_per_launch"] if d["kernel"].startswith(kernel + "<") else None
+
+
+def roofline(workload, n, nl, form, on_chip, iter_s, precision="fp64"):
+    """One plain iteration against what bounds it.  On chip the state does not leave the SMs
+    between iterations: arithmetic (85 operations per cell with the return map, 40
+    elastic) at the nominal rate of the lanes.  Else HBM: U and V read once and written once."""
+    kernel = kernel_name(form, on_chip)
+    bytes_alg = {"fp64": 64, "mixed": 48, "f32": 32}[precision] * n * n
+    out = {"kernel": kernel, "traffic": None if on_chip else ncu_traffic(kernel, workload, precision),
+           "algorithmic_bytes_per_launch": bytes_alg, "avg_launch_us": iter_s * 1e6}
+    if on_chip:
+        lanes = 128 if precision == "f32" else 64
+        peak = lanes * 2 * 148 * 1.965e9 / 1e12
+        achieved = (85 if nl > 1 else 40) * n * n / iter_s / 1e12
+        out.update(bound="fp32" if precision == "f32" else "fp64", unit="TFLOP/s",
+                   peak_source="nominal: %d lanes x 2 x 148 SMs x 1.965 GHz" % lanes)
+    else:
+        peak, source = measured_peaks()
+        achieved = bytes_alg / iter_s / 1e9
+        out.update(bound="hbm", unit="GB/s", peak_source=source)
+    out.update(achieved=achieved, peak=peak, frac=achieved / peak)
+    return out
 
 
 class ClockSampler:
@@ -394,10 +424,8 @@ def run_ours(args, w):
     # roofline of the fused iteration kernel over the timed region
     # (per iteration: a launch of the on-chip form runs many)
     it_ms = st1["kernel_ms"] - st0["kernel_ms"]
-    avg_launch_s = it_ms / 1000.0 / max((st1["cell_updates"] - st0["cell_updates"]) // (n * n), 1)
-    bytes_alg = 64 * n * n  # Ux, Uy, Vx, Vy read once and written once, FP64
-    achieved = bytes_alg / avg_launch_s / 1e9
-    peak, peak_kind = measured_peaks()
+    iters = max((st1["cell_updates"] - st0["cell_updates"]) // (n * n), 1)
+    on_chip = args.kernel == 0 and 2 * (st1["launches"] - st0["launches"]) < iters
     ips = iterations_per_solve(args.workload) or (res["total_iterations"] if res else None)
 
     line = None
@@ -411,15 +439,9 @@ def run_ours(args, w):
             "config": bench_config(w, args.workload, world, ips),
             "kernel": {"form": KERNEL_NAMES[shape[0]], "rows": shape[1]},
             "e2e": None,
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "traffic": ncu_traffic(args.workload),
-                         "kernel": "fused stress, J2 return, momentum update (k_iter_chip for runs of "
-                                   "iterations of a grid that fits on chip, else the kernel form above)",
-                         "algorithmic_bytes_per_launch": bytes_alg, "avg_launch_us": avg_launch_s * 1e6,
-                         "peak_source": peak_kind,
-                         "note": "per iteration; on chip the %d^2 state does not leave the SMs between "
-                                 "iterations, so this fraction measures throughput against a bound the kernel "
-                                 "does not meet here; the HBM-resident case is roofline_hbm" % n},
+            "roofline": dict(roofline(args.workload, n, w["nl"], KERNEL_NAMES[shape[0]], on_chip,
+                                      it_ms / 1000.0 / iters),
+                             note="per iteration, recording launches included; the HBM-resident case is roofline_hbm"),
             "gpu_launches": launches,
             "clocks": clocks.summary(),
             "cell_updates_per_s": iters_per_s * n * n,
@@ -439,11 +461,12 @@ def run_ours(args, w):
                                     "sample": desc + "; converted with %d iterations per solve" % ips,
                                     "single_thread": {"value": rate1 / (n * n * ips), "cores": 1, "sample": desc1}}
         if world == 1 and not args.no_extras:
-            # the HBM-bound case of the same kernel (the 1024^2 state above is L2-resident)
+            # the HBM-bound case of the same iteration (the 1024^2 state above stays on chip)
             line["roofline_hbm"] = dict(kernel_timing("cfg3", args.hbm_iters),
                                         note="2048x2048 grid, FP64: 13 fields of 34 MB (0.45 GB) > 126 MB L2; "
                                              "achieved = 64 B x 2048^2 per launch / CUDA-event time per launch; "
-                                             "traffic from the committed ncu capture of this kernel and grid")
+                                             "traffic from the committed ncu capture of that kernel and grid, "
+                                             "with a cold L2")
             # the metric's batched and served headline, sized to fit this run
             sides = tuple(int(x) for x in args.extra_sides.split(","))
             line["batched"] = batch_object(args.extra_batch, args.seed, args.extra_niter, sides=sides)
@@ -462,7 +485,7 @@ def run_ours(args, w):
 def kernel_timing(workload, iters, kernel=0, rows=0, precision="fp64", w=None):
     """Exactly `iters` pseudo-time iterations of the workload's preload step (no
     convergence test), after one untimed pass of the same length: CUDA-event time per
-    launch of the fused iteration kernel on its own stream, and its HBM roofline.
+    iteration on the handle's stream, and its roofline.
     precision "f32": the FP32 bulk's FP32 form (32 B per cell-update: u' and V in FP32)."""
     import torch
 
@@ -491,15 +514,12 @@ def kernel_timing(workload, iters, kernel=0, rows=0, precision="fp64", w=None):
     # per iteration (a resident-form launch runs many)
     iters_run = (st1["cell_updates"] - st0["cell_updates"]) // (n * n)
     per = (st1["kernel_ms"] - st0["kernel_ms"]) / max(iters_run, 1)
-    bytes_alg = {"fp64": 64, "mixed": 48, "f32": 32}[precision] * n * n
-    peak, kind = measured_peaks()
-    achieved = bytes_alg / (per / 1e3) / 1e9
+    on_chip = kernel == 0 and 2 * (st1["launches"] - st0["launches"]) < iters_run
+    roof = roofline(workload, n, w["nl"], KERNEL_NAMES[shape[0]], on_chip, per / 1e3, precision)
     return {"workload": workload, "grid": "%dx%d" % (n, n), "iterations": iters, "precision": precision,
-            "kernel": {"form": KERNEL_NAMES[shape[0]], "rows": shape[1]},
             "iteration_launches": st1["launches"] - st0["launches"],
-            "avg_launch_us": per * 1e3, "algorithmic_bytes_per_launch": bytes_alg, "achieved": achieved,
-            "peak": peak, "unit": "GB/s", "peak_source": kind, "frac": achieved / peak,
-            "traffic": ncu_traffic(workload), "wall_s": wall, "cell_updates_per_s": n * n / (per / 1e3)}
+            **dict(roof, kernel={"name": roof["kernel"], "form": KERNEL_NAMES[shape[0]], "rows": shape[1]}),
+            "wall_s": wall, "cell_updates_per_s": n * n / (per / 1e3)}
 
 
 KERNEL_NAMES = {0: "auto", 1: "tile", 2: "stream", 3: "resident"}

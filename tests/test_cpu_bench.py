@@ -50,3 +50,21 @@ def test_reference_arm_other_ranks_exit_quietly():
     r = run_reference_arm({"RANK": "1", "LOCAL_RANK": "1", "WORLD_SIZE": "2"})
     assert r.returncode == 0, r.stderr
     assert r.stdout.strip() == ""
+
+
+def test_traffic_is_the_named_kernels():
+    import bench
+
+    # the plain iterations at 2048^2 are k_iter_pairs', and its capture is committed
+    r = bench.roofline("cfg3", 2048, 3, "stream", False, 52e-6)
+    assert r["kernel"] == "k_iter_pairs" and r["bound"] == "hbm"
+    with open(os.path.join(ROOT, "profiles", "iter_pairs_cfg3.json")) as f:
+        d = json.load(f)
+    assert d["kernel"].startswith("k_iter_pairs<") and d["grid"] == [2048, 2048]
+    assert r["traffic"] == d["dram_bytes_per_launch"]
+    # on chip there is no traffic per iteration, and the bound is not HBM's
+    r = bench.roofline("cfg2", 1024, 3, "stream", True, 10e-6)
+    assert r["kernel"] == "k_iter_chip" and r["traffic"] is None and r["bound"] == "fp64" and 0 < r["frac"] < 1
+    # no capture of this kernel on this grid
+    assert bench.roofline("cfg2", 1024, 3, "stream", False, 16e-6)["traffic"] is None
+    assert bench.roofline("cfg3", 2048, 3, "stream", False, 52e-6, "f32")["traffic"] is None
