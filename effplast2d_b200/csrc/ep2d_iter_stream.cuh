@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(32 * STREAM_WARPS) k_iter_stream_batch(const B
 // us per iteration with the return map, k_iter_stream before / this: 2048^2 60.5 / 52.4 (5.1 TB/s of the
 // 64 B per cell, 0.78 of the measured HBM rate), 1536^2 44.5 / 29.5 and 1200^2 25.6 / 17.7 (with
 // segments that fill one wave, shape_of), 2048^2 elastic 61.7 / 45.4, FP32 bulk 41.7 / 31.0.  What bounds it
-// at 2048^2: issue (205 warp instructions per strip row where all yields, 64 % of
+// at 2048^2: issue (211 warp instructions per strip row, 65 % of
 // cycles) together with HBM.
 constexpr int PAIR_DEPTH = 2;
 constexpr int PAIR_SLOTS = PAIR_DEPTH + 2;

@@ -125,10 +125,11 @@ IterShape shape_of(const ep2d_params& p, int sm_count) {
     // 320^2: 6.5 vs 6.1), elastic RVEs below 12 (384^2: 5.6 vs 6.0; 512^2: 6.9 vs 6.2).
     // Both forms round alike.  Tiles of 8 rows where 16-row tiles would give fewer than
     // two per SM (128^2 4.4 vs 5.2 us, 256^2 5.8 vs 7.2 us).  On elastic RVEs with at
-    // most two 8-row tiles per SM (up to ~256^2) the resident form, all iterations of a
-    // checkpoint interval in one launch, is faster still (128^2: 4.03 vs 4.39 us, 256^2:
-    // 4.55 vs 4.90 us; 320^2: 5.12 vs 4.97); with the return map it is slower at every
-    // size (256^2: 6.36 vs 5.77 us).
+    // most two 8-row tiles per SM (up to ~256^2) the resident form beats single tile launches
+    // (128^2: 4.03 vs 4.39 us, 256^2: 4.55 vs 4.90 us; 320^2: 5.12 vs 4.97); with the return map
+    // it is slower at every size (256^2: 6.36 vs 5.77 us).  Of all these forms the on-chip form leaves
+    // a handle's recording launches and its runs below CHIP_MIN_RUN iterations, and everything where a
+    // device has no room for its CTAs.
     if (p.kernel == EP2D_KERNEL_AUTO && 2 * warps(SEG_MIN) < (p.nl == 1 ? 24 : 11) * sms) {
       s.form = FORM_TILE;
       const int64_t tx = (p.nx + TILE_X - 1) / TILE_X;
@@ -1168,13 +1169,15 @@ void dims(int nx, int ny, int field, int* w, int* h) {
 namespace {
 // Have the pages of a large output buffer present before the copy into it: the copy from the
 // device faults pages of fresh memory in one by one (2048^2, 34 MB: 7.5 ms, 1.6 ms into pages that
-// are present; 4.1 with this).  Four threads fault in a quarter each; a kernel that does not know
+// are present; 4.1 with this).  Large means what glibc's malloc always maps anew, 32 MiB and more (its
+// threshold for that rises to there with the sizes that are freed); smaller buffers of a program that reads
+// fields again and again have their pages.  Four threads fault in a quarter each; a kernel that does not know
 // MADV_POPULATE_WRITE, or a buffer it refuses, leaves the copy to do it.  Contents are kept.
 void populate(void* p, size_t bytes) {
 #ifndef MADV_POPULATE_WRITE
 #define MADV_POPULATE_WRITE 23
 #endif
-  constexpr size_t kLarge = (size_t)32 << 20;  // smaller ones come warm from the heap as a rule
+  constexpr size_t kLarge = (size_t)32 << 20;
   constexpr int kThreads = 4;
   if (bytes < kLarge) return;
   const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);

@@ -60,7 +60,7 @@ enum {
 /* form of the fused iteration kernel (both compute the same iteration, operation for
  * operation; they differ in how threads map onto the grid) */
 enum {
-  EP2D_KERNEL_AUTO = 0,   /* the library's choice (the stream form, segments of 4 to 64
+  EP2D_KERNEL_AUTO = 0,   /* the library's choice (the stream form, segments of 4 to 96
                              rows by grid size; the tile form for grids too small to occupy
                              the GPU even with 4-row segments, the resident form for small
                              elastic ones; batches: timed).  A single RVE whose grid fits
@@ -283,7 +283,10 @@ int ep2d_compute_eff_damping(ep2d_handle* h, double init_load_value, const doubl
 
 /* SaveAnStatic2D's numerical fields (EffPlast2D.cu:1098-1134): |u| at nodes (nx*ny),
  * J1 and J2 at corners ((nx-1)*(ny-1)), from the state after the last load step with
- * displacements zeroed inside the pores (EffPlast2D.cu:514-547). */
+ * displacements zeroed inside the pores (EffPlast2D.cu:514-547).
+ * This call and the next ones work in temporary device memory (up to 9 fields); up to 24 MB of it
+ * stays with the handle for the next such call until the handle is destroyed, beyond
+ * ep2d_rve_footprint. */
 int ep2d_static_fields(ep2d_handle* h, double* unu_abs, double* j1nu, double* j2nu);
 
 /* SaveAnStatic2D's analytic part (EffPlast2D.cu:1060-1292): the Yarushina (2010)
