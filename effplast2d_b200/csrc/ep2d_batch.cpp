@@ -473,7 +473,7 @@ int BatchEngine::run_waves(int64_t n, bool* done) {
       if (waves_ok_ && chip_room != 0) {
         if (chip_room > 0) chip_room--;
         if (!held.sms)
-          held.sms = share.take([&](int rves, int) {
+          held.sms = share.take([&](int rves, int, int) {
             if (alone) return most;
             Wave part = w;
             if (wave_shape(&part, 18, (int)((int64_t)CHIP_SMS * n_rves / std::max(rves, n_rves)))) fit = part.shape;

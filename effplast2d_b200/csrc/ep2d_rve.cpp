@@ -364,15 +364,20 @@ SmShare::Call::~Call() {
   std::lock_guard<std::mutex> lk(s.mu_);
   s.rves_ -= rves;
 }
-int SmShare::take(const std::function<int(int, int)>& need) {
+int SmShare::take(const std::function<int(int, int, int)>& need) {
   std::unique_lock<std::mutex> lk(mu_);
   const uint64_t me = next_++;
   cv_.wait(lk, [&] { return serving_ == me; });
-  const int n = std::min(need(rves_, free_), CHIP_SMS);
+  struct Next {  // also where need throws
+    SmShare& s;
+    ~Next() {
+      s.serving_++;
+      s.cv_.notify_all();
+    }
+  } next{*this};
+  const int n = std::min(need(rves_, free_, (int)(next_ - serving_)), CHIP_SMS);
   cv_.wait(lk, [&] { return free_ >= n; });
   free_ -= n;
-  serving_++;
-  cv_.notify_all();
   return n;
 }
 void SmShare::give(int sms) {
@@ -752,13 +757,13 @@ int Rve::run_chip(int64_t* n) {
 ChipShape Rve::take_sms() {
   give_sms();
   ChipShape s = chip;
-  sms_ = SmShare::of(device).take([&](int rves, int free) {
+  sms_ = SmShare::of(device).take([&](int rves, int free, int waiting) {
     if (rves > 1) {
       ChipShape t = chip_shape_beside(prm.nx, prm.ny, rves, CHIP_SMS);
-      // rather than wait, the SMs that are left (a 64^2 handle beside a batch on 138 of them: 8.6 -> 6.3 us
-      // an iteration, a 128^2 one 7.9 -> 4.6)
+      // rather than wait, the SMs that are left (a 64^2 handle beside a batch on 138 of them: 8.6 -> 2.5 us
+      // an iteration, a 128^2 one 7.9 -> 4.8), shared with the launches that wait too
       if (chip_ctas(prm.nx, prm.ny, t.groups, t.warps, t.rows) > free) {
-        const ChipShape left = chip_shape_beside(prm.nx, prm.ny, rves, free);
+        const ChipShape left = chip_shape_beside(prm.nx, prm.ny, waiting, free);
         if (left.warps) t = left;
       }
       if (chip_usable(t)) s = t;
@@ -769,7 +774,7 @@ ChipShape Rve::take_sms() {
 }
 void Rve::take_all_sms() {
   give_sms();
-  sms_ = SmShare::of(device).take([](int, int) { return CHIP_SMS; });
+  sms_ = SmShare::of(device).take([](int, int, int) { return CHIP_SMS; });
 }
 // the stream is idle: other handles may have them
 void Rve::give_sms() {

@@ -81,8 +81,8 @@ class SmShare {
     Call(SmShare& share, int rves);
     ~Call();
   };
-  // wait for need(RVEs of all calls in progress, SMs free now) SMs
-  int take(const std::function<int(int, int)>& need);
+  // wait for need(RVEs of all calls in progress, SMs free now, launches that wait, this one among them) SMs
+  int take(const std::function<int(int, int, int)>& need);
   void give(int sms);
   int rves();  // of all calls in progress
 
