@@ -760,8 +760,8 @@ ChipShape Rve::take_sms() {
   sms_ = SmShare::of(device).take([&](int rves, int free, int waiting) {
     if (rves > 1) {
       ChipShape t = chip_shape_beside(prm.nx, prm.ny, rves, CHIP_SMS);
-      // rather than wait, the SMs that are left (a 64^2 handle beside a batch on 138 of them: 8.6 -> 2.5 us
-      // an iteration, a 128^2 one 7.9 -> 4.8), shared with the launches that wait too
+      // rather than wait, the SMs that are left (a 64^2 handle beside a batch on 138 of them: 8.6 -> 2.5 to
+      // 5.3 us an iteration, a 128^2 one 7.9 -> 4.8), shared with the launches that wait too
       if (chip_ctas(prm.nx, prm.ny, t.groups, t.warps, t.rows) > free) {
         const ChipShape left = chip_shape_beside(prm.nx, prm.ny, waiting, free);
         if (left.warps) t = left;
